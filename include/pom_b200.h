@@ -137,9 +137,22 @@ int pom_gemm_bf16(const pom_gemm_args* a, int* status, void* stream);
  * CTA then changes its column block from tile to tile).  Process-wide, not thread-safe against concurrent launches. */
 int pom_set_gemm_mode(int mode);
 
-/* fp32 SIMT GEMM with the same meaning (fp32 A, Bm, C; out_mode F32 or F32_ACCUM); used by the
- * fp32 precision mode, where tensor-core inputs would not meet the 1e-4 bound. */
+/* fp32 FMA GEMM with the same meaning (fp32 A, Bm, C; out_mode F32 or F32_ACCUM): products too small for the
+ * tensor-core form below. */
 int pom_gemm_f32(const pom_gemm_args* a, void* stream);
+
+/* The same product on the tensor cores, at the accuracy of float32 sums: each operand is written as three bf16 planes
+ * that hold all its bits, and the six largest plane products are summed (batches must be 1; any strides, sizes and
+ * alignment).  `a_planes` / `b_planes`: 16-byte aligned buffers of pom_f32_planes_bytes(rows, cols) of the operand as
+ * it is stored; *_ready != 0 when an earlier call with the same operand (whichever major it was read in) has filled
+ * them.  `scratch`: pom_gemm_f32_planes_scratch bytes (0: may be NULL).  Operands with infinities, NaN or magnitudes of
+ * 2^56 and more are computed by the FMA kernel, which is always enqueued behind the product and returns at once
+ * otherwise.  Results are the same bits on every run; K is split (partial sums in `scratch`) in accumulate mode only, so
+ * that a row of a plain product does not depend on how many rows there are. */
+uint64_t pom_f32_planes_bytes(int64_t rows, int64_t cols);
+uint64_t pom_gemm_f32_planes_scratch(int64_t M, int64_t N, int64_t K, int32_t out_mode);
+int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_planes, int b_ready, void* scratch,
+                        int* status, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Context phase, fused (bf16): hp = X·Wpoᵀ on tensor cores; the epilogue rounds hp to bf16,

@@ -1,5 +1,4 @@
-// Host launchers for the tcgen05 GEMM engine and its fused PoM epilogues, plus
-// the fp32 SIMT GEMM of the high-precision mode.
+// Host launchers for the tcgen05 GEMM engine and its fused PoM epilogues.
 #include <cudaTypedefs.h>
 #include <mutex>
 #include "common.cuh"
@@ -14,77 +13,6 @@ std::atomic<long long> g_launches{0};
 // 0: automatic choice, 1: always the one-CTA kernel, 2: always the two-CTA (pair) kernel.
 std::atomic<int> g_gemm_mode{0};
 }
-
-namespace {
-
-// ---------------------------------------------------------------- fp32 SIMT GEMM
-// 64x64 tile, 16-deep k step, 256 threads with 4x4 outputs each.  Strided operand
-// access covers both storage orders.  Accuracy, not speed, is the purpose.
-__global__ void __launch_bounds__(256)
-sgemm_kernel(const float* __restrict__ A, const float* __restrict__ Bm, float* __restrict__ C, int M, int N, int K,
-             long long sam, long long sak, long long sbn, long long sbk, long long ldc, float alpha, int accumulate) {
-  __shared__ float As[16][64 + 1];
-  __shared__ float Bs[16][64 + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += 16) {
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      // choose the faster-varying index to follow the contiguous dimension
-      int mm, kk;
-      if (sak == 1) {
-        kk = i & 15;
-        mm = i >> 4;
-      } else {
-        mm = i & 63;
-        kk = i >> 6;
-      }
-      const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? A[gm * sam + gk * sak] : 0.f;
-    }
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      int nn, kk;
-      if (sbk == 1) {
-        kk = i & 15;
-        nn = i >> 4;
-      } else {
-        nn = i & 63;
-        kk = i >> 6;
-      }
-      const int gn = n0 + nn, gk = k0 + kk;
-      Bs[kk][nn] = (gn < N && gk < K) ? Bm[gn * sbn + gk * sbk] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty * 4 + i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn >= N) continue;
-      float* c = C + static_cast<long long>(gm) * ldc + gn;
-      const float v = alpha * acc[i][j];
-      *c = accumulate ? (*c + v) : v;
-    }
-  }
-}
-
-}  // namespace
 
 // =========================================================================== C ABI
 extern "C" {
@@ -134,25 +62,6 @@ int pom_set_gemm_mode(int mode) {
   if (mode < 0 || mode % 10 > 2 || (mode / 10) % 10 > 3 || mode / 100 > 1) return POM_ERR_UNSUPPORTED;
   g_gemm_mode.store(mode);
   return POM_OK;
-}
-
-int pom_gemm_f32(const pom_gemm_args* a, void* stream) {
-  if (!a || !a->A || !a->Bm || !a->C) return POM_ERR_NULL;
-  if (a->M <= 0 || a->N <= 0 || a->K <= 0 || a->batches <= 0) return POM_ERR_BAD_SHAPE;
-  if (a->out_mode != POM_OUT_F32 && a->out_mode != POM_OUT_F32_ACCUM) return POM_ERR_UNSUPPORTED;
-  if (a->a_mn_major && a->batches != 1) return POM_ERR_UNSUPPORTED;
-  const long long Mtot = a->M * a->batches;
-  if (Mtot > INT32_MAX || a->N > INT32_MAX || a->K > INT32_MAX) return POM_ERR_TOO_LARGE;
-  const long long sam = a->a_mn_major ? 1 : a->lda, sak = a->a_mn_major ? a->lda : 1;
-  const long long sbn = a->b_mn_major ? 1 : a->ldb, sbk = a->b_mn_major ? a->ldb : 1;
-  dim3 grid(static_cast<unsigned>(ceil_div(a->N, 64)), static_cast<unsigned>(ceil_div(Mtot, 64)));
-  if (grid.y > 65535) return POM_ERR_TOO_LARGE;
-  sgemm_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const float*>(a->A), static_cast<const float*>(a->Bm), static_cast<float*>(a->C),
-      static_cast<int>(Mtot), static_cast<int>(a->N), static_cast<int>(a->K), sam, sak, sbn, sbk, a->ldc, a->alpha,
-      a->out_mode == POM_OUT_F32_ACCUM);
-  count_launch();
-  return check_launch();
 }
 
 int pom_ctx_gemm(const pom_ctx_args* a, int* status, void* stream) {

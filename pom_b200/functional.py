@@ -367,12 +367,14 @@ class _PoMLayer(torch.autograd.Function):
                                        rope=spec.rope_ctx)
             S_part = partial  # per-tile sums; reduced (and normalised, when no exchange is needed) below
         else:
+            # float32: the projections feed the kinks of the activation and of the gate, where the rounding of a sum
+            # picks the side and with it a whole gradient term: they keep the FMA chain's order of additions
             if spec.self_mixing:
-                hs = ops.gemm(xq.view(B * T, D), w_qc).view(B, T, P + S)
+                hs = ops.gemm(xq.view(B * T, D), w_qc, fma=True).view(B, T, P + S)
                 hp, z = hs[..., :P], hs[..., P:]
             else:
-                hp = ops.gemm(xc.view(B * N, D), w_po).view(B, N, P)
-                z = ops.gemm(xq.view(B * T, D), w_se).view(B, T, S)
+                hp = ops.gemm(xc.view(B * N, D), w_po, fma=True).view(B, N, P)
+                z = ops.gemm(xq.view(B * T, D), w_se, fma=True).view(B, T, S)
             if not causal and not full:
                 S_part = ops.poly_agg_fwd(hp, coeff32, row_weight=maskf, rope=spec.rope_ctx)  # per-chunk sums
         if fused_causal:
@@ -511,8 +513,9 @@ class _PoMLayer(torch.autograd.Function):
         d_bias = flat[n_qc + n_ag:n_qc + n_ag + S]
         d_coeff = flat[n_qc + n_ag + S:n_flat].view(P, K)
         # dWo[d, p] = sum_t dY[t, d] * SH[t, p]   (collapsed multi-head path: formed from dMb further down)
+        dy_pl = ops.F32Planes()  # float32: the planes of dY and G serve two products each
         if not ctx.collapsed:
-            ops.gemm(dy2, sh.view(B * T, P), a_mn=True, b_mn=True, out=d_wag, accumulate=True)
+            ops.gemm(dy2, sh.view(B * T, P), a_mn=True, b_mn=True, out=d_wag, accumulate=True, a_planes=dy_pl)
 
         if spec.self_mixing:
             G = torch.empty((B * T, P + S), dtype=dt, device=dev)
@@ -551,7 +554,7 @@ class _PoMLayer(torch.autograd.Function):
             ops.select_bwd(ds, z, bias32, _ones(B, heads, dev), g_z.view(B, T, heads), rope=spec.rope_qry,
                            dbias_out=d_bias)
         else:
-            dsh = ops.gemm(dy2, w_ag, b_mn=True).view(B, T, P)
+            dsh = ops.gemm(dy2, w_ag, b_mn=True, a_planes=dy_pl).view(B, T, P)
             if heads:
                 ds32 = ops.zeros_f32(B * T * heads, dev).view(B, T, heads)
                 dH = ops.select_heads_bwd(dsh, s32, Hc if (causal or full) else H, ds32)
@@ -614,11 +617,12 @@ class _PoMLayer(torch.autograd.Function):
         # beside the data-gradient products.  The GEMM's CTAs fill the shared memory of the SMs they occupy, so the
         # all-reduce's CTAs run on the SMs the GEMM leaves idle (its last, partial wave) and otherwise right after
         # it; no rank can block another for longer than that, and every wait is bounded
+        g_pl, z_pl = ops.F32Planes(), ops.F32Planes()
         if spec.self_mixing:
-            ops.gemm(G, xq.view(B * T, D), a_mn=True, b_mn=True, out=d_wqc, accumulate=True)
+            ops.gemm(G, xq.view(B * T, D), a_mn=True, b_mn=True, out=d_wqc, accumulate=True, a_planes=g_pl)
         else:
-            ops.gemm(g_hp, xc.view(B * N, D), a_mn=True, b_mn=True, out=d_wqc[:P], accumulate=True)
-            ops.gemm(g_z, xq.view(B * T, D), a_mn=True, b_mn=True, out=d_wqc[P:], accumulate=True)
+            ops.gemm(g_hp, xc.view(B * N, D), a_mn=True, b_mn=True, out=d_wqc[:P], accumulate=True, a_planes=g_pl)
+            ops.gemm(g_z, xq.view(B * T, D), a_mn=True, b_mn=True, out=d_wqc[P:], accumulate=True, a_planes=z_pl)
         # all parameters bf16 and the peer transport: the gradients cross NVLink as bf16 (half the bytes; the result
         # image is copied out because the next backward pass reuses it)
         wire_bf16 = peer_flat and dts == {torch.bfloat16}
@@ -628,11 +632,11 @@ class _PoMLayer(torch.autograd.Function):
             with torch.cuda.stream(side):
                 f16 = ops.clone(shard.peer.allreduce_flat_bf16(n_flat))
         if spec.self_mixing:
-            dxq = ops.gemm(G, w_qc, b_mn=True).view(B, T, D)
+            dxq = ops.gemm(G, w_qc, b_mn=True, a_planes=g_pl).view(B, T, D)
             dxc = None
         else:
-            dxc = ops.gemm(g_hp, w_qc[:P], b_mn=True).view(B, N, D)
-            dxq = ops.gemm(g_z, w_qc[P:], b_mn=True).view(B, T, D)
+            dxc = ops.gemm(g_hp, w_qc[:P], b_mn=True, a_planes=g_pl).view(B, N, D)
+            dxq = ops.gemm(g_z, w_qc[P:], b_mn=True, a_planes=z_pl).view(B, T, D)
         if overlap:
             main.wait_stream(side)
             f16.record_stream(main)

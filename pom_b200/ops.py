@@ -146,15 +146,40 @@ def _rope_c(spec: Optional[RopeSpec]) -> Rope:
 
 
 # ---------------------------------------------------------------------------- GEMM
+class F32Planes:
+    """The three bf16 planes of a float32 GEMM operand (``pom_gemm_f32_planes``).  Pass one object to two products of
+    the same, unchanged tensor and the second finds the planes in place."""
+    __slots__ = ("buf", "ready")
+
+    def __init__(self):
+        self.buf, self.ready = None, 0
+
+    def take(self, t: torch.Tensor) -> torch.Tensor:
+        if self.buf is None:
+            nbytes = int(_abi.lib().pom_f32_planes_bytes(t.shape[0], t.shape[1]))
+            self.buf = torch.empty((nbytes,), dtype=torch.uint8, device=t.device)
+        return self.buf
+
+
+def f32_planes_pay(K: int) -> bool:
+    """Whether a float32 product runs on the tensor cores (``pom_gemm_f32_planes``) or on the FMA kernel.  At K = 64 and
+    64 to 256 rows and columns the planes take 8 to 10 us (three launches) and the FMA kernel 5; at K = 128 11 and 8 to
+    9.5; at K = 256 14 and 14 to 17, and from there on, or with more rows, the planes win by up to five times.  M and N
+    do not enter: a sample's result has the same bits whatever batch it came in."""
+    return K >= 128
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          accumulate: bool = False, split_k: int = 0, alpha: float = 1.0, act: Optional[str] = None,
-         residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+         residual: Optional[torch.Tensor] = None, a_planes: Optional[F32Planes] = None,
+         b_planes: Optional[F32Planes] = None, fma: bool = False) -> torch.Tensor:
     """C[m, n] = alpha * sum_k A[m, k] * B[n, k].
 
     ``a`` is (M, K) — or (K, M) when ``a_mn`` — and ``b`` is (N, K) — or (K, N) when ``b_mn``;
     both row-major with a contiguous last dimension.  bf16 inputs run on the tcgen05 kernel,
-    fp32 inputs on the SIMT kernel.  ``accumulate`` adds into a fp32 ``out``.  For bf16 outputs the epilogue can
+    fp32 inputs on its three-plane form (``a_planes`` / ``b_planes``: see :class:`F32Planes`) or, with ``fma`` or a short
+    K, on the FMA kernel, which sums every output as one chain over k.  ``accumulate`` adds into a fp32 ``out``.  For bf16 outputs the epilogue can
     apply ``act="gelu"`` and add a bf16 ``residual`` of the output's shape.
     """
     dev = _require_cuda(a, b, out)
@@ -198,7 +223,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     else:
         if a.dtype != torch.float32 or out.dtype != torch.float32:
             raise TypeError("fp32 GEMM needs float32 operands and output")
-        _abi.check(L.pom_gemm_f32(C.byref(g), _abi.stream_ptr()), "pom_gemm_f32")
+        if not fma and f32_planes_pay(K):
+            pa, pb = a_planes or F32Planes(), b_planes or F32Planes()
+            nbytes = int(L.pom_gemm_f32_planes_scratch(M, N, K, g.out_mode))
+            scratch = torch.empty((nbytes,), dtype=torch.uint8, device=dev) if nbytes else None
+            _abi.check(L.pom_gemm_f32_planes(C.byref(g), ptr(pa.take(a)), pa.ready, ptr(pb.take(b)), pb.ready,
+                                             ptr(scratch), ptr(_abi.status_word(dev)), _abi.stream_ptr()),
+                       "pom_gemm_f32_planes")
+            pa.ready = pb.ready = 1
+        else:
+            _abi.check(L.pom_gemm_f32(C.byref(g), _abi.stream_ptr()), "pom_gemm_f32")
     return out
 
 

@@ -1,0 +1,108 @@
+"""float32 GEMM on the tensor cores (three bf16 planes) against float64: every operand order, edges of tiles, K splits,
+and the values that the planes cannot carry."""
+import itertools
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _gemm64(a, b, a_mn, b_mn):
+    a64, b64 = a.double(), b.double()
+    return (a64.t() if a_mn else a64) @ (b64 if b_mn else b64.t())
+
+
+def _operands(M, N, K, a_mn, b_mn, seed, pad=0):
+    g = torch.Generator().manual_seed(seed)
+    a = torch.randn((K, M + pad) if a_mn else (M, K + pad), generator=g).cuda()
+    b = torch.randn((K, N + pad) if b_mn else (N, K + pad), generator=g).cuda()
+    return (a[:, :M] if a_mn else a[:, :K]), (b[:, :N] if b_mn else b[:, :K])
+
+
+def _planes(a, b, use=True, **kw):
+    from unittest import mock
+
+    from pom_b200 import ops
+
+    with mock.patch.object(ops, "f32_planes_pay", lambda *_: use):
+        return ops.gemm(a, b, **kw)
+
+
+# A float32 chain of K fused multiply-adds is off by about sqrt(K) / 4 units of 2^-24 of sum |a||b| / sqrt(K): 4e-7 at
+# K = 1000 for these inputs.  The planes add K / 64 block sums; 2.5e-7 holds for every K here.
+BOUND = 2.5e-7
+SHAPES = [(1, 1, 1), (3, 5, 7), (128, 128, 64), (129, 127, 65), (256, 256, 128), (257, 300, 63), (500, 1152, 200),
+          (512, 256, 1000), (255, 513, 4100), (2048, 2312, 96)]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_every_operand_order_matches_float64(shape):
+    M, N, K = shape
+    for i, (a_mn, b_mn) in enumerate(itertools.product((False, True), repeat=2)):
+        for pad in (0, 3):
+            a, b = _operands(M, N, K, a_mn, b_mn, 10 * i + pad, pad)
+            want = _gemm64(a, b, a_mn, b_mn)
+            got = _planes(a, b, a_mn=a_mn, b_mn=b_mn)
+            assert ((got.double() - want).norm() / want.norm()).item() <= BOUND, (a_mn, b_mn, pad)
+            acc = torch.randn(M, N, device="cuda")
+            both = _planes(a, b, a_mn=a_mn, b_mn=b_mn, out=acc.clone(), accumulate=True, alpha=0.5)
+            want = acc.double() + 0.5 * want
+            assert ((both.double() - want).norm() / want.norm()).item() <= BOUND
+
+
+@pytest.mark.parametrize("scale", [1e-12, 1.0, 1e9])
+def test_sums_of_one_sign_and_far_scales_keep_float32_accuracy(scale):
+    """Sums of positive terms are where a truncating accumulator drifts; rows of very different magnitude are where a
+    common scale would lose bits."""
+    M, N, K = 384, 320, 6000
+    g = torch.Generator().manual_seed(3)
+    a = torch.rand(M, K, generator=g).cuda() * scale
+    a *= torch.logspace(-6, 6, M).cuda()[:, None]
+    b = torch.rand(N, K, generator=g).cuda()
+    want = _gemm64(a, b, False, False)
+    err = ((_planes(a, b).double() - want).abs() / want).max().item()
+    assert err <= 1e-6  # a chain of 6000 float32 FMAs is 5e-6 off on these inputs
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (63, 65, 17), (200, 1000, 40), (129, 257, 100), (2049, 2500, 33)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_fma_kernel_is_one_chain_over_k(shape):
+    """Every output is the chain of fused multiply-adds over k from zero, whatever the tile, the storage order and the
+    alignment: bit for bit the chain formed here in float64 and rounded after every step (exact: a product of two
+    float32 values has 48 bits, its sum with a float32 value is rounded once by a float64 addition only when it needs
+    more than 53, so the inputs are kept to 12 bits)."""
+    M, N, K = shape
+    for i, (a_mn, b_mn) in enumerate(itertools.product((False, True), repeat=2)):
+        for pad in (0, 3):
+            a, b = (t.half().float() for t in _operands(M, N, K, a_mn, b_mn, 20 * i + pad))
+            if pad:  # rows that do not start on 16 bytes
+                a = torch.nn.functional.pad(a, (1, 2))[:, 1:-2]
+                b = torch.nn.functional.pad(b, (1, 2))[:, 1:-2]
+            a64, b64 = (a.double().t() if a_mn else a.double()), (b.double().t() if b_mn else b.double())
+            want = torch.zeros(M, N, device="cuda")
+            for k in range(K):
+                want = (want.double() + a64[:, k, None] * b64[None, :, k]).float()
+            assert torch.equal(_planes(a, b, use=False, a_mn=a_mn, b_mn=b_mn), want), (a_mn, b_mn, pad)
+
+
+def test_infinities_nan_and_huge_values_take_the_fma_kernel():
+    a, b = _operands(300, 290, 260, False, False, 5)
+    for value in (float("inf"), float("-inf"), float("nan"), 1e30, -2e38):
+        x = a.clone()
+        x[17, 31] = value
+        got = _planes(x, b)
+        want = _planes(x, b, use=False)
+        assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
+        acc = _planes(x, b, out=torch.ones_like(want), accumulate=True)
+        assert torch.equal(torch.isnan(acc), torch.isnan(want))
+
+
+def test_shared_planes_and_repeated_runs_give_the_same_bits():
+    from pom_b200 import ops
+
+    a, b = _operands(640, 1152, 700, False, False, 6)
+    w = torch.randn(1152, 640, device="cuda")
+    pl = ops.F32Planes()
+    first, second = _planes(a, b, a_planes=pl), _planes(a, w, a_mn=True, a_planes=pl)
+    assert torch.equal(first, _planes(a, b)) and torch.equal(second, _planes(a, w, a_mn=True))
