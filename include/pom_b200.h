@@ -464,6 +464,12 @@ int pom_heads_mix_bwd(const pom_heads_args* a, void* stream);
  *   h_new[b,:] = (n_past * h_past[b,:] + h_cur[b,:]) / (n_past + 1)        (fp32, B*P elements) */
 int pom_state_merge(const float* h_past, const float* h_cur, float* h_new, float n_past, int64_t count, void* stream);
 
+/* Rows of a (rows, n) mask as a GEMM operand: dst row r starts at dst + r * ld (bf16 or fp32; values past n are not
+ * written) and sums[r] is the fp32 sum of the row as given.  src_kind: bool / unsigned bytes, bf16 or fp32, rows packed. */
+enum { POM_MASK_U8 = 0, POM_MASK_BF16 = 1, POM_MASK_F32 = 2 };
+int pom_mask_rows(const void* src, int32_t src_kind, void* dst, int32_t dst_dtype, float* sums, int64_t rows, int32_t n,
+                  int64_t ld, void* stream);
+
 /* Block-causal aggregate over equal frames: the single-pass form of calling state_forward once per frame
  * (reference pom/pom.py:251-259, where every call weighs equally) and of a block-lower-triangular (B, N, N) mask
  * (pom/pom.py:41-45, 98-99).  in/out (B, F, P) fp32, in = per-frame means.

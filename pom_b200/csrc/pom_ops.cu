@@ -3,11 +3,14 @@
 // backward passes, optional rotary embedding in all of them, and the small
 // reductions that finish the per-tile partial sums of the fused GEMM epilogues.
 //
-// Common traversal: grid = (column blocks, token chunks, batch); one thread owns
-// VEC adjacent channels (16 bytes when alignment allows, plus their rotary
-// partners) and walks the tokens of its chunk four at a time, so every global
-// access is a coalesced 16-byte vector, several are in flight per thread, and every
-// sum is formed in a fixed order (deterministic, no float atomics).
+// Common traversal: grid = (column blocks, 64-token chunks, batch); a block is 32 (or, for few channels, fewer)
+// threads across the channels times 1 to 8 token lanes that share the chunk.  One thread owns VEC adjacent channels
+// (16 bytes when alignment allows, plus their rotary partners) and walks its tokens a few at a time, so every global
+// access is a coalesced 16-byte vector, several are in flight per thread, and every sum is formed in a fixed order
+// (deterministic, no float atomics).
+// Lanes: one keeps a thread's set-up (its coefficients above all) to one per 64 tokens; where that would leave the SMs
+// with a few warps each, more lanes shorten the walk.  Forward sums and causal walks keep one lane at every size: a
+// sample's result has the same bits whatever batch it came in.
 #include "common.cuh"
 #include "gemm_launch.cuh"
 #include "pom_math.cuh"
@@ -85,6 +88,32 @@ struct Vec {
       } else {
         p[0] = __float2bfloat16_rn(v[0]);
       }
+    }
+  }
+};
+
+// VEC values as they were loaded (bf16 stays packed): a walk keeps several tokens of these in flight and unpacks each
+// when its turn comes, at half the registers of unpacked values.
+template <typename T, int VEC>
+struct Raw {
+  static constexpr bool kPacked = std::is_same<T, __nv_bfloat16>::value && VEC == 8;
+  uint4 q;
+  float f[kPacked ? 1 : VEC];
+  __device__ __forceinline__ void ld(const T* __restrict__ p) {
+    if constexpr (kPacked) q = __ldg(reinterpret_cast<const uint4*>(p));
+    else Vec<T, VEC>::ld(p, f);
+  }
+  __device__ __forceinline__ void get(float (&v)[VEC]) const {
+    if constexpr (kPacked) {
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[2 * e] = __uint_as_float(w[e] << 16);
+        v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[e] = f[e];
     }
   }
 };
@@ -183,6 +212,40 @@ __device__ __forceinline__ float poly_grad_reg(float a, const float (&c)[KR]) {
   return r;
 }
 
+constexpr int kWalkThreads = 256;  // most threads of a block
+
+extern __shared__ float walk_sm[];  // blocks of more than one lane: see walk_smem
+
+// The tokens [n0, n1) of this thread in the c-th run of `span` tokens of a sequence of n tokens.
+__device__ __forceinline__ void lane_tokens(int c, int span, int n, bool on, int& n0, int& n1) {
+  const int per = span / blockDim.y;
+  n0 = min(n, c * span + static_cast<int>(threadIdx.y) * per);
+  n1 = on ? min(n, n0 + per) : n0;
+}
+
+// Adds v over the token lanes of the block, in lane order; put(e, sum) runs in one thread per value.  Every thread of
+// the block calls it.
+template <int VEC, class Put>
+__device__ __forceinline__ void sum_lanes(const float (&v)[VEC], bool on, Put put) {
+  const int nx = blockDim.x, ny = blockDim.y, x = threadIdx.x, y = threadIdx.y;
+  if (ny == 1) {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e)
+      if (on) put(e, v[e]);
+    return;
+  }
+  __syncthreads();  // the previous use of the buffer is over
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) walk_sm[(e * ny + y) * nx + x] = v[e];
+  __syncthreads();
+  if (on)
+    for (int e = y; e < VEC; e += ny) {
+      float s = walk_sm[e * ny * nx + x];
+      for (int k = 1; k < ny; ++k) s += walk_sm[(e * ny + k) * nx + x];
+      put(e, s);
+    }
+}
+
 struct AggDev {
   const void* x;
   const float* coeff;
@@ -191,18 +254,21 @@ struct AggDev {
   void* out;
   long long ldx, ld_out, token_offset;
   int B, N, P, K, chunks;
-  int per_token;  // PREFIX kernel only: write each token's own (rotated) features, no running sum
+  int span;  // TOKEN mode: tokens per block
   pom_rope rope;
 };
 
 // ------------------------------------------------------------------ forward: chunk sums / prefix apply
-// PREFIX == false: partial[b, c, :] = sum over the chunk of w * R·poly.
-// PREFIX == true : partial holds the exclusive prefix per chunk; writes out[b, n, :].
-template <typename T, int VEC, int KR, bool PREFIX, bool ROPE>
-__global__ void __launch_bounds__(128) agg_fwd_kernel(const AggDev a) {
+// SUM   : partial[b, c, :] = sum over the chunk of w * R·poly.
+// PREFIX: partial holds the exclusive prefix per chunk; writes out[b, n, :].
+// TOKEN : writes each token's own (rotated) features.
+enum AggMode { kAggSum, kAggPrefix, kAggToken };
+template <typename T, int VEC, int KR, AggMode MODE, bool ROPE>
+__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : KR <= 2 ? 4 : 3) agg_fwd_kernel(const AggDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
   constexpr bool rope = ROPE;
+  constexpr bool PREFIX = MODE != kAggSum, per_token = MODE == kAggToken;
   const ColMap m = map_unit(u, a.P, a.rope.kind);
   if (!m.valid) return;
   Coefs<VEC, KR> cf;
@@ -213,18 +279,20 @@ __global__ void __launch_bounds__(128) agg_fwd_kernel(const AggDev a) {
   float acc1[VEC], acc2[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
-    acc1[e] = (PREFIX && !a.per_token) ? part[m.p1 + e] : 0.f;
-    acc2[e] = (PREFIX && rope && !a.per_token) ? part[m.p2 + e] : 0.f;
+    acc1[e] = (PREFIX && !per_token) ? part[m.p1 + e] : 0.f;
+    acc2[e] = (PREFIX && rope && !per_token) ? part[m.p2 + e] : 0.f;
   }
-  const int n0 = c * kChunk, n1 = min(a.N, n0 + kChunk);
+  int n0, n1;
+  lane_tokens(c, MODE == kAggToken ? a.span : kChunk, a.N, true, n0, n1);
   for (int nb = n0; nb < n1; nb += kTB) {
-    float x1[kTB][VEC], x2[kTB][VEC], cs[kTB][VEC], sn[kTB][VEC], w[kTB];
+    Raw<T, VEC> r1[kTB], r2[kTB];
+    float cs[kTB][VEC], sn[kTB][VEC], w[kTB];
 #pragma unroll
     for (int q = 0; q < kTB; ++q) {
       const int n = min(nb + q, n1 - 1);
-      Vec<T, VEC>::ld(x + n * a.ldx + m.p1, x1[q]);
+      r1[q].ld(x + n * a.ldx + m.p1);
       if (rope) {
-        Vec<T, VEC>::ld(x + n * a.ldx + m.p2, x2[q]);
+        r2[q].ld(x + n * a.ldx + m.p2);
         rope_coeffs<VEC>(a.rope, m, n, cs[q], sn[q]);
       }
       w[q] = (!PREFIX && a.row_weight) ? __ldg(a.row_weight + static_cast<long long>(b) * a.N + n) : 1.f;
@@ -233,15 +301,18 @@ __global__ void __launch_bounds__(128) agg_fwd_kernel(const AggDev a) {
     for (int q = 0; q < kTB; ++q) {
       const int n = nb + q;
       if (n >= n1) break;
-      if (PREFIX && a.per_token) {
+      if (per_token) {
 #pragma unroll
         for (int e = 0; e < VEC; ++e) acc1[e] = acc2[e] = 0.f;
       }
+      float x1[VEC], x2[VEC];
+      r1[q].get(x1);
+      if (rope) r2[q].get(x2);
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
-        const float f1 = poly_reg<KR>(pom_act(x1[q][e]), cf.c1[e]);
+        const float f1 = poly_reg<KR>(pom_act(x1[e]), cf.c1[e]);
         if (rope) {
-          const float f2 = poly_reg<KR>(pom_act(x2[q][e]), cf.c2[e]);
+          const float f2 = poly_reg<KR>(pom_act(x2[e]), cf.c2[e]);
           acc1[e] += w[q] * (f1 * cs[q][e] - f2 * sn[q][e]);
           acc2[e] += w[q] * (f2 * cs[q][e] + f1 * sn[q][e]);
         } else {
@@ -249,7 +320,7 @@ __global__ void __launch_bounds__(128) agg_fwd_kernel(const AggDev a) {
         }
       }
       if (PREFIX) {
-        const float inv = a.per_token ? 1.f : 1.f / static_cast<float>(a.token_offset + n + 1);
+        const float inv = per_token ? 1.f : 1.f / static_cast<float>(a.token_offset + n + 1);
         float o[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) o[e] = acc1[e] * inv;
@@ -301,35 +372,37 @@ __global__ void chunk_scan_kernel(float* partial, const float* carry, float* tot
   if (total) total[static_cast<long long>(b) * P + p] = own;
 }
 
-// out[b, p] = scale * sum_c partial[b, c, p] / denom[b].  Block = 32 columns x 8 chunk lanes; each
-// lane adds every 8th chunk, then the 8 lane sums are combined in lane order.
-__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                                                               const float* __restrict__ denom, float scale, int chunks,
-                                                               int P) {
+// out[b, p] = scale * sum_c partial[b, c, p] / denom[b].  Block = 32 columns x LANES chunk lanes; each lane adds every
+// LANES-th chunk, then the lane sums are combined in lane order.  A latency chain of chunks / LANES loads: 8 lanes up to
+// 64 chunks, 32 above (512 chunks of 2048 channels: 21 us with 8, 9.6 us with 32).
+template <int LANES>
+__global__ void __launch_bounds__(32 * LANES) reduce_partials_kernel(const float* __restrict__ partial,
+                                                                     float* __restrict__ out,
+                                                                     const float* __restrict__ denom, float scale,
+                                                                     int chunks, int P) {
   pomk::griddep_wait();  // launched with programmatic stream serialization
   pomk::griddep_launch();
-  __shared__ float sm[8][33];
+  __shared__ float sm[LANES][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int p = blockIdx.x * 32 + tx;
   const int b = blockIdx.y;
   float s = 0.f;
   if (p < P) {
     const float* base = partial + static_cast<long long>(b) * chunks * P + p;
-    float s0 = 0.f, s1 = 0.f;
+    float t[4] = {0.f, 0.f, 0.f, 0.f};
     int c = ty;
-    for (; c + 8 < chunks; c += 16) {
-      s0 += base[static_cast<long long>(c) * P];
-      s1 += base[static_cast<long long>(c + 8) * P];
-    }
-    if (c < chunks) s0 += base[static_cast<long long>(c) * P];
-    s = s0 + s1;
+    for (; c + 3 * LANES < chunks; c += 4 * LANES)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) t[q] += base[static_cast<long long>(c + q * LANES) * P];
+    for (; c < chunks; c += LANES) t[0] += base[static_cast<long long>(c) * P];
+    s = (t[0] + t[1]) + (t[2] + t[3]);
   }
   sm[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && p < P) {
     float t = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) t += sm[q][tx];
+    for (int q = 0; q < LANES; ++q) t += sm[q][tx];
     t *= scale;
     if (denom) {
       const float d = denom[b];
@@ -337,6 +410,42 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
     }
     out[static_cast<long long>(b) * P + p] = t;
   }
+}
+
+// The same for one column (row sums of a mask): a warp per row, or a block per row of more than 4096 values.
+template <int THREADS>
+__global__ void __launch_bounds__(256) row_sum_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                      const float* __restrict__ denom, float scale, int rows, int n) {
+  pomk::griddep_wait();
+  pomk::griddep_launch();
+  __shared__ float sm[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long row = THREADS == 32 ? blockIdx.x * 8ll + warp : blockIdx.x;
+  if (row >= rows) return;  // whole warps (THREADS == 32); never taken otherwise
+  const int t = THREADS == 32 ? lane : static_cast<int>(threadIdx.x);
+  const float* r = in + row * n;
+  float a[4] = {0.f, 0.f, 0.f, 0.f};
+  int i = t;
+  for (; i + 3 * THREADS < n; i += 4 * THREADS)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] += __ldg(r + i + q * THREADS);
+  for (; i < n; i += THREADS) a[0] += __ldg(r + i);
+  float s = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if constexpr (THREADS > 32) {
+    if (lane == 0) sm[warp] = s;
+    __syncthreads();
+    s = 0.f;
+    for (int w = 0; w < THREADS / 32; ++w) s += sm[w];
+  }
+  if (t != 0) return;
+  s *= scale;
+  if (denom) {
+    const float d = denom[row];
+    s = d != 0.f ? s / d : 0.f;
+  }
+  out[row] = s;
 }
 
 // ------------------------------------------------------------------ backward
@@ -359,15 +468,16 @@ struct AggBwdDev {
 
 // Causal backward, pass 1: partial[b, c, :] = sum over the chunk of dout[b, n, :] / (n + 1 + offset).
 template <typename T, int VEC>
-__global__ void __launch_bounds__(128) causal_bwd_sum_kernel(const AggBwdDev a) {
+__global__ void __launch_bounds__(kWalkThreads) causal_bwd_sum_kernel(const AggBwdDev a) {
   const int p = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  if (p >= a.P) return;
+  const bool on = p < a.P;
+  int n0, n1;
+  lane_tokens(c, kChunk, a.N, on, n0, n1);
   const T* __restrict__ g = static_cast<const T*>(a.dout) + static_cast<long long>(b) * a.N * a.ld_dout + p;
   float acc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) acc[e] = 0.f;
-  const int n0 = c * kChunk, n1 = min(a.N, n0 + kChunk);
   for (int nb = n0; nb < n1; nb += kTB) {
     float v[kTB][VEC];
 #pragma unroll
@@ -381,42 +491,46 @@ __global__ void __launch_bounds__(128) causal_bwd_sum_kernel(const AggBwdDev a) 
     }
   }
   float* part = a.partial + (static_cast<long long>(b) * a.chunks + c) * a.P + p;
-#pragma unroll
-  for (int e = 0; e < VEC; ++e) part[e] = acc[e];
+  sum_lanes<VEC>(acc, on, [&](int e, float v) { part[e] = v; });
 }
 
 // CAUSAL == false: the gradient reaching every token is w[b,n] * dH[b, :].
 // CAUSAL == true : walk the chunk backwards; W[n] = suffix + sum_{m >= n} dout[m]/(m+1+offset).
 // Either way: un-rotate, then dx = g * poly'(a) * act'(x) and the coefficient gradient sums.
 template <typename T, int VEC, int KR, bool CAUSAL, bool ROPE>
-__global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
+__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : 2) agg_bwd_kernel(const AggBwdDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
   constexpr bool rope = ROPE;
   const ColMap m = map_unit(u, a.P, a.rope.kind);
-  if (!m.valid) return;
+  const bool on = m.valid;
   Coefs<VEC, KR> cf;
-  cf.load(a.coeff, m, a.K, rope);
+  if (on) cf.load(a.coeff, m, a.K, rope);
   const T* __restrict__ x = static_cast<const T*>(a.x) + static_cast<long long>(b) * a.N * a.ldx;
   T* __restrict__ dx = static_cast<T*>(a.dx) + static_cast<long long>(b) * a.N * a.ld_dx;
   const T* __restrict__ dout =
       CAUSAL ? static_cast<const T*>(a.dout) + static_cast<long long>(b) * a.N * a.ld_dout : nullptr;
   float g1[VEC], g2[VEC];
   float dc1[VEC][KR], dc2[VEC][KR];
+  int n0, n1;
+  lane_tokens(c, kChunk, a.N, on, n0, n1);
+  const int cnt = n1 - n0;
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
-    if (CAUSAL) {
-      const float* part = a.partial + (static_cast<long long>(b) * a.chunks + c) * a.P;
-      g1[e] = a.per_token ? 0.f : part[m.p1 + e];
-      g2[e] = (rope && !a.per_token) ? part[m.p2 + e] : 0.f;
-    } else {
-      g1[e] = a.dH[static_cast<long long>(b) * a.P + m.p1 + e];
-      g2[e] = rope ? a.dH[static_cast<long long>(b) * a.P + m.p2 + e] : 0.f;
-    }
+    g1[e] = (!CAUSAL && on) ? a.dH[static_cast<long long>(b) * a.P + m.p1 + e] : 0.f;
+    g2[e] = (!CAUSAL && rope && on) ? a.dH[static_cast<long long>(b) * a.P + m.p2 + e] : 0.f;
 #pragma unroll
     for (int i = 0; i < KR; ++i) {
       dc1[e][i] = 0.f;
       dc2[e][i] = 0.f;
+    }
+  }
+  if (CAUSAL && !a.per_token && on) {  // one lane: the walk itself carries the suffix sum
+    const float* part = a.partial + (static_cast<long long>(b) * a.chunks + c) * a.P;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      g1[e] = part[m.p1 + e];
+      g2[e] = rope ? part[m.p2 + e] : 0.f;
     }
   }
   float wb = a.scale;
@@ -424,23 +538,22 @@ __global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
     const float dn = a.denom[b];
     wb = dn != 0.f ? wb / dn : 0.f;
   }
-  const int n0 = c * kChunk, n1 = min(a.N, n0 + kChunk);
-  const int cnt = n1 - n0;
-  constexpr int TBW = !ROPE ? 8 : (CAUSAL && VEC > 2) ? 2 : kTB;  // tokens in flight, as registers allow
+  constexpr int TBW = (ROPE && VEC > 2) || KR > 4 ? 2 : kTB;  // tokens in flight, as registers allow
   for (int ib = 0; ib < cnt; ib += TBW) {
-    float x1[TBW][VEC], x2[TBW][VEC], cs[TBW][VEC], sn[TBW][VEC], go1[TBW][VEC], go2[TBW][VEC], w[TBW];
+    Raw<T, VEC> r1[TBW], r2[TBW], go1[TBW], go2[TBW];
+    float cs[TBW][VEC], sn[TBW][VEC], w[TBW];
 #pragma unroll
     for (int q = 0; q < TBW; ++q) {
       const int i = min(ib + q, cnt - 1);
       const int n = CAUSAL ? (n1 - 1 - i) : (n0 + i);
-      Vec<T, VEC>::ld(x + n * a.ldx + m.p1, x1[q]);
+      r1[q].ld(x + n * a.ldx + m.p1);
       if (rope) {
-        Vec<T, VEC>::ld(x + n * a.ldx + m.p2, x2[q]);
+        r2[q].ld(x + n * a.ldx + m.p2);
         rope_coeffs<VEC>(a.rope, m, n, cs[q], sn[q]);
       }
       if (CAUSAL) {
-        Vec<T, VEC>::ld(dout + n * a.ld_dout + m.p1, go1[q]);
-        if (rope) Vec<T, VEC>::ld(dout + n * a.ld_dout + m.p2, go2[q]);
+        go1[q].ld(dout + n * a.ld_dout + m.p1);
+        if (rope) go2[q].ld(dout + n * a.ld_dout + m.p2);
         w[q] = 1.f;
       } else {
         w[q] = a.row_weight ? wb * __ldg(a.row_weight + static_cast<long long>(b) * a.N + n) : wb;
@@ -451,18 +564,23 @@ __global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
       const int i = ib + q;
       if (i >= cnt) break;
       const int n = CAUSAL ? (n1 - 1 - i) : (n0 + i);
+      float x1[VEC], x2[VEC];
       if (CAUSAL) {
         const float inv = a.per_token ? 1.f : 1.f / static_cast<float>(a.token_offset + n + 1);
+        go1[q].get(x1);
+        if (rope) go2[q].get(x2);
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
-          g1[e] = fmaf(go1[q][e], inv, a.per_token ? 0.f : g1[e]);
-          if (rope) g2[e] = fmaf(go2[q][e], inv, a.per_token ? 0.f : g2[e]);
+          g1[e] = fmaf(x1[e], inv, a.per_token ? 0.f : g1[e]);
+          if (rope) g2[e] = fmaf(x2[e], inv, a.per_token ? 0.f : g2[e]);
         }
       }
       float o1[VEC], o2[VEC];
+      r1[q].get(x1);
+      if (rope) r2[q].get(x2);
       if (!CAUSAL && w[q] == 0.f) {  // a token of weight zero: its saved projection may never have been written
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) x1[q][e] = 0.f, x2[q][e] = 0.f;
+        for (int e = 0; e < VEC; ++e) x1[e] = 0.f, x2[e] = 0.f;
       }
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
@@ -473,8 +591,8 @@ __global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
         } else {
           d1 = w[q] * g1[e];
         }
-        const float av = pom_act(x1[q][e]);
-        o1[e] = d1 * poly_grad_reg<KR>(av, cf.c1[e]) * pom_act_grad(x1[q][e]);
+        const float av = pom_act(x1[e]);
+        o1[e] = d1 * poly_grad_reg<KR>(av, cf.c1[e]) * pom_act_grad(x1[e]);
         float pw = av;
 #pragma unroll
         for (int k = 0; k < KR; ++k) {
@@ -482,8 +600,8 @@ __global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
           pw *= av;
         }
         if (rope) {
-          const float bv = pom_act(x2[q][e]);
-          o2[e] = d2 * poly_grad_reg<KR>(bv, cf.c2[e]) * pom_act_grad(x2[q][e]);
+          const float bv = pom_act(x2[e]);
+          o2[e] = d2 * poly_grad_reg<KR>(bv, cf.c2[e]) * pom_act_grad(x2[e]);
           float pv = bv;
 #pragma unroll
           for (int k = 0; k < KR; ++k) {
@@ -498,13 +616,18 @@ __global__ void __launch_bounds__(128) agg_bwd_kernel(const AggBwdDev a) {
   }
   float* dcp = a.dcoeff_partial + (static_cast<long long>(b) * a.chunks + c) * a.P * a.K;
 #pragma unroll
-  for (int e = 0; e < VEC; ++e)
+  for (int k = 0; k < KR; ++k) {
+    if (k >= a.K) break;
+    float v[VEC];
 #pragma unroll
-    for (int k = 0; k < KR; ++k)
-      if (k < a.K) {
-        dcp[static_cast<long long>(m.p1 + e) * a.K + k] = dc1[e][k];
-        if (rope) dcp[static_cast<long long>(m.p2 + e) * a.K + k] = dc2[e][k];
-      }
+    for (int e = 0; e < VEC; ++e) v[e] = dc1[e][k];
+    sum_lanes<VEC>(v, on, [&](int e, float t) { dcp[static_cast<long long>(m.p1 + e) * a.K + k] = t; });
+    if (rope) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) v[e] = dc2[e][k];
+      sum_lanes<VEC>(v, on, [&](int e, float t) { dcp[static_cast<long long>(m.p2 + e) * a.K + k] = t; });
+    }
+  }
 }
 
 // ------------------------------------------------------------------ streamed backward
@@ -1091,26 +1214,27 @@ struct SelDev {
   void* dh_tok;
   long long ld_z, ld_h, ld_sh, ld_dsh, ld_dz, ld_dh;
   int B, T, P, chunks, h_per_token, activated;
+  int span;  // forward: tokens per block
   const float* row_denom;  // per-token H only: H[b,t,:] is divided by row_denom[b*T + t] (0 -> the row counts as 0)
   pom_rope rope;
 };
 
 template <typename T, int VEC, bool BWD, bool ROPE>
-__global__ void __launch_bounds__(128) select_kernel(const SelDev a) {
+__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_kernel(const SelDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
   constexpr bool rope = ROPE;
   const ColMap m = map_unit(u, a.P, a.rope.kind);
-  if (!m.valid) return;
+  const bool on = m.valid;
   const long long rowb = static_cast<long long>(b) * a.T;
   const T* __restrict__ z = static_cast<const T*>(a.z) + rowb * a.ld_z;
   float b1[VEC], b2[VEC], hb1[VEC], hb2[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
-    b1[e] = a.activated ? 0.f : a.bias[m.p1 + e];
-    b2[e] = (rope && !a.activated) ? a.bias[m.p2 + e] : 0.f;
+    b1[e] = a.activated || !on ? 0.f : a.bias[m.p1 + e];
+    b2[e] = (rope && !a.activated && on) ? a.bias[m.p2 + e] : 0.f;
     hb1[e] = hb2[e] = 0.f;
-    if (!a.h_per_token) {
+    if (!a.h_per_token && on) {
       const float* H = static_cast<const float*>(a.H) + static_cast<long long>(b) * a.P;
       hb1[e] = H[m.p1 + e];
       if (rope) hb2[e] = H[m.p2 + e];
@@ -1119,53 +1243,65 @@ __global__ void __launch_bounds__(128) select_kernel(const SelDev a) {
   float accH1[VEC], accH2[VEC], accB1[VEC], accB2[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) accH1[e] = accH2[e] = accB1[e] = accB2[e] = 0.f;
-  const int t0 = c * kChunk, t1 = min(a.T, t0 + kChunk);
+  int t0, t1;
+  lane_tokens(c, BWD ? kChunk : a.span, a.T, on, t0, t1);
   constexpr int TB = 2;
   for (int tb = t0; tb < t1; tb += TB) {
-    float z1[TB][VEC], z2[TB][VEC], cs[TB][VEC], sn[TB][VEC], h1[TB][VEC], h2[TB][VEC], g1[TB][VEC], g2[TB][VEC];
-    float rs[TB];
+    Raw<T, VEC> rz1[TB], rz2[TB], rh1[TB], rh2[TB], rg1[TB], rg2[TB];
+    float cs[TB][VEC], sn[TB][VEC], rs[TB];
 #pragma unroll
     for (int q = 0; q < TB; ++q) rs[q] = 1.f;
 #pragma unroll
     for (int q = 0; q < TB; ++q) {
       const int t = min(tb + q, t1 - 1);
-      Vec<T, VEC>::ld(z + t * a.ld_z + m.p1, z1[q]);
+      rz1[q].ld(z + t * a.ld_z + m.p1);
       if (rope) {
-        Vec<T, VEC>::ld(z + t * a.ld_z + m.p2, z2[q]);
+        rz2[q].ld(z + t * a.ld_z + m.p2);
         rope_coeffs<VEC>(a.rope, m, t, cs[q], sn[q]);
       }
       if (a.h_per_token) {
         const T* __restrict__ H = static_cast<const T*>(a.H) + (rowb + t) * a.ld_h;
-        Vec<T, VEC>::ld(H + m.p1, h1[q]);
-        if (rope) Vec<T, VEC>::ld(H + m.p2, h2[q]);
+        rh1[q].ld(H + m.p1);
+        if (rope) rh2[q].ld(H + m.p2);
         if (a.row_denom) {
           const float dn = __ldg(a.row_denom + rowb + t);
           rs[q] = dn != 0.f ? 1.f / dn : 0.f;
-#pragma unroll
-          for (int e = 0; e < VEC; ++e) h1[q][e] *= rs[q], h2[q][e] = rope ? h2[q][e] * rs[q] : 0.f;
         }
-      } else {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) h1[q][e] = hb1[e], h2[q][e] = hb2[e];
       }
       if (BWD) {
         const T* __restrict__ dsh = static_cast<const T*>(a.dsh) + (rowb + t) * a.ld_dsh;
-        Vec<T, VEC>::ld(dsh + m.p1, g1[q]);
-        if (rope) Vec<T, VEC>::ld(dsh + m.p2, g2[q]);
+        rg1[q].ld(dsh + m.p1);
+        if (rope) rg2[q].ld(dsh + m.p2);
       }
     }
 #pragma unroll
     for (int q = 0; q < TB; ++q) {
       const int t = tb + q;
       if (t >= t1) break;
+      float z1[VEC], z2[VEC], h1[VEC], h2[VEC], g1[VEC], g2[VEC];
+      rz1[q].get(z1);
+      if (rope) rz2[q].get(z2);
+      if (a.h_per_token) {
+        rh1[q].get(h1);
+        if (rope) rh2[q].get(h2);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) h1[e] *= rs[q], h2[e] = rope ? h2[e] * rs[q] : 0.f;
+      } else {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) h1[e] = hb1[e], h2[e] = hb2[e];
+      }
+      if (BWD) {
+        rg1[q].get(g1);
+        if (rope) rg2[q].get(g2);
+      }
       float s1[VEC], s2[VEC];
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
-        z1[q][e] += b1[e];
-        const float r1 = a.activated ? z1[q][e] : pom_hardsigmoid(z1[q][e]);
+        z1[e] += b1[e];
+        const float r1 = a.activated ? z1[e] : pom_hardsigmoid(z1[e]);
         if (rope) {
-          z2[q][e] += b2[e];
-          const float r2 = a.activated ? z2[q][e] : pom_hardsigmoid(z2[q][e]);
+          z2[e] += b2[e];
+          const float r2 = a.activated ? z2[e] : pom_hardsigmoid(z2[e]);
           s1[e] = r1 * cs[q][e] - r2 * sn[q][e];
           s2[e] = r2 * cs[q][e] + r1 * sn[q][e];
         } else {
@@ -1177,11 +1313,11 @@ __global__ void __launch_bounds__(128) select_kernel(const SelDev a) {
         float o[VEC];
         T* __restrict__ sh = static_cast<T*>(a.sh) + (rowb + t) * a.ld_sh;
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) o[e] = s1[e] * h1[q][e];
+        for (int e = 0; e < VEC; ++e) o[e] = s1[e] * h1[e];
         Vec<T, VEC>::st(sh + m.p1, o);
         if (rope) {
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) o[e] = s2[e] * h2[q][e];
+          for (int e = 0; e < VEC; ++e) o[e] = s2[e] * h2[e];
           Vec<T, VEC>::st(sh + m.p2, o);
         }
       } else {
@@ -1189,21 +1325,21 @@ __global__ void __launch_bounds__(128) select_kernel(const SelDev a) {
         float dh1[VEC], dh2[VEC], o1[VEC], o2[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) {
-          dh1[e] = g1[q][e] * s1[e];
+          dh1[e] = g1[e] * s1[e];
           accH1[e] += dh1[e];
-          const float t1v = g1[q][e] * h1[q][e];  // gradient of the rotated gate
+          const float t1v = g1[e] * h1[e];  // gradient of the rotated gate
           float ds1 = t1v;
           dh2[e] = o2[e] = 0.f;
           if (rope) {
-            dh2[e] = g2[q][e] * s2[e];
+            dh2[e] = g2[e] * s2[e];
             accH2[e] += dh2[e];
-            const float t2v = g2[q][e] * h2[q][e];
+            const float t2v = g2[e] * h2[e];
             ds1 = t1v * cs[q][e] + t2v * sn[q][e];
             const float ds2 = t2v * cs[q][e] - t1v * sn[q][e];
-            o2[e] = a.activated ? ds2 : ds2 * pom_hardsigmoid_grad(z2[q][e]);
+            o2[e] = a.activated ? ds2 : ds2 * pom_hardsigmoid_grad(z2[e]);
             accB2[e] += o2[e];
           }
-          o1[e] = a.activated ? ds1 : ds1 * pom_hardsigmoid_grad(z1[q][e]);
+          o1[e] = a.activated ? ds1 : ds1 * pom_hardsigmoid_grad(z1[e]);
           accB1[e] += o1[e];
         }
         Vec<T, VEC>::st(dz + m.p1, o1);
@@ -1220,14 +1356,11 @@ __global__ void __launch_bounds__(128) select_kernel(const SelDev a) {
   }
   if (BWD) {
     const long long o = (static_cast<long long>(b) * a.chunks + c) * a.P;
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) {
-      a.dbias_partial[o + m.p1 + e] = accB1[e];
-      if (rope) a.dbias_partial[o + m.p2 + e] = accB2[e];
-      if (!a.h_per_token) {
-        a.dh_partial[o + m.p1 + e] = accH1[e];
-        if (rope) a.dh_partial[o + m.p2 + e] = accH2[e];
-      }
+    sum_lanes<VEC>(accB1, on, [&](int e, float v) { a.dbias_partial[o + m.p1 + e] = v; });
+    if (rope) sum_lanes<VEC>(accB2, on, [&](int e, float v) { a.dbias_partial[o + m.p2 + e] = v; });
+    if (!a.h_per_token) {
+      sum_lanes<VEC>(accH1, on, [&](int e, float v) { a.dh_partial[o + m.p1 + e] = v; });
+      if (rope) sum_lanes<VEC>(accH2, on, [&](int e, float v) { a.dh_partial[o + m.p2 + e] = v; });
     }
   }
 }
@@ -1248,19 +1381,20 @@ struct SelHeadsDev {
 };
 
 template <typename T, int VEC, bool BWD>
-__global__ void __launch_bounds__(128) select_heads_kernel(const SelHeadsDev a) {
+__global__ void __launch_bounds__(kWalkThreads) select_heads_kernel(const SelHeadsDev a) {
   const int p = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  if (p >= a.P) return;
+  const bool on = p < a.P;
   const int head = p / a.head_dim;  // VEC divides head_dim, so the thread's channels share one head
   const long long rowb = static_cast<long long>(b) * a.T;
   float hb[VEC], accH[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
-    hb[e] = a.h_per_token ? 0.f : static_cast<const float*>(a.H)[static_cast<long long>(b) * a.P + p + e];
+    hb[e] = a.h_per_token || !on ? 0.f : static_cast<const float*>(a.H)[static_cast<long long>(b) * a.P + p + e];
     accH[e] = 0.f;
   }
-  const int t0 = c * kChunk, t1 = min(a.T, t0 + kChunk);
+  int t0, t1;
+  lane_tokens(c, kChunk, a.T, on, t0, t1);
   constexpr int TB = 4;
   for (int tb = t0; tb < t1; tb += TB) {
     float h[TB][VEC], g[TB][VEC], sv[TB];
@@ -1300,8 +1434,7 @@ __global__ void __launch_bounds__(128) select_heads_kernel(const SelHeadsDev a) 
   }
   if (BWD && !a.h_per_token) {
     float* dst = a.dh_partial + (static_cast<long long>(b) * a.chunks + c) * a.P + p;
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) dst[e] = accH[e];
+    sum_lanes<VEC>(accH, on, [&](int e, float v) { dst[e] = v; });
   }
 }
 
@@ -1321,6 +1454,52 @@ __global__ void tile_weights_kernel(const float* __restrict__ w, float* __restri
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) out[static_cast<long long>(b) * tiles + t] = s;
+}
+
+// Rows of a mask (bool or uint8, bf16, fp32) -> the same values as rows of bf16 or fp32 `ld` apart, and the sum of every
+// row as it was given.  One pass, a warp per row and 8 values per lane and step; 6144 x 1536 bool to bf16: 7 us, where a copy to
+// bf16, one to fp32 and their row sums took 244 us.
+template <typename S>
+__device__ __forceinline__ float mask_value(S v) { return static_cast<float>(v); }
+template <>
+__device__ __forceinline__ float mask_value<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+template <typename S, typename T>
+__global__ void __launch_bounds__(256) mask_rows_kernel(const S* __restrict__ src, T* __restrict__ dst,
+                                                        float* __restrict__ sums, long long rows, int n, long long ld,
+                                                        int vec) {
+  const int lane = threadIdx.x & 31;
+  for (long long row = blockIdx.x * 8ll + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8ll) {
+    const S* s = src + row * n;
+    T* d = dst + row * ld;
+    float acc = 0.f;
+    for (int i = lane * 8; i < n; i += 256) {
+      float v[8];
+      if (vec && i + 8 <= n) {
+        S raw[8];
+        if constexpr (sizeof(S) == 1) *reinterpret_cast<uint2*>(raw) = __ldg(reinterpret_cast<const uint2*>(s + i));
+        else
+#pragma unroll
+          for (int q = 0; q < static_cast<int>(sizeof(S)) / 2; ++q)
+            reinterpret_cast<uint4*>(raw)[q] = __ldg(reinterpret_cast<const uint4*>(s + i) + q);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = mask_value<S>(raw[e]);
+        Vec<T, 8>::st(d + i, v);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          v[e] = i + e < n ? mask_value<S>(s[i + e]) : 0.f;
+          const float one[1] = {v[e]};
+          if (i + e < n) Vec<T, 1>::st(d + i + e, one);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc += v[e];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) sums[row] = acc;
+  }
 }
 
 // Running mean over frames: forward out[b,f,:] = (1/(f+1)) sum_{g<=f} in[b,g,:];
@@ -1402,25 +1581,37 @@ int pick_vec(int P, const pom_rope& rope, int dtype, int K, std::initializer_lis
 }
 
 struct WalkLaunch {
-  dim3 grid;
-  int block;
+  dim3 grid, block;
+  size_t smem;
+  int span;  // tokens per block
 };
 
-WalkLaunch walk_launch(int P, int rope_kind, int vec, int chunks, int B) {
+// 32 threads across the channels (512 bytes of a row at 16 bytes each).  Where one 64-token walk per warp leaves the SMs
+// with fewer than kWalkWarps warps each, the walk is cut: into token lanes of a block if sums are formed over a chunk
+// (kLanes), into blocks of fewer tokens if not (kSpans; blocks of one warp run up to half as fast again as blocks of
+// two to four).  Channels that fill less than 32 threads take fewer threads and more lanes, up to one token per lane.
+// Selection at 4 x 1536 x 2048, forward / backward: 33 / 80 us before, 12 / 27 us with 2 to 4 lanes; at
+// 32 x 1024 x 2304 157 / 263 and 74 / 126 us.
+enum WalkCut { kWhole, kLanes, kSpans };
+constexpr int kWalkWarps = 24;
+WalkLaunch walk_launch(int P, int rope_kind, int vec, int N, int B, WalkCut cut) {
   const int units = static_cast<int>(ceil_div(first_channels(P, rope_kind), vec));
-  // block size: a multiple of 32 up to 128 that wastes the fewest lanes
-  int best = 128;
-  long long best_waste = -1;
-  for (int bs = 128; bs >= 32; bs -= 32) {
-    const long long waste = ceil_div(units, bs) * bs - units;
-    if (best_waste < 0 || waste < best_waste) {
-      best_waste = waste;
-      best = bs;
-    }
-  }
+  const long long warps = ceil_div(units, 32) * ceil_div(N, kChunk) * B;
+  int nx = 32, parts = 1;
+  if (cut != kWhole)
+    while (parts < 8 && warps * parts < 1ll * kWalkWarps * sm_count()) parts *= 2;
   WalkLaunch w;
-  w.block = best;
-  w.grid = dim3(static_cast<unsigned>(ceil_div(units, best)), static_cast<unsigned>(chunks), static_cast<unsigned>(B));
+  int ny = cut == kLanes ? parts : 1;
+  w.span = cut == kSpans ? kChunk / parts : kChunk;
+  if (cut != kWhole && units < 32) {
+    while (nx > 4 && nx / 2 >= units) nx /= 2;
+    ny = kWalkThreads / nx;
+    w.span = kChunk;
+  }
+  w.block = dim3(static_cast<unsigned>(nx), static_cast<unsigned>(ny));
+  w.grid = dim3(static_cast<unsigned>(ceil_div(units, nx)), static_cast<unsigned>(ceil_div(N, w.span)),
+                static_cast<unsigned>(B));
+  w.smem = ny == 1 ? 0 : sizeof(float) * nx * ny * vec;
   return w;
 }
 
@@ -1451,6 +1642,22 @@ WalkLaunch walk_launch(int P, int rope_kind, int vec, int chunks, int B) {
     }                                                                         \
   } while (0)
 
+int launch_reduce(const float* partial, float* out, const float* denom, float scale, int B, int chunks, int P,
+                  cudaStream_t st) {
+  const dim3 grid(static_cast<unsigned>(ceil_div(P, 32)), static_cast<unsigned>(B));
+  if (P == 1 && chunks > 4096)
+    (void)launch_pdl(row_sum_kernel<256>, dim3(B), dim3(256), 0, st, partial, out, denom, scale, B, chunks);
+  else if (P == 1)
+    (void)launch_pdl(row_sum_kernel<32>, dim3(static_cast<unsigned>(ceil_div(B, 8))), dim3(256), 0, st, partial, out,
+                     denom, scale, B, chunks);
+  else if (chunks <= 64)
+    (void)launch_pdl(reduce_partials_kernel<8>, grid, dim3(256), 0, st, partial, out, denom, scale, chunks, P);
+  else
+    (void)launch_pdl(reduce_partials_kernel<32>, grid, dim3(1024), 0, st, partial, out, denom, scale, chunks, P);
+  count_launch();
+  return check_launch();
+}
+
 }  // namespace
 
 // =========================================================================== C ABI
@@ -1463,11 +1670,7 @@ int pom_reduce_partials(const float* partial, float* out, const float* denom, fl
   if (!partial || !out) return POM_ERR_NULL;
   if (B <= 0 || chunks <= 0 || P <= 0) return POM_ERR_BAD_SHAPE;
   if (B > 65535) return POM_ERR_TOO_LARGE;
-  dim3 grid(static_cast<unsigned>(ceil_div(P, 32)), static_cast<unsigned>(B));
-  (void)launch_pdl(reduce_partials_kernel, grid, dim3(256), 0, static_cast<cudaStream_t>(stream), partial, out, denom, scale, chunks,
-                                                                             P);
-  count_launch();
-  return check_launch();
+  return launch_reduce(partial, out, denom, scale, B, chunks, P, static_cast<cudaStream_t>(stream));
 }
 
 int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
@@ -1496,16 +1699,16 @@ int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
   d.P = a->P;
   d.K = a->K;
   d.chunks = pom_agg_chunks(a->N);
-  d.per_token = a->causal == 2;
   d.rope = a->rope;
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx, a->causal ? a->ld_out : 0},
                            {a->x, a->causal ? a->out : nullptr});
-  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, d.chunks, a->B);
+  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 2 ? kSpans : kWhole);
+  d.span = wl.span;
   const bool has_rope = a->rope.kind != POM_ROPE_NONE;
   if (a->causal != 2) {  // per-token features (causal == 2) need neither the sums nor the scan
 #define CALL_SUM(T, V, KR)                                                                    \
-  if (has_rope) agg_fwd_kernel<T, V, KR, false, true><<<wl.grid, wl.block, 0, st>>>(d);        \
-  else agg_fwd_kernel<T, V, KR, false, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) agg_fwd_kernel<T, V, KR, kAggSum, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
+  else agg_fwd_kernel<T, V, KR, kAggSum, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_SUM);
 #undef CALL_SUM
     count_launch();
@@ -1515,11 +1718,19 @@ int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
     chunk_scan_kernel<<<sgrid, 128, 0, st>>>(a->partial, a->carry, a->total, d.chunks, a->P, 0);
     count_launch();
   }
-#define CALL_PFX(T, V, KR)                                                                   \
-  if (has_rope) agg_fwd_kernel<T, V, KR, true, true><<<wl.grid, wl.block, 0, st>>>(d);        \
-  else agg_fwd_kernel<T, V, KR, true, false><<<wl.grid, wl.block, 0, st>>>(d)
-  POM_DISPATCH_K(a->dtype, vec, a->K, CALL_PFX);
+  if (a->causal == 2) {
+#define CALL_TOK(T, V, KR)                                                                            \
+  if (has_rope) agg_fwd_kernel<T, V, KR, kAggToken, true><<<wl.grid, wl.block, wl.smem, st>>>(d);      \
+  else agg_fwd_kernel<T, V, KR, kAggToken, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+    POM_DISPATCH_K(a->dtype, vec, a->K, CALL_TOK);
+#undef CALL_TOK
+  } else {
+#define CALL_PFX(T, V, KR)                                                                            \
+  if (has_rope) agg_fwd_kernel<T, V, KR, kAggPrefix, true><<<wl.grid, wl.block, wl.smem, st>>>(d);     \
+  else agg_fwd_kernel<T, V, KR, kAggPrefix, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+    POM_DISPATCH_K(a->dtype, vec, a->K, CALL_PFX);
 #undef CALL_PFX
+  }
   count_launch();
   return check_launch();
 }
@@ -1583,24 +1794,21 @@ int pom_poly_agg_mean_noalloc(const pom_agg_args* a, const float* denom, float s
   d.P = a->P;
   d.K = a->K;
   d.chunks = chunks;
-  d.per_token = 0;
   d.rope = a->rope;
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx}, {a->x});
-  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, chunks, a->B);
+  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, kWhole);
+  d.span = wl.span;
   const bool has_rope = a->rope.kind != POM_ROPE_NONE;
   // Every (sample, chunk, channel) slot that the reduction below reads is written by this launch first,
   // so nothing left in the workspace by an earlier call can leak into the result.
 #define CALL_NA(T, V, KR)                                                                      \
-  if (has_rope) agg_fwd_kernel<T, V, KR, false, true><<<wl.grid, wl.block, 0, st>>>(d);        \
-  else agg_fwd_kernel<T, V, KR, false, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) agg_fwd_kernel<T, V, KR, kAggSum, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
+  else agg_fwd_kernel<T, V, KR, kAggSum, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
   POM_DISPATCH_K(a->dtype, vec, a->K, CALL_NA);
 #undef CALL_NA
   count_launch();
   if ((rc = check_launch())) return rc;
-  dim3 grid(static_cast<unsigned>(ceil_div(a->P, 32)), static_cast<unsigned>(a->B));
-  (void)launch_pdl(reduce_partials_kernel, grid, dim3(256), 0, st, ws, out, denom, scale, chunks, a->P);
-  count_launch();
-  return check_launch();
+  return launch_reduce(ws, out, denom, scale, a->B, chunks, a->P, st);
 }
 
 int32_t pom_poly_agg_bwd_slots(const pom_agg_bwd_args* a) {
@@ -1720,15 +1928,15 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
   if (a->causal == 3) return POM_ERR_UNSUPPORTED;  // the fused token-causal form exists only as the paired stream
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx, a->ld_dx, a->causal ? a->ld_dout : 0},
                            {a->x, a->dx, a->causal ? a->dout : nullptr});
-  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, d.chunks, a->B);
+  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 1 ? kWhole : kLanes);
   const bool has_rope = a->rope.kind != POM_ROPE_NONE;
   if (a->causal) {
     if (a->causal == 1) {
       // Plain column walk (no channel pairing) for the scaled chunk sums.
       pom_rope none{};
       const int v2 = pick_vec(a->P, none, a->dtype, 1, {a->ld_dout}, {a->dout});
-      const WalkLaunch w1 = walk_launch(a->P, POM_ROPE_NONE, v2, d.chunks, a->B);
-#define CALL_CS(T, V, KR) causal_bwd_sum_kernel<T, V><<<w1.grid, w1.block, 0, st>>>(d)
+      const WalkLaunch w1 = walk_launch(a->P, POM_ROPE_NONE, v2, a->N, a->B, kWhole);
+#define CALL_CS(T, V, KR) causal_bwd_sum_kernel<T, V><<<w1.grid, w1.block, w1.smem, st>>>(d)
       POM_DISPATCH(a->dtype, v2, CALL_CS);
 #undef CALL_CS
       count_launch();
@@ -1738,14 +1946,14 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
       if (a->phase == 1) return check_launch();  // totals only
     }
 #define CALL_BC(T, V, KR)                                                                    \
-  if (has_rope) agg_bwd_kernel<T, V, KR, true, true><<<wl.grid, wl.block, 0, st>>>(d);        \
-  else agg_bwd_kernel<T, V, KR, true, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) agg_bwd_kernel<T, V, KR, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
+  else agg_bwd_kernel<T, V, KR, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BC);
 #undef CALL_BC
   } else {
 #define CALL_BN(T, V, KR)                                                                    \
-  if (has_rope) agg_bwd_kernel<T, V, KR, false, true><<<wl.grid, wl.block, 0, st>>>(d);       \
-  else agg_bwd_kernel<T, V, KR, false, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) agg_bwd_kernel<T, V, KR, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);       \
+  else agg_bwd_kernel<T, V, KR, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BN);
 #undef CALL_BN
   }
@@ -1762,18 +1970,19 @@ static int select_common(SelDev& d, int dtype, bool bwd, std::initializer_list<l
   int rc = check_rope(d.rope, d.P);
   if (rc) return rc;
   const int vec = pick_vec(d.P, d.rope, dtype, 1, lds, ptrs);
-  const WalkLaunch wl = walk_launch(d.P, d.rope.kind, vec, d.chunks, d.B);
+  const WalkLaunch wl = walk_launch(d.P, d.rope.kind, vec, d.T, d.B, bwd ? kLanes : kSpans);
+  d.span = wl.span;
   const bool has_rope = d.rope.kind != POM_ROPE_NONE;
   if (bwd) {
 #define CALL_SB(T, V, KR)                                                          \
-  if (has_rope) select_kernel<T, V, true, true><<<wl.grid, wl.block, 0, st>>>(d);   \
-  else select_kernel<T, V, true, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) select_kernel<T, V, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);   \
+  else select_kernel<T, V, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SB);
 #undef CALL_SB
   } else {
 #define CALL_SF(T, V, KR)                                                          \
-  if (has_rope) select_kernel<T, V, false, true><<<wl.grid, wl.block, 0, st>>>(d);  \
-  else select_kernel<T, V, false, false><<<wl.grid, wl.block, 0, st>>>(d)
+  if (has_rope) select_kernel<T, V, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);  \
+  else select_kernel<T, V, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SF);
 #undef CALL_SF
   }
@@ -1866,14 +2075,14 @@ static int select_heads_common(const pom_select_heads_args* a, bool bwd, void* s
   int vec = pick_vec(d.head_dim, none, a->dtype, 1,
                      {a->h_per_token ? a->ld_h : 0, bwd ? a->ld_dsh : a->ld_sh, (bwd && a->h_per_token) ? a->ld_dh : 0},
                      {a->h_per_token ? a->H : nullptr, bwd ? a->dsh : a->sh, (bwd && a->h_per_token) ? a->dh_tok : nullptr});
-  const WalkLaunch wl = walk_launch(a->P, POM_ROPE_NONE, vec, d.chunks, a->B);
+  const WalkLaunch wl = walk_launch(a->P, POM_ROPE_NONE, vec, a->T, a->B, kLanes);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (bwd) {
-#define CALL_HB(T, V, KR) select_heads_kernel<T, V, true><<<wl.grid, wl.block, 0, st>>>(d)
+#define CALL_HB(T, V, KR) select_heads_kernel<T, V, true><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(a->dtype, vec, CALL_HB);
 #undef CALL_HB
   } else {
-#define CALL_HF(T, V, KR) select_heads_kernel<T, V, false><<<wl.grid, wl.block, 0, st>>>(d)
+#define CALL_HF(T, V, KR) select_heads_kernel<T, V, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(a->dtype, vec, CALL_HF);
 #undef CALL_HF
   }
@@ -1900,6 +2109,32 @@ int pom_tile_weights(const float* w, float* out, int32_t B, int32_t N, void* str
   const int tiles = (N + 127) / 128;
   tile_weights_kernel<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(B)), 32, 0,
                         static_cast<cudaStream_t>(stream)>>>(w, out, N, tiles);
+  count_launch();
+  return check_launch();
+}
+
+int pom_mask_rows(const void* src, int32_t src_kind, void* dst, int32_t dst_dtype, float* sums, int64_t rows, int32_t n,
+                  int64_t ld, void* stream) {
+  if (!src || !dst || !sums) return POM_ERR_NULL;
+  if (rows <= 0 || n <= 0) return POM_ERR_BAD_SHAPE;
+  if (ld < n) return POM_ERR_BAD_STRIDE;
+  if (src_kind < 0 || src_kind > 2 || (dst_dtype != POM_BF16 && dst_dtype != POM_F32)) return POM_ERR_UNSUPPORTED;
+  // 8 values at a time where every row of both matrices keeps the alignment of its vector
+  const int vec = n % 8 == 0 && ld % 8 == 0 && aligned16(src) && aligned16(dst);
+  const int64_t want = ceil_div(rows, 8), cap = 16ll * sm_count();
+  const dim3 grid(static_cast<unsigned>(want < cap ? want : cap));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const auto go = [&](auto* s, auto* d) {
+    mask_rows_kernel<<<grid, 256, 0, st>>>(s, d, sums, static_cast<long long>(rows), static_cast<int>(n),
+                                          static_cast<long long>(ld), vec);
+  };
+  const auto from = [&](auto* d) {
+    if (src_kind == POM_MASK_U8) go(static_cast<const uint8_t*>(src), d);
+    else if (src_kind == POM_MASK_BF16) go(static_cast<const __nv_bfloat16*>(src), d);
+    else go(static_cast<const float*>(src), d);
+  };
+  if (dst_dtype == POM_BF16) from(static_cast<__nv_bfloat16*>(dst));
+  else from(static_cast<float*>(dst));
   count_launch();
   return check_launch();
 }

@@ -225,6 +225,17 @@ def _mask_operand(mask: torch.Tensor, device, dtype) -> torch.Tensor:
     return out
 
 
+def _mask_and_sums(mask: torch.Tensor, device, dtype):
+    """A (B, T, N) mask as a GEMM operand and its (B*T,) fp32 row sums: one kernel for the dtypes it reads, copies and
+    a reduction for the others (integers, fp64)."""
+    mask = mask.to(device=device)
+    if mask.dtype in ops.MASK_KINDS:
+        return ops.mask_rows(mask, dtype)
+    rows = mask.to(torch.float32).contiguous().view(-1, mask.shape[2])
+    sums = torch.cat([ops.reduce_partials(r.unsqueeze(-1)).view(-1) for r in rows.split(32768)])
+    return _mask_operand(mask, device, dtype), sums
+
+
 def _inv_rows(row_sums: torch.Tensor) -> torch.Tensor:
     """1 / row sum of a (B, T, N) mask, 0 where a row is empty (fp32)."""
     return torch.where(row_sums > 0, 1.0 / row_sums, torch.zeros_like(row_sums))
@@ -298,15 +309,11 @@ class _PoMLayer(torch.autograd.Function):
                 raise NotImplementedError("(B, M, N) masks are not combined with token sharding or state")
             if mask.dim() != 3 or mask.shape[0] != B or mask.shape[2] != N or mask.shape[1] != T:
                 raise ValueError(f"expected a (B, T, N) = ({B}, {T}, {N}) mask, got {tuple(mask.shape)}")
-            maskd = _mask_operand(mask, xq.device, xq.dtype)
-            rowden = _row_sums(mask.to(device=xq.device, dtype=torch.float32).contiguous().view(B * T, N))
+            maskd, rowden = _mask_and_sums(mask, xq.device, xq.dtype)
         if spec.mask_kind == "keypad":
             if tuple(mask.shape) != (B, N):
                 raise ValueError(f"expected a (B, N) = ({B}, {N}) mask, got {tuple(mask.shape)}")
             maskf = mask.to(device=xq.device, dtype=torch.float32).contiguous()
-            denom = ops.reduce_partials(maskf.view(B, N, 1)).view(B)
-            if shard is not None:
-                shard.all_reduce(denom)
         # rotary embedding rides in the GEMM epilogues when the positions of every aligned 32-token group are
         # constant or consecutive (RopeSpec.steps) and the degree is at most 4; otherwise on the operator path
         rotary = spec.rope_ctx is not None or spec.rope_qry is not None
@@ -353,6 +360,10 @@ class _PoMLayer(torch.autograd.Function):
                                   None)
             ctx.param_like = (w_qc, se_bias, coeff, w_ag)
             return (y, H.view(B, 1, P)) if spec.want_state else (y, None)
+        if maskf is not None:
+            denom = ops.reduce_partials(maskf.view(B, N, 1)).view(B)
+            if shard is not None:
+                shard.all_reduce(denom)
         # ---------------------------------------------------------------- context phase
         if fused_causal:
             carry, hp, Hc = ops.ctx_gemm(xc, w_po, coeff32, save_hp=need_grad, rope=spec.rope_ctx, causal=True)
@@ -659,16 +670,6 @@ class _PoMLayer(torch.autograd.Function):
         return (dxq, dxc, g_qc, g_bias, g_coeff, g_ag, None, d_hpast, None, dy if ctx.has_residual else None)
 
 
-def _row_sums(m: torch.Tensor) -> torch.Tensor:
-    """Row sums of a (rows, N) fp32 matrix through the partial-sum reduction kernel (grid-limited slices)."""
-    rows, n = m.shape
-    out = torch.empty((rows,), dtype=torch.float32, device=m.device)
-    for lo in range(0, rows, 32768):
-        hi = min(rows, lo + 32768)
-        ops.reduce_partials(m[lo:hi].view(hi - lo, n, 1), out=out[lo:hi].view(hi - lo, 1))
-    return out
-
-
 _ones_cache = {}
 
 
@@ -782,8 +783,7 @@ class _PolyAggFull(torch.autograd.Function):
         if x.stride(-1) != 1 or (B > 1 and x.stride(0) != x.stride(1) * N):
             x = x.contiguous()
         coeff32 = _f32(coeff.contiguous())
-        maskd = _mask_operand(mask, x.device, x.dtype)
-        rowden = _row_sums(mask.to(device=x.device, dtype=torch.float32).contiguous().view(B * M, N))
+        maskd, rowden = _mask_and_sums(mask, x.device, x.dtype)
         feat = ops.poly_agg_fwd(x, coeff32, rope=rope, per_token=True)
         Hc = torch.empty((B, M, P), dtype=x.dtype, device=x.device)
         if x.dtype == torch.bfloat16:

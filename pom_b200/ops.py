@@ -291,9 +291,9 @@ def reduce_partials(partial: torch.Tensor, *, denom: Optional[torch.Tensor] = No
     assert partial.dtype == torch.float32 and partial.is_contiguous()
     if out is None:
         out = torch.empty((B, P), dtype=torch.float32, device=partial.device)
-    # Few samples and many chunks (one long sequence): the kernel's grid is (P/32, B), so first fold groups of
+    # Few samples and very many chunks (one long sequence): the kernel's grid is (P/32, B), so first fold groups of
     # chunks into (B*G, P) with G times as many CTAs, then finish over the G group sums.
-    if chunks >= 128 and B * ((P + 31) // 32) < 256:
+    if P > 1 and chunks >= 1024 and B * ((P + 31) // 32) < 256:
         G = next((g for g in (32, 16, 8, 4) if chunks % g == 0), 0)
         if G:
             part = torch.empty((B * G, P), dtype=torch.float32, device=partial.device)
@@ -789,6 +789,23 @@ def state_merge(h_past: torch.Tensor, h_cur: torch.Tensor, n_past: float) -> tor
     _abi.check(_abi.lib().pom_state_merge(ptr(h_past), ptr(h_cur), ptr(out), float(n_past), h_cur.numel(),
                                           _abi.stream_ptr()), "pom_state_merge")
     return out
+
+
+MASK_KINDS = {torch.bool: 0, torch.uint8: 0, torch.bfloat16: 1, torch.float32: 2}
+
+
+def mask_rows(mask: torch.Tensor, dtype: torch.dtype):
+    """(B, T, N) mask of a dtype in MASK_KINDS -> (the mask in ``dtype`` with rows on 16-byte boundaries, its (B*T,) fp32 row
+    sums).  The row stride is N rounded up to 8 elements; the columns past N belong to nobody."""
+    _require_cuda(mask)
+    B, T, N = mask.shape
+    mask = mask.contiguous()
+    ld = (N + 7) // 8 * 8
+    out = torch.empty((B, T, ld), dtype=dtype, device=mask.device)
+    sums = torch.empty((B * T,), dtype=torch.float32, device=mask.device)
+    _abi.check(_abi.lib().pom_mask_rows(ptr(mask), MASK_KINDS[mask.dtype], ptr(out), _abi.dtype_code(dtype), ptr(sums),
+                                        B * T, N, ld, _abi.stream_ptr()), "pom_mask_rows")
+    return out[..., :N], sums
 
 
 def frame_prefix_mean(h: torch.Tensor, frames: int, adjoint: bool = False) -> torch.Tensor:
