@@ -33,9 +33,19 @@ from .ops import RopeSpec
 
 def eager_only(fn):
     """Keeps ``torch.compile`` out of ``fn``: the library is called through ctypes with raw pointers, which a tracing
-    compiler can neither follow nor fake, so a compiled model runs these calls as they are (a graph break)."""
-    disable = getattr(getattr(torch, "compiler", None), "disable", None)
-    return disable(fn) if disable is not None else fn
+    compiler can neither follow nor fake, so a compiled model runs these calls as they are (a graph break).  A call
+    outside a trace goes straight to ``fn``: the switch that ``torch.compiler.disable`` makes around it costs 6 us."""
+    compiler = getattr(torch, "compiler", None)
+    disable, tracing = getattr(compiler, "disable", None), getattr(compiler, "is_compiling", None)
+    if disable is None or tracing is None:
+        return disable(fn) if disable is not None else fn
+    untraced = disable(fn)
+
+    @functools.wraps(fn)
+    def wrapper(*args, **kwargs):
+        return untraced(*args, **kwargs) if torch.compiler.is_compiling() else fn(*args, **kwargs)
+
+    return wrapper
 
 
 def on_tensor_device(fn):
@@ -45,11 +55,13 @@ def on_tensor_device(fn):
 
     @functools.wraps(fn)
     def wrapper(*args, **kwargs):
-        dev = next((a.device for a in args if torch.is_tensor(a) and a.is_cuda), None)
-        if dev is None or dev.index == torch.cuda.current_device():
-            return fn(*args, **kwargs)
-        with torch.cuda.device(dev):
-            return fn(*args, **kwargs)
+        for a in args:
+            if isinstance(a, torch.Tensor) and a.is_cuda:
+                if a.device.index != torch.cuda.current_device():
+                    with torch.cuda.device(a.device):
+                        return fn(*args, **kwargs)
+                break
+        return fn(*args, **kwargs)
 
     return wrapper
 
@@ -248,25 +260,25 @@ def _like_param(g: torch.Tensor, p: torch.Tensor) -> torch.Tensor:
 
 
 def _check_inputs(xq, xc, w_qc, w_ag, coeff, spec: LayerSpec):
-    if xq.dim() != 3 or xc.dim() != 3:
+    q, c = xq.shape, xc.shape
+    if len(q) != 3 or len(c) != 3:
         raise ValueError("expected (B, T, D) / (B, N, D) inputs")
-    if xq.shape[0] != xc.shape[0]:
-        raise ValueError(f"queries and context differ in batch size: {xq.shape[0]} vs {xc.shape[0]}")
-    if xq.shape[2] != xc.shape[2]:
-        raise ValueError(f"queries and context differ in feature size: {xq.shape[2]} vs {xc.shape[2]}")
-    if spec.mask_kind == "causal" and xq.shape[1] != xc.shape[1]:
+    if q[0] != c[0]:
+        raise ValueError(f"queries and context differ in batch size: {q[0]} vs {c[0]}")
+    if q[2] != c[2]:
+        raise ValueError(f"queries and context differ in feature size: {q[2]} vs {c[2]}")
+    if spec.mask_kind == "causal" and q[1] != c[1]:
         # token m gates with the prefix aggregate of token m (reference pom/pom.py:115 asserts g == t)
-        raise ValueError(f'mask="causal" needs as many query tokens as context tokens, got {xq.shape[1]} and '
-                         f"{xc.shape[1]}")
+        raise ValueError(f'mask="causal" needs as many query tokens as context tokens, got {q[1]} and {c[1]}')
     if coeff.shape[1] > 16:
         raise NotImplementedError(f"polynomial degree {coeff.shape[1]} > 16 is not implemented")
     if not xq.is_cuda:
         raise RuntimeError("pom_b200 has no CPU path: move the module and its inputs to a CUDA device")
-    if xq.dtype not in (torch.bfloat16, torch.float32):
-        raise TypeError(f"unsupported dtype {xq.dtype}; use bfloat16 or float32")
-    for t in (xc, w_qc, w_ag):
-        if t.dtype != xq.dtype:
-            raise TypeError("inputs and projection weights must share one dtype")
+    dt = xq.dtype
+    if dt not in (torch.bfloat16, torch.float32):
+        raise TypeError(f"unsupported dtype {dt}; use bfloat16 or float32")
+    if xc.dtype != dt or w_qc.dtype != dt or w_ag.dtype != dt:
+        raise TypeError("inputs and projection weights must share one dtype")
 
 
 class _PoMLayer(torch.autograd.Function):
@@ -276,7 +288,7 @@ class _PoMLayer(torch.autograd.Function):
 
     @staticmethod
     @on_tensor_device
-    def forward(ctx, xq, xc, w_qc, se_bias, coeff, w_ag, mask, h_past, spec: LayerSpec, residual=None):
+    def forward(ctx, xq, xc, w_qc, se_bias, coeff, w_ag, mask, h_past, spec: LayerSpec, residual=None, track=True):
         _check_inputs(xq, xc, w_qc, w_ag, coeff, spec)
         B, T, D = xq.shape
         N = xc.shape[1]
@@ -293,9 +305,11 @@ class _PoMLayer(torch.autograd.Function):
         xc = xq if spec.self_mixing else xc.contiguous()
         w_qc = w_qc.contiguous()
         w_ag = w_ag.contiguous()
-        w_po, w_se = w_qc[:P], w_qc[P:]
         coeff32, bias32 = _f32_cached(coeff), _f32_cached(se_bias)
-        need_grad = any(ctx.needs_input_grad[:6]) or (h_past is not None and ctx.needs_input_grad[7])
+        # needs_input_grad says which inputs require a gradient, under no_grad too: only `track` (grad mode of the
+        # caller; it is off in here) tells whether a backward pass can come and anything has to be kept for it
+        needs = ctx.needs_input_grad
+        need_grad = track and (True in needs[:6] or (h_past is not None and needs[7]))
         shard = spec.shard
         n_glob = shard.n_global if shard is not None else N
         offset = shard.token_offset if shard is not None else 0
@@ -317,12 +331,12 @@ class _PoMLayer(torch.autograd.Function):
         # rotary embedding rides in the GEMM epilogues when the positions of every aligned 32-token group are
         # constant or consecutive (RopeSpec.steps) and the degree is at most 4; otherwise on the operator path
         rotary = spec.rope_ctx is not None or spec.rope_qry is not None
-        rope_ok = K <= 4 and all(r is None or r.fusable(P) for r in (spec.rope_ctx, spec.rope_qry))
+        rope_ok = not rotary or (K <= 4 and all(r is None or r.fusable(P) for r in (spec.rope_ctx, spec.rope_qry)))
         fused = (bf16 and not heads and (not rotary or rope_ok) and not causal and not full
                  and P % 8 == 0 and D % 8 == 0)
         # token-causal: the prefix means ride in the same epilogues (running sums per 32-token group + a scan over
         # the groups), with or without rotation
-        two_d = any(r is not None and r.kind == _abi.ROPE_2D for r in (spec.rope_ctx, spec.rope_qry))
+        two_d = rotary and any(r is not None and r.kind == _abi.ROPE_2D for r in (spec.rope_ctx, spec.rope_qry))
         fused_causal = (causal and bf16 and not heads and (not rotary or rope_ok) and K <= 4 and D % 8 == 0
                         and P % (64 if two_d else 16) == 0)
 
@@ -347,19 +361,22 @@ class _PoMLayer(torch.autograd.Function):
             out = ops.layer_fwd(
                 xq, None if spec.self_mixing else xc, w_qc, w_ag, bias32, coeff32, mask=maskf, h_past=h_past32,
                 n_past=spec.n_past, residual=None if residual is None else residual.contiguous(), frames=spec.frames,
-                save=need_grad, rope_c=spec.rope_ctx, rope_q=spec.rope_qry, causal=fused_causal, token_offset=offset)
+                save=need_grad, keep_h=need_grad or spec.want_state, rope_c=spec.rope_ctx, rope_q=spec.rope_qry,
+                causal=fused_causal, token_offset=offset)
             y, hp, z, sh, H, denom = out[:6]
             if fused_causal:
                 h_past32 = out[6]  # the running sums `pre` travel in the slot that holds h_past otherwise
-            ctx.has_residual = residual is not None
-            ctx.spec = spec
-            ctx.fused = True
-            ctx.dims = (B, T, N, D, P, K, S, heads, n_glob, offset)
-            ctx.h_past_dtype = None if h_past is None else h_past.dtype
-            ctx.save_for_backward(xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, h_past32, sh, maskf, denom, None, None,
-                                  None)
-            ctx.param_like = (w_qc, se_bias, coeff, w_ag)
+            if track and True in needs:
+                ctx.has_residual = residual is not None
+                ctx.spec = spec
+                ctx.fused = True
+                ctx.dims = (B, T, N, D, P, K, S, heads, n_glob, offset)
+                ctx.h_past_dtype = None if h_past is None else h_past.dtype
+                ctx.save_for_backward(xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, h_past32, sh, maskf, denom, None,
+                                      None, None)
+                ctx.param_like = (w_qc, se_bias, coeff, w_ag)
             return (y, H.view(B, 1, P)) if spec.want_state else (y, None)
+        w_po, w_se = w_qc[:P], w_qc[P:]
         if maskf is not None:
             denom = ops.reduce_partials(maskf.view(B, N, 1)).view(B)
             if shard is not None:
@@ -505,7 +522,8 @@ class _PoMLayer(torch.autograd.Function):
                 g_bias = flat[n_qc + n_ag:n_qc + n_ag + P]
             if p_coeff.dtype == torch.float32:
                 g_coeff = flat[n_qc + n_ag + P:].view(P, K)
-            return (dxq, dxc, g_qc, g_bias, g_coeff, g_ag, None, d_hpast, None, dy if ctx.has_residual else None)
+            return (dxq, dxc, g_qc, g_bias, g_coeff, g_ag, None, d_hpast, None, dy if ctx.has_residual else None,
+                    None)
 
         # one flat fp32 buffer for all parameter gradients: a single zero fill, cast and (when sharded) all-reduce
         n_qc, n_ag = (P + S) * D, D * P
@@ -667,7 +685,8 @@ class _PoMLayer(torch.autograd.Function):
                 d_bias, d_coeff = own[n_qc + n_ag:n_qc + n_ag + S], own[n_qc + n_ag + S:].view(P, K)
             g_qc, g_ag = _like_param(d_wqc, p_qc), _like_param(d_wag, p_ag)
             g_bias, g_coeff = _like_param(d_bias, p_bias), _like_param(d_coeff, p_coeff)
-        return (dxq, dxc, g_qc, g_bias, g_coeff, g_ag, None, d_hpast, None, dy if ctx.has_residual else None)
+        return (dxq, dxc, g_qc, g_bias, g_coeff, g_ag, None, d_hpast, None, dy if ctx.has_residual else None,
+                    None)
 
 
 _ones_cache = {}
@@ -711,9 +730,10 @@ def pom_layer(xq, xc, w_qc, se_bias, coeff, w_ag, mask=None, h_past=None, spec: 
             raise ValueError("BlockCausal needs equal query and context lengths, a multiple of frame_len")
         fold = lambda t: None if t is None else t.contiguous().view(B * F, T // F, t.shape[-1])
         y, h = _PoMLayer.apply(fold(xq), fold(xc) if xc is not None else fold(xq), w_qc, se_bias, coeff, w_ag, None,
-                               None, spec, fold(residual))
+                               None, spec, fold(residual), torch.is_grad_enabled())
         return y.view(B, T, -1), h
-    y, h = _PoMLayer.apply(xq, xc if xc is not None else xq, w_qc, se_bias, coeff, w_ag, mask, h_past, spec, residual)
+    y, h = _PoMLayer.apply(xq, xc if xc is not None else xq, w_qc, se_bias, coeff, w_ag, mask, h_past, spec, residual,
+                           torch.is_grad_enabled())
     return y, h
 
 

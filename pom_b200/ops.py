@@ -7,6 +7,7 @@ module computes on the CPU or with PyTorch operators.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import weakref
 from dataclasses import dataclass
 from typing import Optional, Tuple
@@ -19,16 +20,23 @@ from ._abi import (AggArgs, AggBwdArgs, CtxArgs, GateArgs, GateBwdArgs, GemmArgs
 
 
 def _require_cuda(*tensors) -> torch.device:
-    dev = None
+    index = None
     for t in tensors:
         if t is None:
             continue
-        if not t.is_cuda:
+        i = t.get_device()  # -1 for a CPU tensor; one C call, where is_cuda and device are two and build an object
+        if i < 0:
             raise RuntimeError("pom_b200 runs on CUDA tensors only (no CPU fallback)")
-        dev = dev or t.device
-        if t.device != dev:
+        if index is None:
+            index = i
+        elif i != index:
             raise RuntimeError("all tensors of one call must live on the same GPU")
-    return dev
+    return None if index is None else _device(index)
+
+
+@functools.lru_cache(maxsize=None)
+def _device(index: int) -> torch.device:
+    return torch.device("cuda", index)
 
 
 def _ld(t: torch.Tensor, dim: int) -> int:
@@ -45,17 +53,18 @@ def _row_stride(t: torch.Tensor) -> int:
     """Leading dimension of a 2-D or 3-D tensor whose last dim is contiguous and whose
     leading dims collapse to one row index.  PyTorch leaves the stride of a dimension of size 1 arbitrary (a slice
     of a (B, 1, W) tensor may report any value there), so such a dimension never decides the answer."""
-    if t.stride(-1) != 1:
+    shape, stride = t.shape, t.stride()
+    if stride[-1] != 1:
         raise ValueError("last dimension must be contiguous")
-    if t.dim() == 2:
-        return t.stride(0) if t.shape[0] > 1 else t.shape[1]
-    if t.dim() == 3:
-        B, N = t.shape[0], t.shape[1]
+    if len(shape) == 2:
+        return stride[0] if shape[0] > 1 else shape[1]
+    if len(shape) == 3:
+        B, N = shape[0], shape[1]
         if N == 1:
-            return t.stride(0) if B > 1 else t.shape[2]
-        if B > 1 and t.stride(0) != t.stride(1) * N:
+            return stride[0] if B > 1 else shape[2]
+        if B > 1 and stride[0] != stride[1] * N:
             raise ValueError("batch and token dimensions must collapse to one row stride")
-        return t.stride(1)
+        return stride[1]
     raise ValueError("expected a 2-D or 3-D tensor")
 
 
@@ -136,13 +145,12 @@ def transpose_bf16(src: torch.Tensor) -> torch.Tensor:
     return dst
 
 
+_NO_ROPE = Rope()
+_NO_ROPE.kind, _NO_ROPE.pos_stride = _abi.ROPE_NONE, 1
+
+
 def _rope_c(spec: Optional[RopeSpec]) -> Rope:
-    if spec is None:
-        r = Rope()
-        r.kind = _abi.ROPE_NONE
-        r.pos_stride = 1
-        return r
-    return spec.to_c()
+    return _NO_ROPE if spec is None else spec.to_c()  # assigned by value: never written through
 
 
 # ---------------------------------------------------------------------------- GEMM
@@ -450,38 +458,69 @@ def _layer_args(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, n_past, frames, r
     a.se_bias, a.coeff, a.mask, a.h_past = ptr(bias), ptr(coeff), ptr(mask), ptr(h_past)
     a.rope_c, a.rope_q = _rope_c(rope_c), _rope_c(rope_q)
     a.causal, a.token_offset = int(bool(causal)), int(token_offset)
+    return a, B, T, N, D, P, K
+
+
+def _scratch(a, device, sizes):
+    """One allocation for the call's workspace and the tensors of ``sizes`` bytes that nobody keeps; returns it (alive
+    until the launches are enqueued: the caching allocator then orders its reuse) and the addresses of the tensors."""
     nbytes = int(_abi.lib().pom_layer_workspace_bytes(C.byref(a)))
-    ws = torch.empty((nbytes,), dtype=torch.uint8, device=xq.device)
-    a.workspace, a.workspace_bytes = ptr(ws), nbytes
-    return a, ws
+    a.workspace_bytes = nbytes
+    total = nbytes = (nbytes + 255) & ~255
+    for n in sizes:
+        total += (n + 255) & ~255
+    ws = torch.empty((total,), dtype=torch.uint8, device=device)
+    a.workspace = base = ws.data_ptr()
+    base += nbytes
+    at = []
+    for n in sizes:
+        at.append(base)
+        base += (n + 255) & ~255
+    return ws, at
 
 
 def layer_fwd(xq, xc, w_qc, w_ag, bias, coeff, *, mask=None, h_past=None, n_past=0.0, residual=None, frames=1,
-              save=True, rope_c: Optional[RopeSpec] = None, rope_q: Optional[RopeSpec] = None, causal=False,
+              save=True, keep_h=True, rope_c: Optional[RopeSpec] = None, rope_q: Optional[RopeSpec] = None, causal=False,
               token_offset=0):
     """Whole fused forward (``xc`` None = self-mixing), optionally with rotary embedding of the context features
-    (``rope_c``) and of the gate (``rope_q``).  Returns (y, hp, z, sh, H, denom); hp and z are None unless ``save``;
-    denom is None without a mask.  ``causal``: the token-causal prefix mean; H is then the (B, ceil(N/32), P) group
-    carries and the seventh return value the (B, N, P) bf16 running sums ``pre`` (both needed by :func:`layer_bwd`)."""
+    (``rope_c``) and of the gate (``rope_q``).  Returns (y, hp, z, sh, H, denom); hp, z and sh are None unless ``save``,
+    H unless ``keep_h``; denom is None without a mask.  ``causal``: the token-causal prefix mean; H is then the
+    (B, ceil(N/32), P) group carries and the seventh return value the (B, N, P) bf16 running sums ``pre`` (both needed
+    by :func:`layer_bwd`; pre is None unless ``save``)."""
     dev = _require_cuda(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, residual)
-    a, ws = _layer_args(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, n_past, frames, rope_c, rope_q, causal,
-                        token_offset)
-    B, T, N, D, P = a.B, a.T, a.N, a.D, a.P
-    bf = dict(dtype=torch.bfloat16, device=dev)
-    y, sh = torch.empty((B, T, D), **bf), torch.empty((B, T, P), **bf)
-    hp = torch.empty((B, N, P), **bf) if save else None
-    z = torch.empty((B, T, P), **bf) if save else None
-    denom = torch.empty((B,), dtype=torch.float32, device=dev) if mask is not None else None
-    a.save, a.residual = int(save), ptr(residual)
-    a.y, a.hp, a.z, a.sh, a.denom = ptr(y), ptr(hp), ptr(z), ptr(sh), ptr(denom)
-    pre = None
-    if causal:
-        pre = torch.empty((B, N, P), **bf)
-        H = torch.empty((B, token_groups(N), P), dtype=torch.float32, device=dev)
-        a.pre, a.carry = ptr(pre), ptr(H)
+    a, B, T, N, D, P, K = _layer_args(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, n_past, frames, rope_c, rope_q,
+                                      causal, token_offset)
+    y = torch.empty((B, T, D), dtype=torch.bfloat16, device=dev)
+    hp = z = sh = H = pre = None
+    h_shape = (B, token_groups(N), P) if causal else (B, P)
+    a.save, a.residual, a.y = int(save), ptr(residual), y.data_ptr()
+    if mask is not None:
+        denom = torch.empty((B,), dtype=torch.float32, device=dev)
+        a.denom = denom.data_ptr()
     else:
-        H = torch.empty((B, P), dtype=torch.float32, device=dev)
-        a.H = ptr(H)
+        denom = None
+    drop = []  # (field, bytes) of what this call's caller does not keep
+    if save:
+        hp = torch.empty((B, N, P), dtype=torch.bfloat16, device=dev)
+        z = torch.empty((B, T, P), dtype=torch.bfloat16, device=dev)
+        sh = torch.empty((B, T, P), dtype=torch.bfloat16, device=dev)
+        a.hp, a.z, a.sh = hp.data_ptr(), z.data_ptr(), sh.data_ptr()
+        if causal:
+            pre = torch.empty((B, N, P), dtype=torch.bfloat16, device=dev)
+            a.pre = pre.data_ptr()
+    else:
+        drop.append(("sh", 2 * B * T * P))
+        if causal:
+            drop.append(("pre", 2 * B * N * P))
+    h_field = "carry" if causal else "H"
+    if keep_h:
+        H = torch.empty(h_shape, dtype=torch.float32, device=dev)
+        setattr(a, h_field, H.data_ptr())
+    else:
+        drop.append((h_field, 4 * h_shape[0] * h_shape[1] * (P if causal else 1)))
+    ws, at = _scratch(a, dev, [n for _, n in drop])
+    for (field, _), address in zip(drop, at):
+        setattr(a, field, address)
     _abi.check(_abi.lib().pom_layer_fwd(C.byref(a), ptr(_abi.status_word(dev)), _abi.stream_ptr()), "pom_layer_fwd")
     if causal:
         return y, hp, z, sh, H, denom, pre
@@ -497,14 +536,13 @@ def layer_bwd(dy, xq, xc, w_qc, w_ag, bias, coeff, hp, z, sh, H, *, mask=None, d
     weight ``w_ag_t`` (P, D) is required; ``causal`` = the running sums ``pre`` of the forward call, whose carries
     come in ``H``.  The flat buffer is zero-filled by the call."""
     dev = _require_cuda(dy, xq, xc, w_qc, w_ag, bias, coeff, hp, z, sh, H, mask, denom, h_past, dh_state, w_ag_t, causal)
-    a, ws = _layer_args(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, n_past, frames, rope_c, rope_q,
-                        causal is not None, token_offset)
+    a, B, T, N, D, P, K = _layer_args(xq, xc, w_qc, w_ag, bias, coeff, mask, h_past, n_past, frames, rope_c, rope_q,
+                                      causal is not None, token_offset)
     a.w_ag_t = ptr(w_ag_t)
-    B, T, N, D, P, K = a.B, a.T, a.N, a.D, a.P, a.K
-    bf = dict(dtype=torch.bfloat16, device=dev)
-    G = torch.empty((B * T * 2 * P if xc is None else (B * N + B * T) * P,), **bf)
-    dxq = torch.empty((B, T, D), **bf)
-    dxc = None if xc is None else torch.empty((B, N, D), **bf)
+    # G = [dhp | dz] lives as long as the call
+    ws, (a.G,) = _scratch(a, dev, [2 * (B * T * 2 * P if xc is None else (B * N + B * T) * P)])
+    dxq = torch.empty((B, T, D), dtype=torch.bfloat16, device=dev)
+    dxc = None if xc is None else torch.empty((B, N, D), dtype=torch.bfloat16, device=dev)
     n_flat = 2 * P * D + D * P + P + P * K
     flat = flat_out  # ``flat_out``: caller-owned fp32 accumulators (e.g. the gradient region of a peer exchange)
     if flat is None:
@@ -517,7 +555,7 @@ def layer_bwd(dy, xq, xc, w_qc, w_ag, bias, coeff, hp, z, sh, H, *, mask=None, d
         a.pre, a.carry = ptr(causal), ptr(H)
     else:
         a.H = ptr(H)
-    a.dy, a.dh_state, a.G, a.dxq, a.dxc = ptr(dy), ptr(dh_state), ptr(G), ptr(dxq), ptr(dxc)
+    a.dy, a.dh_state, a.dxq, a.dxc = ptr(dy), ptr(dh_state), ptr(dxq), ptr(dxc)
     a.grads, a.d_hpast = ptr(flat), ptr(d_hpast)
     _abi.check(_abi.lib().pom_layer_bwd(C.byref(a), ptr(_abi.status_word(dev)), _abi.stream_ptr()), "pom_layer_bwd")
     return dxq, dxc, flat, d_hpast

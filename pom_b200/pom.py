@@ -20,6 +20,10 @@ from .functional import polynomial_aggregation_, polynomial_selection_, pom  # n
 from .operators import pom_activation  # noqa: F401
 
 
+# True while autocast is active for any device type (one C call; the CUDA-specific queries follow only then)
+_any_autocast = getattr(torch._C, "_is_any_autocast_enabled", lambda: True)
+
+
 class PoM(nn.Module):
     """Polynomial Mixer layer.
 
@@ -99,8 +103,10 @@ class PoM(nn.Module):
     def _cast(self, t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
         """A token tensor or projection weight in the autocast dtype (unchanged outside autocast).  The cast of a
         weight that needs no gradient is kept until the weight changes."""
+        if t is None or not _any_autocast():
+            return t
         dt = self._autocast_dtype()
-        if t is None or dt is None or t.dtype == dt or not t.is_floating_point():
+        if dt is None or t.dtype == dt or not t.is_floating_point():
             return t
         if isinstance(t, nn.Parameter) and not (torch.is_grad_enabled() and t.requires_grad):
             return _derived_of(t, "autocast", lambda w: w.detach().to(dt))
@@ -112,8 +118,10 @@ class PoM(nn.Module):
         of the gate weight (and bias, and rotary column) r times: r * heads heads of head_dim / r channels gate
         exactly as heads heads of head_dim channels, and autograd sums the copies' gradients."""
         h = self.n_sel_heads
+        if h <= 1:
+            return 1
         ws = self.qc_proj.weight if self.n_groups == 1 else self.se_proj.weight
-        if h <= 1 or (self._autocast_dtype() or ws.dtype) != torch.bfloat16 or h % 8 == 0:
+        if (self._autocast_dtype() or ws.dtype) != torch.bfloat16 or h % 8 == 0:
             return 1
         r = 8 // math.gcd(h, 8)
         if self._po_dim % (h * r):
