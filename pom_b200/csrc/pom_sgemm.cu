@@ -5,8 +5,8 @@
 // of the result.  It does not depend on the tile, the batch or the operands' storage order.  Small products and those
 // that the three-plane form (pom_gemm_f32.cu) cannot carry come here too.
 //
-// What bounds it: FMA issue (74 TFLOP/s at 1.965 GHz; 38 to 45 reached at 4080 x 4608 x 1152, 22 with the 4 x 4
-// outputs per thread and single buffer it had before).  A thread keeps TM x TN outputs, so that 4 (or 3) shared-memory
+// What bounds it: FMA issue (74 TFLOP/s at 1.965 GHz; 48 reached at 4080 x 4608 x 1152, 22 with the 4 x 4
+// outputs per thread and single buffer it had before; 8 x 16 outputs at one block per SM reach 47, scalar FMAs 44).  A thread keeps TM x TN outputs, so that 4 (or 3) shared-memory
 // reads feed 64 (or 32) FMAs; the next k-step is loaded into registers while the current one is computed from a
 // double-buffered tile, one barrier per step.
 #include "common.cuh"
@@ -27,8 +27,9 @@ struct SgemmOperand {
   int vec;   // 16-byte loads are possible (base and leading dimension)
 };
 
-// This thread's share of a TILE x kStep block: TILE * kStep / NT values.  K-major: runs of adjacent k of one row, lanes
-// on adjacent rows (whole 32-byte sectors, conflict-free transposed stores); MN-major: 16-byte pieces of a k-row.
+// This thread's share of a TILE x kStep block: TILE * kStep / NT values in 16-byte pieces.  K-major: four lanes take the
+// 64 bytes of a row and store them transposed (rows of TILE + 4 floats: two-way bank conflicts); MN-major: pieces of a
+// k-row.
 template <int TILE, int NT>
 struct BlockLoader {
   static constexpr int kValues = TILE * kStep / NT;  // 4 or 8
@@ -40,7 +41,7 @@ struct BlockLoader {
     for (int j = 0; j < kPieces; ++j) {
       int r, k;
       if (!o.mn) {
-        r = tid % TILE, k = (tid / TILE) * kValues + j * 4;
+        r = tid / 4 + j * (NT / 4), k = (tid % 4) * 4;
       } else {
         const int piece = tid + j * NT;
         r = (piece % (TILE / 4)) * 4, k = piece / (TILE / 4);
@@ -63,11 +64,11 @@ struct BlockLoader {
       v[j] = x;
     }
   }
-  __device__ __forceinline__ void store(float (*s)[TILE], int mn, int tid) const {
+  __device__ __forceinline__ void store(float (*s)[TILE + 4], int mn, int tid) const {
 #pragma unroll
     for (int j = 0; j < kPieces; ++j) {
       if (!mn) {
-        const int r = tid % TILE, k = (tid / TILE) * kValues + j * 4;
+        const int r = tid / 4 + j * (NT / 4), k = (tid % 4) * 4;
         s[k][r] = v[j].x, s[k + 1][r] = v[j].y, s[k + 2][r] = v[j].z, s[k + 3][r] = v[j].w;
       } else {
         const int piece = tid + j * NT;
@@ -93,8 +94,8 @@ sgemm_kernel(const SgemmOperand A, const SgemmOperand Bm, float* __restrict__ C,
              int accumulate, const SgemmFlags flags) {
   constexpr int kCols = TILE / 8;  // threads along n
   static_assert(NT == kCols * (TILE / TM), "thread layout");
-  __shared__ __align__(16) float As[2][kStep][TILE];
-  __shared__ __align__(16) float Bs[2][kStep][TILE];
+  __shared__ __align__(16) float As[2][kStep][TILE + 4];
+  __shared__ __align__(16) float Bs[2][kStep][TILE + 4];
   const int tid = threadIdx.x, tx = tid % kCols, ty = tid / kCols;
   griddep_wait();
   griddep_launch();
