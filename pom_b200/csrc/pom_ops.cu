@@ -390,11 +390,10 @@ __global__ void __launch_bounds__(32 * LANES) reduce_partials_kernel(const float
   if (p < P) {
     const float* base = partial + static_cast<long long>(b) * chunks * P + p;
     float t[4] = {0.f, 0.f, 0.f, 0.f};
-    int c = ty;
-    for (; c + 3 * LANES < chunks; c += 4 * LANES)
+    for (int c = ty; c < chunks; c += 4 * LANES)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) t[q] += base[static_cast<long long>(c + q * LANES) * P];
-    for (; c < chunks; c += LANES) t[0] += base[static_cast<long long>(c) * P];
+      for (int q = 0; q < 4; ++q)
+        if (c + q * LANES < chunks) t[q] += base[static_cast<long long>(c + q * LANES) * P];
     s = (t[0] + t[1]) + (t[2] + t[3]);
   }
   sm[ty][tx] = s;
