@@ -83,11 +83,16 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16_m256(int bn, bool a_mn_ma
          (static_cast<uint32_t>(256 >> 4) << 24);
 }
 
-// Work unit -> the tile of THIS CTA (rank r takes the r-th 128-row half of the 256-row pair tile).
-// A pair may hang over the end of a batch: then rows_valid is 0 and the tile contributes nothing.
+// Work unit -> the tile of THIS CTA.  A pair is two consecutive 128-row tiles of the whole problem, which may belong to
+// different batches: each CTA loads its own rows of A and keeps its own accumulator, only the B tile is shared.  (With
+// one B matrix per batch the pair stays inside its batch and may hang over its end.)  The odd tile at the end of the
+// problem, or of such a batch, has rows_valid = 0 and contributes nothing.  32 samples of 576 rows are 80 pairs, not 96
+// (rotary context phase, D = 1152, P = 2304: 123 -> 106 us).
+__device__ __forceinline__ int pairs_of(const GemmGeom& g) {
+  return g.b_batched ? g.batches * ((g.m_tiles_per_batch + 1) >> 1) : (g.batches * g.m_tiles_per_batch + 1) >> 1;
+}
 __device__ __forceinline__ TileCtx decode_pair_tile(const GemmGeom& g, int unit, int bn, int rank) {
-  const int pairs_per_batch = (g.m_tiles_per_batch + 1) >> 1;
-  const int pairs_m = g.batches * pairs_per_batch;
+  const int pairs_m = pairs_of(g);
   const int per_split = pairs_m * g.n_tiles;
   TileCtx t;
   t.split = unit / per_split;
@@ -100,18 +105,31 @@ __device__ __forceinline__ TileCtx decode_pair_tile(const GemmGeom& g, int unit,
   const int band_rows = min(gm, pairs_m - m_lo);
   const int n = in_band / band_rows;
   const int mp = m_lo + (in_band - n * band_rows);
-  t.b = mp / pairs_per_batch;
-  t.mt = 2 * (mp - t.b * pairs_per_batch) + rank;
+  const int tiles_m = g.batches * g.m_tiles_per_batch;
+  int m0 = 2 * mp, m1 = m0 + 1;  // the pair's tiles, counted over all batches
+  bool second = m1 < tiles_m;
+  if (g.b_batched) {
+    const int per_batch = (g.m_tiles_per_batch + 1) >> 1;
+    const int b = mp / per_batch, mt = 2 * (mp - b * per_batch);
+    m0 = b * g.m_tiles_per_batch + mt;
+    m1 = m0 + 1;
+    second = mt + 1 < g.m_tiles_per_batch;
+  }
+  if (rank == 0 || second) {
+    const int m = rank == 0 ? m0 : m1;
+    t.b = m / g.m_tiles_per_batch;
+    t.mt = m - t.b * g.m_tiles_per_batch;
+  } else {  // a tile past the end of the batch of the pair's first tile: its rows are zero-filled
+    t.b = m0 / g.m_tiles_per_batch;
+    t.mt = g.m_tiles_per_batch;
+  }
   t.row0 = t.mt * kBM;
   t.rows_valid = max(0, min(kBM, g.rows_per_batch - t.row0));
   set_tile_cols(g, t, n, bn);
   // the two halves of a pair share one main loop: it is skipped only when both are empty
   t.live = true;
-  if (g.tile_weight) {
-    const int m0 = t.b * g.m_tiles_per_batch + 2 * (mp - t.b * pairs_per_batch);
-    const bool second = 2 * (mp - t.b * pairs_per_batch) + 1 < g.m_tiles_per_batch;
-    t.live = __ldg(g.tile_weight + m0) != 0.f || (second && __ldg(g.tile_weight + m0 + 1) != 0.f);
-  }
+  if (g.tile_weight)
+    t.live = __ldg(g.tile_weight + m0) != 0.f || (second && __ldg(g.tile_weight + m1) != 0.f);
   return t;
 }
 
@@ -188,8 +206,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   griddep_wait();
   griddep_launch();
 
-  const int pairs_per_batch = (geom.m_tiles_per_batch + 1) >> 1;
-  const int total_units = geom.batches * pairs_per_batch * geom.n_tiles * geom.split_k;
+  const int total_units = pairs_of(geom) * geom.n_tiles * geom.split_k;
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
 

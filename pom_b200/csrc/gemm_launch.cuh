@@ -258,6 +258,12 @@ int launch(const Operands& o, int split_k, const EpiMaps& maps, const typename E
   return launch_overlapped(kern, grid, smem, st, tmA, tmB, maps, g, ep, status);
 }
 
+// Pairs of 128-row tiles (decode_pair_tile): of the whole problem, or of every batch where each has its own B matrix.
+inline long long pair_rows(const Operands& o) {
+  const long long mt = ceil_div(o.M, kBM);
+  return o.b_batched ? o.batches * ((mt + 1) / 2) : (o.batches * mt + 1) / 2;
+}
+
 // Two CTAs (one cluster) per 256 x BN tile; each CTA loads BN/2 rows of the B tile.
 template <int BN, int STAGES, bool A_MN, bool B_MN, class Epi>
 int launch_pair(const Operands& o, int split_k, const EpiMaps& maps, const typename Epi::Params& ep, int* status,
@@ -270,7 +276,7 @@ int launch_pair(const Operands& o, int split_k, const EpiMaps& maps, const typen
   auto kern = gemm_tcgen05_2cta_kernel<BN, STAGES, A_MN, B_MN, Epi>;
   static std::atomic<uint64_t> attr_set{0};
   if ((rc = set_smem_once(kern, smem, &attr_set))) return rc;
-  const long long units = 1ll * g.batches * ((g.m_tiles_per_batch + 1) / 2) * g.n_tiles * g.split_k;
+  const long long units = pair_rows(o) * g.n_tiles * g.split_k;
   if (units > INT32_MAX) return POM_ERR_TOO_LARGE;
   int clusters = static_cast<int>(units < sm_count() / 2 ? units : sm_count() / 2);
   if constexpr (Epi::kStager) {
@@ -301,7 +307,7 @@ inline TilePlan pick_plan(const Operands& o, bool allow_192, bool splittable = f
   const int knob = g_gemm_mode.load(std::memory_order_relaxed) % 100;
   const int mode = knob % 10;
   const int force_bn = knob / 10 == 1 ? 128 : knob / 10 == 2 ? 192 : knob / 10 == 3 ? 256 : 0;
-  const long long m_tiles = 1ll * o.batches * ceil_div(o.M, kBM);
+  const long long m_tiles = 1ll * o.batches * ceil_div(o.M, kBM), m_pairs = pair_rows(o);
   TilePlan best{false, 128};
   double best_cost = -1.0;
   for (int pair = 1; pair >= 0; --pair) {
@@ -314,7 +320,7 @@ inline TilePlan pick_plan(const Operands& o, bool allow_192, bool splittable = f
       if (o.N <= 128 && bn != 128) continue;
       if (force_bn && bn != force_bn && !(force_bn == 192 && !has_192)) continue;
       const long long n_tiles = o.pair_q ? ceil_div(1ll * o.pair_sections * o.pair_q, bn / 2) : ceil_div(o.N, bn);
-      const long long units = (pair ? (m_tiles + 1) / 2 : m_tiles) * n_tiles;
+      const long long units = (pair ? m_pairs : m_tiles) * n_tiles;
       const int slots = pair ? sm_count() / 2 : sm_count();
       // split-K products fill the last wave with K slices (pick_split): their cost is the work itself (an odd row
       // of tiles that leaves half a pair empty is not charged either: the split spreads it)
@@ -350,9 +356,8 @@ inline int pick_split(long long units, long long kblocks, int slots) {
 }
 
 inline long long plan_units(const Operands& o, const TilePlan& p) {
-  const long long mt = ceil_div(o.M, kBM);
   const long long nt = o.pair_q ? ceil_div(1ll * o.pair_sections * o.pair_q, p.bn / 2) : ceil_div(o.N, p.bn);
-  return 1ll * o.batches * (p.pair ? (mt + 1) / 2 : mt) * nt;
+  return (p.pair ? pair_rows(o) : o.batches * ceil_div(o.M, kBM)) * nt;
 }
 
 // Pipeline depth: as many stages as fit beside the epilogue staging area and scratch in the

@@ -162,7 +162,7 @@ gemm_f32_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   griddep_wait();
   griddep_launch();
 
-  const int total_units = ((geom.m_tiles_per_batch + 1) >> 1) * geom.n_tiles * geom.split_k;
+  const int total_units = pairs_of(geom) * geom.n_tiles * geom.split_k;
   const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
 
   if (warp == 0) {
