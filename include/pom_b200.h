@@ -69,10 +69,10 @@ long long pom_launch_count(void);
  * no clamp).
  * step0 / step1 describe the positions that section 0 (1-D, or the row half of 2-D) and section 1 (the
  * column half) use, per aligned group of 32 tokens:  0 = the tokens of a group share one position,
- * 1 = they hold consecutive positions (base, base + 1, ...), -1 = anything else.  The stand-alone
- * operators ignore it; the fused tensor-core phases (pom_ctx_gemm, pom_gate_gemm, pom_gate_bwd_gemm)
- * need 0 or 1 (they build every token's angle from its group's base angle and a lane offset) and return
- * POM_ERR_UNSUPPORTED otherwise.  pom_rope_pos_info computes both from the positions.
+ * 1 = they hold consecutive positions (base, base + 1, ...), 2 = their positions are at most 61 apart,
+ * -1 = anything else.  The stand-alone operators take any positions; the fused tensor-core phases
+ * (pom_ctx_gemm, pom_gate_gemm, pom_gate_bwd_gemm) need 0, 1 or 2 (token-causal: 0 or 1; they build every token's
+ * angle from its group's base angle and an offset of at most 31 either way) and return POM_ERR_UNSUPPORTED otherwise.  pom_rope_pos_info computes both from the positions.
  * ------------------------------------------------------------------------------------------ */
 typedef struct pom_rope {
   int32_t kind; /* POM_ROPE_* */
@@ -88,7 +88,8 @@ typedef struct pom_rope {
 
 /* Scans positions (n, pos_stride) int64 on the device and writes, for column c of the positions (c = 0, 1;
  * only c = 0 when pos_stride == 1), info[4c + 0] = min, info[4c + 1] = max, info[4c + 2] = 1 when every aligned
- * 32-token group is constant, info[4c + 3] = 1 when every aligned 32-token group is consecutive.  info is 8 int64
+ * 32-token group is constant, info[4c + 3] = 1 when every aligned 32-token group is consecutive, else 2 when the positions
+ * of every aligned 32-token group are at most 61 apart, else 0.  info is 8 int64
  * in device memory; the call only enqueues work.  (Host helper of the rotary epilogues: no reference counterpart,
  * the reference indexes its tables with the positions directly, pom/pom_rope.py:171-172.) */
 int pom_rope_pos_info(const int64_t* pos, int64_t n, int32_t pos_stride, int64_t* info, void* stream);
@@ -160,7 +161,7 @@ int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, voi
  * 128-token tile.  partial is (B * ceil(N/128), P) fp32; reduce it with pom_reduce_partials.
  * With rope.kind != POM_ROPE_NONE the polynomial features of every token are rotated by its position before
  * the reduction (reference pom/pom_rope.py:513-515, pom_triton_rope.py:93-217): needs K <= 4, P % 16 == 0
- * (1-D) or P % 64 == 0 (2-D) and rope.step0/1 in {0, 1}; otherwise POM_ERR_UNSUPPORTED (use pom_poly_agg_fwd).
+ * (1-D) or P % 64 == 0 (2-D) and rope.step0/1 in {0, 1, 2}; otherwise POM_ERR_UNSUPPORTED (use pom_poly_agg_fwd).
  * Replaces: pom/pom.py:205-206 + pom/pom.py:83-91 / 35-38 (and pom_triton.py:68-153).
  * ------------------------------------------------------------------------------------------ */
 typedef struct pom_ctx_args {

@@ -131,7 +131,7 @@ struct EpiCtxCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
   }
   template <int BN>
   static __device__ __forceinline__ void prologue(const Params&, const EpiMaps&, const GemmGeom&, const TileCtx&, int,
@@ -140,7 +140,7 @@ struct EpiCtxCausal {
   template <int KT, int BN>
   static __device__ __forceinline__ void body(const Params& p, const EpiMaps& maps, const GemmGeom& g,
                                               const TileCtx& t, uint32_t tmem_acc, int quarter, int lane, int half,
-                                              const float* cst, const RopeView& rs, EpiIO& io) {
+                                              const float* cst, const RopeView<false>& rs, EpiIO& io) {
     const int y = t.row0 + quarter * 32;
     const int grp = (t.row0 >> 5) + quarter;
     const bool grp_ok = grp < p.causal.groups && t.rows_valid > 0;
@@ -150,7 +150,7 @@ struct EpiCtxCausal {
     for (int su = half; su < BN / 32; su += kEpiColSplit) {
       const PairPos pp = pair_pos(g, t, 16 * su);
       if (!pp.ok) break;  // warp-uniform
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       float v[32];
       tmem_ld16<0>(tmem_acc + 16 * su, v);
       tmem_ld16<16>(tmem_acc + BN / 2 + 16 * su, v);
@@ -165,7 +165,7 @@ struct EpiCtxCausal {
         for (int e = 0; e < 4; ++e) a1[e] = act_fast(v[i + e]), a2[e] = act_fast(v[16 + i + e]);
         poly4<KT, BN>(cst + 16 * su + i, p.K, a1, f1);
         poly4<KT, BN>(cst + BN / 2 + 16 * su + i, p.K, a2, f2);
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           v[i + e] = f1[e] * c[e] - f2[e] * s[e];
@@ -206,7 +206,7 @@ struct EpiCtxCausal {
     const Scratch<BN> sc(scratch);
     const int slot = iter & 1;
     const float* cst = sc.cols();
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<false> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     switch (p.K) {
       case 1: body<1, BN>(p, maps, g, t, tmem_acc, quarter, lane, half, cst, rs, io); break;
       case 2: body<2, BN>(p, maps, g, t, tmem_acc, quarter, lane, half, cst, rs, io); break;
@@ -258,7 +258,7 @@ struct EpiGateCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_carry<BN>(sc.tile(slot), p.causal, g, t, lane);
   }
   // Each warp starts the load of its first `pre` blocks while the tile's main loop is still running.
@@ -279,7 +279,7 @@ struct EpiGateCausal {
     const int slot = iter & 1;
     const float* bias = sc.cols();
     const float* carry = sc.tile(slot) + quarter * BN;
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<false> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     const int y = t.row0 + quarter * 32;
     const float inv_n = 1.f / static_cast<float>(p.causal.token_offset + y + lane + 1);
     uint8_t* out = io.buf0 + 4096;
@@ -289,7 +289,7 @@ struct EpiGateCausal {
     for (int su = half; su < BN / 32; su += kEpiColSplit) {
       const PairPos pp = pair_pos(g, t, 16 * su);
       if (!pp.ok) break;  // warp-uniform
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       float v[32];
       tmem_ld16<0>(tmem_acc + 16 * su, v);
       tmem_ld16<16>(tmem_acc + BN / 2 + 16 * su, v);
@@ -320,7 +320,7 @@ struct EpiGateCausal {
         float pr1[4], pr2[4], c[4], s[4];
         read_block16_4(in, lane, i, pr1);
         read_block16_4(in + 1024, lane, i, pr2);
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float s1 = pom_hardsigmoid(v[i + e] + bb1[e]);
@@ -404,7 +404,7 @@ struct EpiGateBwdCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_carry<BN>(sc.tile(slot), p.causal, g, t, lane);
   }
   // Each warp starts the load of its first input blocks while the tile's main loop is still running.
@@ -426,7 +426,7 @@ struct EpiGateBwdCausal {
     float* buf_b = sc.sums(slot);
     const float* bias = sc.cols();
     const float* carry = sc.tile(slot) + quarter * BN;
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<false> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     const int y = t.row0 + quarter * 32;
     const int grp = (t.row0 >> 5) + quarter;
     const bool grp_ok = grp < p.causal.groups && t.rows_valid > 0;
@@ -438,7 +438,7 @@ struct EpiGateBwdCausal {
     for (int su = half; su < BN / 32; su += kEpiColSplit) {
       float* b1p = buf_b + quarter * BN + 16 * su;
       const PairPos pp = pair_pos(g, t, 16 * su);
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       if (!pp.ok) {  // warp-uniform
         if (lane < 16) b1p[lane] = 0.f;
         else b1p[BN / 2 + lane - 16] = 0.f;
@@ -473,7 +473,7 @@ struct EpiGateBwdCausal {
         float pr1[4], pr2[4], c[4], s[4];
         read_block16_4(in + 2048, lane, i, pr1);
         read_block16_4(in + 3072, lane, i, pr2);
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float zz1 = z[i + e] + bb1[e], zz2 = z[16 + i + e] + bb2[e];

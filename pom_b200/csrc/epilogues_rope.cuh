@@ -8,16 +8,20 @@
 // rows of one CTA.  An epilogue warp walks the tile in sub-units of 16 pairs.
 //
 // cos/sin of (token, channel) never come from memory per element.  The tokens of a 32-row group (one
-// epilogue warp = one TMEM lane quarter) either share one position or hold consecutive positions
-// (RopeEpi::step, checked on the host), so
-//     angle(lane, j) = angle(group base, j) + lane * step * freq_j
+// epilogue warp = one TMEM lane quarter) share one position, hold consecutive positions, or lie within 61 of one
+// another (RopeEpi::step, checked on the host), so
+//     angle(token, j) = angle(group base, j) + offset(token) * freq_j,     |offset| <= 31
 // and the epilogue combines, per pair,
 //     the table row of the group's base position (staged one tile ahead by the stager warp: 4 groups x BN/2
 //     channels), and
-//     rows 0..31 of the same table (cos/sin of lane * freq_j; one 32 x 16 block per sub-unit, bulk-loaded once per
-//     column block)
+//     row |offset| of the same table (cos/sin of |offset| * freq_j, the sine with the offset's sign; rows 0..31 as one
+//     32 x 16 block per sub-unit, bulk-loaded once per column block)
 // with the angle-addition formulas: 4 multiply-adds instead of two table reads per element.
+// Offsets that are not the lane number (2-D grids whose rows do not end on 32 tokens: 24 x 24, 28 x 28, ...) cost a
+// load of the token's position and two warp reductions per tile and section.  At 32 x 24 x 24 x 1152 the three
+// phases take 106 + 107 + 130 us; three plain GEMMs and the operator passes with table reads took 450.
 #pragma once
+#include <climits>
 #include "epilogues.cuh"
 
 namespace pomk {
@@ -28,7 +32,7 @@ struct RopeEpi {
   const long long* pos;  // (rows, pos_stride) int64 token positions; section s reads column s (pos_stride 2)
   int pos_stride;
   int len[2];
-  int step[2];           // 0: the tokens of an aligned 32-token group share one position; 1: consecutive
+  int step[2];           // the tokens of an aligned 32-token group: 0 share one position; 1 consecutive; 2 span <= 61
   int rotate;            // 0: no rotation at all (cos = 1, sin = 0; tables and positions are not read)
   // selections by ternary keep the kernel parameters out of local memory (no dynamically indexed arrays)
   __device__ __forceinline__ int step_of(int sec) const { return sec ? step[1] : step[0]; }
@@ -67,11 +71,50 @@ struct PairScratch {
   }
 };
 
-// What an epilogue warp needs of the rotary constants of its tile.
+// Position of token n in section `sec`, clamped to the table (the host validates positions: the clamp only keeps reads
+// inside it).
+__device__ __forceinline__ int rope_pos(const RopeEpi& r, int n, int sec) {
+  const long long p = __ldg(r.pos + static_cast<long long>(n) * r.pos_stride + (r.pos_stride == 2 ? sec : 0));
+  const int len = r.len_of(sec);
+  return p < 0 ? 0 : p >= len ? len - 1 : static_cast<int>(p);
+}
+// Base of the 32-token group that starts at token n0 (whole warp; `own` receives the lane's own position): the first
+// token's position, or, where they only span <= 61, the smallest from which none is more than 31 away.
+__device__ __forceinline__ int rope_group_base(const RopeEpi& r, int n0, int rows, int sec, int lane, int& own) {
+  const bool ok = n0 + lane < rows;
+  own = ok ? rope_pos(r, n0 + lane, sec) : 0;
+  const int lo = __reduce_min_sync(0xffffffffu, ok ? own : INT_MAX);
+  const int hi = __reduce_max_sync(0xffffffffu, ok ? own : 0);
+  const int base = max(lo, hi - 31);
+  if (!ok) own = base;
+  return base;
+}
+
+// What an epilogue warp needs of the rotary constants of its tile.  SPAN: offsets other than the lane number are
+// possible (the token-causal epilogues, which have no registers left for them, never see such positions).
+template <bool SPAN>
 struct RopeView {
   const float* base_cos;  // [4 quarters][BN/2]
   const float* base_sin;
   const uint8_t* lane;
+  int row[2];        // per section: row of the lane tables that holds this token's offset
+  uint32_t flip[2];  // sign bit of a negative offset
+  __device__ __forceinline__ RopeView(const RopeEpi& r, const GemmGeom& g, const TileCtx& t, int quarter, int lane_id,
+                                      const float* bc, const float* bs, const uint8_t* lt)
+      : base_cos(bc), base_sin(bs), lane(lt) {
+#pragma unroll
+    for (int sec = 0; sec < 2; ++sec) {
+      row[sec] = lane_id;
+      flip[sec] = 0;
+      const int n0 = t.row0 + 32 * quarter;
+      if (SPAN && r.rotate && r.step_of(sec) == 2 && n0 < g.rows_per_batch && (sec == 0 || r.pos_stride == 2)) {
+        int own;
+        const int d = -rope_group_base(r, n0, g.rows_per_batch, sec, lane_id, own) + own;
+        row[sec] = abs(d);
+        flip[sec] = d < 0 ? 0x80000000u : 0u;
+      }
+    }
+  }
 };
 
 // Stager warp: starts the bulk loads of the lane tables of the tile's columns on `bar`; returns their bytes.
@@ -95,22 +138,23 @@ __device__ __forceinline__ uint32_t rope_stage_lane(const RopeEpi& r, const EpiM
 // Stager warp: cos / sin of the base position of the tile's four 32-row groups for its BN/2 pairs, four pairs per
 // load (pair_q and the tile's first pair are multiples of 4, the tables 16-byte aligned: the lane-table tensor maps
 // have the same needs).
-template <int BN>
+template <int BN, bool SPAN>
 __device__ __forceinline__ void rope_stage_base(const RopeEpi& r, const GemmGeom& g, const TileCtx& t, int lane,
                                                 float* base_cos, float* base_sin) {
   constexpr int kHalf = BN / 2;
   constexpr int kVec = kHalf / 4;  // float4 per row group
-  long long pos[4][2];  // [row group][section]; the host validates positions: the clamp only keeps reads inside the table
+  int pos[4][2];  // [row group][section]
 #pragma unroll
   for (int quarter = 0; quarter < 4; ++quarter) {
     const int n = t.row0 + 32 * quarter;
 #pragma unroll
     for (int sec = 0; sec < 2; ++sec) {
-      long long p = 0;
-      if (r.rotate && n < g.rows_per_batch && (sec == 0 || r.pos_stride == 2))
-        p = __ldg(r.pos + static_cast<long long>(n) * r.pos_stride + sec);
-      const long long len = r.len_of(sec);
-      pos[quarter][sec] = p < 0 ? 0 : (p >= len ? len - 1 : p);
+      int p = 0;
+      if (r.rotate && n < g.rows_per_batch && (sec == 0 || r.pos_stride == 2)) {
+        int own;
+        p = SPAN && r.step_of(sec) == 2 ? rope_group_base(r, n, g.rows_per_batch, sec, lane, own) : rope_pos(r, n, sec);
+      }
+      pos[quarter][sec] = p;
     }
   }
   static_assert((4 * kVec) % 32 == 0, "tile width");
@@ -123,8 +167,8 @@ __device__ __forceinline__ void rope_stage_base(const RopeEpi& r, const GemmGeom
     float4 c = make_float4(1.f, 1.f, 1.f, 1.f), s = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r.rotate && n < g.rows_per_batch && pp.ok) {
       const int which = r.pos_stride == 2 ? pp.sec : 0;
-      const long long p0 = quarter == 0 ? pos[0][0] : quarter == 1 ? pos[1][0] : quarter == 2 ? pos[2][0] : pos[3][0];
-      const long long p1 = quarter == 0 ? pos[0][1] : quarter == 1 ? pos[1][1] : quarter == 2 ? pos[2][1] : pos[3][1];
+      const int p0 = quarter == 0 ? pos[0][0] : quarter == 1 ? pos[1][0] : quarter == 2 ? pos[2][0] : pos[3][0];
+      const int p1 = quarter == 0 ? pos[0][1] : quarter == 1 ? pos[1][1] : quarter == 2 ? pos[2][1] : pos[3][1];
       const long long p = which ? p1 : p0;
       c = __ldg(reinterpret_cast<const float4*>(r.cos_of(pp.sec) + p * g.pair_q + pp.u));
       s = __ldg(reinterpret_cast<const float4*>(r.sin_of(pp.sec) + p * g.pair_q + pp.u));
@@ -150,16 +194,23 @@ __device__ __forceinline__ bool tail_last_warp(EpiIO& io, int parity, int lane) 
   return true;
 }
 
-// cos/sin of this lane's token for pairs [16 su + i, 16 su + i + 4) of the tile.
-template <int BN>
-__device__ __forceinline__ void rope_cs4(const RopeView& rs, bool stepped, int quarter, int lane, int su, int i,
+// cos/sin of this lane's token for pairs [16 su + i, 16 su + i + 4) of the tile; `step`: RopeEpi::step of the
+// sub-unit's section `sec`.
+template <int BN, bool SPAN>
+__device__ __forceinline__ void rope_cs4(const RopeView<SPAN>& rs, int step, int sec, int quarter, int su, int i,
                                          float (&c)[4], float (&s)[4]) {
   const float4 C0 = *reinterpret_cast<const float4*>(rs.base_cos + quarter * (BN / 2) + 16 * su + i);
   const float4 S0 = *reinterpret_cast<const float4*>(rs.base_sin + quarter * (BN / 2) + 16 * su + i);
-  if (stepped) {
+  if (step) {
     const uint8_t* blk = rs.lane + su * 4096;
-    const float4 cl = *reinterpret_cast<const float4*>(blk + swz64(lane, i >> 2));
-    const float4 sl = *reinterpret_cast<const float4*>(blk + 2048 + swz64(lane, i >> 2));
+    const int row = SPAN && sec ? rs.row[1] : rs.row[0];
+    const float4 cl = *reinterpret_cast<const float4*>(blk + swz64(row, i >> 2));
+    float4 sl = *reinterpret_cast<const float4*>(blk + 2048 + swz64(row, i >> 2));
+    if (SPAN && step == 2) {
+      const uint32_t f = sec ? rs.flip[1] : rs.flip[0];
+      sl.x = __uint_as_float(__float_as_uint(sl.x) ^ f), sl.y = __uint_as_float(__float_as_uint(sl.y) ^ f);
+      sl.z = __uint_as_float(__float_as_uint(sl.z) ^ f), sl.w = __uint_as_float(__float_as_uint(sl.w) ^ f);
+    }
     c[0] = C0.x * cl.x - S0.x * sl.x, s[0] = S0.x * cl.x + C0.x * sl.x;
     c[1] = C0.y * cl.y - S0.y * sl.y, s[1] = S0.y * cl.y + C0.y * sl.y;
     c[2] = C0.z * cl.z - S0.z * sl.z, s[2] = S0.z * cl.z + C0.z * sl.z;
@@ -255,7 +306,7 @@ struct EpiCtxRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
   }
   template <int BN>
   static __device__ __forceinline__ void prologue(const Params&, const EpiMaps&, const GemmGeom&, const TileCtx&, int,
@@ -264,7 +315,7 @@ struct EpiCtxRope {
   template <int KT, int BN>
   static __device__ __forceinline__ void body(const Params& p, const EpiMaps& maps, const GemmGeom& g,
                                               const TileCtx& t, uint32_t tmem_acc, int quarter, int lane, int half,
-                                              float* buf, const float* cst, const RopeView& rs, EpiIO& io) {
+                                              float* buf, const float* cst, const RopeView<true>& rs, EpiIO& io) {
     const int row = quarter * 32 + lane;
     const bool weighted = p.row_weight != nullptr;
     float w = 1.f;
@@ -277,7 +328,7 @@ struct EpiCtxRope {
       float* b1 = buf + quarter * BN + 16 * su;
       float* b2 = b1 + BN / 2;
       const PairPos pp = pair_pos(g, t, 16 * su);
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       if (!pp.ok || !t.live) {  // warp-uniform
         if (lane < 16) b1[lane] = 0.f;
         else b2[lane - 16] = 0.f;
@@ -312,7 +363,7 @@ struct EpiCtxRope {
         for (int e = 0; e < 4; ++e) a1[e] = act_fast(v[i + e]), a2[e] = act_fast(v[16 + i + e]);
         poly4<KT, BN>(cst + 16 * su + i, p.K, a1, f1);
         poly4<KT, BN>(cst + BN / 2 + 16 * su + i, p.K, a2, f2);
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float r1 = f1[e] * c[e] - f2[e] * s[e];
@@ -336,7 +387,7 @@ struct EpiCtxRope {
     const int slot = iter & 1;
     float* buf = sc.sums(slot);
     const float* cst = sc.cols();
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<true> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     switch (p.K) {
       case 1: body<1, BN>(p, maps, g, t, tmem_acc, quarter, lane, half, buf, cst, rs, io); break;
       case 2: body<2, BN>(p, maps, g, t, tmem_acc, quarter, lane, half, buf, cst, rs, io); break;
@@ -398,7 +449,7 @@ struct EpiGateRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_paired_vector<BN>(sc.tile(slot), p.H + static_cast<long long>(t.b) * p.h_batch_stride, g, t, lane);
   }
   template <int BN>
@@ -413,13 +464,13 @@ struct EpiGateRope {
     const int slot = iter & 1;
     const float* bias = sc.cols();
     const float* hrow = sc.tile(slot);
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<true> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     const int y = t.row0 + quarter * 32;
 #pragma unroll 1
     for (int su = half; su < BN / 32; su += kEpiColSplit) {
       const PairPos pp = pair_pos(g, t, 16 * su);
       if (!pp.ok) break;  // warp-uniform
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       float v[32];
       tmem_ld16<0>(tmem_acc + 16 * su, v);
       tmem_ld16<16>(tmem_acc + BN / 2 + 16 * su, v);
@@ -437,7 +488,7 @@ struct EpiGateRope {
         const float bb1[4] = {b1.x, b1.y, b1.z, b1.w}, bb2[4] = {b2.x, b2.y, b2.z, b2.w};
         const float hh1[4] = {h1.x, h1.y, h1.z, h1.w}, hh2[4] = {h2.x, h2.y, h2.z, h2.w};
         float c[4], s[4];
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float s1 = pom_hardsigmoid(v[i + e] + bb1[e]);
@@ -522,7 +573,7 @@ struct EpiGateBwdRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_paired_vector<BN>(sc.tile(slot), p.H + static_cast<long long>(t.b) * p.h_batch_stride, g, t, lane);
   }
   // Each warp starts the load of its first z blocks while the tile's main loop is still running.
@@ -545,7 +596,7 @@ struct EpiGateBwdRope {
     float* buf_b = buf_h + 4 * BN;
     const float* bias = sc.cols();
     const float* hrow = sc.tile(slot);
-    const RopeView rs{sc.base_cos(slot), sc.base_sin(slot), sc.lane()};
+    const RopeView<true> rs(p.rope, g, t, quarter, lane, sc.base_cos(slot), sc.base_sin(slot), sc.lane());
     const int y = t.row0 + quarter * 32;
     uint8_t* out_blk = io.buf0 + 2048;
     bool alive = true;
@@ -554,7 +605,7 @@ struct EpiGateBwdRope {
       float* h1p = buf_h + quarter * BN + 16 * su;
       float* b1p = buf_b + quarter * BN + 16 * su;
       const PairPos pp = pair_pos(g, t, 16 * su);
-      const bool stepped = p.rope.step_of(pp.sec) != 0;
+      const int step = p.rope.step_of(pp.sec);
       if (!pp.ok) {  // warp-uniform
         if (lane < 16) h1p[lane] = 0.f, b1p[lane] = 0.f;
         else h1p[BN / 2 + lane - 16] = 0.f, b1p[BN / 2 + lane - 16] = 0.f;
@@ -585,7 +636,7 @@ struct EpiGateBwdRope {
         const float bb1[4] = {b1.x, b1.y, b1.z, b1.w}, bb2[4] = {b2.x, b2.y, b2.z, b2.w};
         const float hh1[4] = {h1.x, h1.y, h1.z, h1.w}, hh2[4] = {h2.x, h2.y, h2.z, h2.w};
         float c[4], s[4];
-        rope_cs4<BN>(rs, stepped, quarter, lane, su, i, c, s);
+        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float zz1 = z[i + e] + bb1[e], zz2 = z[16 + i + e] + bb2[e];

@@ -44,7 +44,7 @@ int make_rope(const pom_rope& r, const PairShape& ps, RopeEpi* e, EpiMaps* maps)
   e->step[0] = r.step0, e->step[1] = ps.sections == 2 ? r.step1 : r.step0;
   for (int s = 0; s < ps.sections; ++s) {
     if (e->len[s] < 1) return POM_ERR_BAD_SHAPE;
-    if (e->step[s] != 0 && e->step[s] != 1) return POM_ERR_UNSUPPORTED;
+    if (e->step[s] < 0 || e->step[s] > 2) return POM_ERR_UNSUPPORTED;
     int rc;
     if ((rc = make_lane_table_map(&maps->lane[2 * s], e->cos[s], ps.q, e->len[s]))) return rc;
     if ((rc = make_lane_table_map(&maps->lane[2 * s + 1], e->sin[s], ps.q, e->len[s]))) return rc;
@@ -54,7 +54,7 @@ int make_rope(const pom_rope& r, const PairShape& ps, RopeEpi* e, EpiMaps* maps)
 
 // ---------------------------------------------------------------- position scan
 // One CTA: per column of the positions, min / max and whether every aligned 32-token group is constant /
-// consecutive.  Thread i owns tokens i, i + 1024, ... (a warp therefore always holds one aligned group).
+// consecutive / at most 61 wide.  Thread i owns tokens i, i + 1024, ... (a warp therefore always holds one aligned group).
 __global__ void __launch_bounds__(1024) rope_pos_info_kernel(const long long* __restrict__ pos, long long n, int stride,
                                                              long long* __restrict__ info) {
   __shared__ long long s_min[2][32], s_max[2][32];
@@ -62,12 +62,19 @@ __global__ void __launch_bounds__(1024) rope_pos_info_kernel(const long long* __
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c = 0; c < stride; ++c) {
     long long mn = LLONG_MAX, mx = LLONG_MIN;
-    int flat = 1, step = 1;
+    int flat = 1, step = 1, near = 1;
     for (long long base = 0; base < n; base += 1024) {
       const long long i = base + threadIdx.x;
       const bool ok = i < n;
       const long long p = ok ? pos[i * stride + c] : 0;
       const long long p0 = __shfl_sync(0xffffffffu, p, 0);  // lane 0 of a group that has any token is valid
+      long long lo = ok ? p : p0, hi = lo;
+      for (int off = 16; off; off >>= 1) {
+        const long long ol = __shfl_xor_sync(0xffffffffu, lo, off), oh = __shfl_xor_sync(0xffffffffu, hi, off);
+        lo = ol < lo ? ol : lo;
+        hi = oh > hi ? oh : hi;
+      }
+      if (base + (threadIdx.x & ~31u) < n && hi - lo > 61) near = 0;
       if (ok) {
         mn = p < mn ? p : mn;
         mx = p > mx ? p : mx;
@@ -81,21 +88,21 @@ __global__ void __launch_bounds__(1024) rope_pos_info_kernel(const long long* __
       mx = omx > mx ? omx : mx;
       flat &= __shfl_xor_sync(0xffffffffu, flat, off);
       step &= __shfl_xor_sync(0xffffffffu, step, off);
-    }
-    if (lane == 0) s_min[c][warp] = mn, s_max[c][warp] = mx, s_flat[c][warp] = flat, s_step[c][warp] = step;
+    }  // `near` is warp-uniform
+    if (lane == 0) s_min[c][warp] = mn, s_max[c][warp] = mx, s_flat[c][warp] = flat, s_step[c][warp] = step | near << 1;
   }
   __syncthreads();
   if (threadIdx.x < stride) {
     const int c = threadIdx.x;
     long long mn = LLONG_MAX, mx = LLONG_MIN;
-    int flat = 1, step = 1;
+    int flat = 1, step = 3;
     for (int w = 0; w < 32; ++w) {
       mn = s_min[c][w] < mn ? s_min[c][w] : mn;
       mx = s_max[c][w] > mx ? s_max[c][w] : mx;
       flat &= s_flat[c][w];
       step &= s_step[c][w];
     }
-    info[4 * c + 0] = mn, info[4 * c + 1] = mx, info[4 * c + 2] = flat, info[4 * c + 3] = step;
+    info[4 * c + 0] = mn, info[4 * c + 1] = mx, info[4 * c + 2] = flat, info[4 * c + 3] = (step & 1) ? 1 : step;
   }
 }
 

@@ -863,7 +863,9 @@ constexpr int kStHalf = kStCols / 2;
 // CAUSAL (the fused token-causal layer): tiles are one 32-token group; beside hp the ring carries `suf`, the
 // running sums (up the group's rows) of the gradient of the prefix means written by the causal gate-backward
 // epilogue, and the gradient of token n's features is suf[n] + carry[group] instead of w[n]·dH.
-template <int KR, bool CAUSAL>
+// TABLE: positions of any order; every token's table row is read (the rows of the block's 128 channels stay in L1)
+// instead of being built from its group's base row.
+template <int KR, bool CAUSAL, bool TABLE>
 __global__ void __launch_bounds__(256, 2)
 agg_bwd_stream_pair_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tms,
                            const AggBwdDev a, int tiles_per_cta, int splits, int q, int blocks_per_section,
@@ -964,7 +966,7 @@ agg_bwd_stream_pair_kernel(const __grid_constant__ CUtensorMap tmx, const __grid
   for (int j = 0; j < 4; ++j) {
     cl[j] = make_float4(1.f, 1.f, 1.f, 1.f);
     sl[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (stepped && live) {
+    if (!TABLE && stepped && live) {
       long long row = ty + 8 * j;
       row = row >= tab_len ? tab_len - 1 : row;  // offsets past the table belong to tokens that do not exist
       cl[j] = __ldg(reinterpret_cast<const float4*>(cos_t + row * q));
@@ -996,7 +998,7 @@ agg_bwd_stream_pair_kernel(const __grid_constant__ CUtensorMap tmx, const __grid
       c0[g] = make_float4(1.f, 1.f, 1.f, 1.f);
       s0[g] = make_float4(0.f, 0.f, 0.f, 0.f);
       const int n = n0 + 32 * g;
-      if (rotate && live && n < a.N) {
+      if (!TABLE && rotate && live && n < a.N) {
         long long idx = __ldg(a.rope.pos + static_cast<long long>(n) * a.rope.pos_stride + which);
         idx = idx < 0 ? 0 : (idx >= tab_len ? tab_len - 1 : idx);
         c0[g] = __ldg(reinterpret_cast<const float4*>(cos_t + idx * q));
@@ -1046,15 +1048,22 @@ agg_bwd_stream_pair_kernel(const __grid_constant__ CUtensorMap tmx, const __grid
           }
         }
         const float2 w2 = make_float2(w, w), nw2 = make_float2(-w, -w);
-        const float2 C0[H] = {make_float2(c0[g].x, c0[g].y), make_float2(c0[g].z, c0[g].w)};
-        const float2 S0[H] = {make_float2(s0[g].x, s0[g].y), make_float2(s0[g].z, s0[g].w)};
-        const float2 nS0[H] = {make_float2(-s0[g].x, -s0[g].y), make_float2(-s0[g].z, -s0[g].w)};
+        float4 ct = c0[g], st = s0[g];
+        if (TABLE) {
+          long long idx = __ldg(a.rope.pos + static_cast<long long>(n) * a.rope.pos_stride + which);
+          idx = idx < 0 ? 0 : (idx >= tab_len ? tab_len - 1 : idx);
+          ct = __ldg(reinterpret_cast<const float4*>(cos_t + idx * q));
+          st = __ldg(reinterpret_cast<const float4*>(sin_t + idx * q));
+        }
+        const float2 C0[H] = {make_float2(ct.x, ct.y), make_float2(ct.z, ct.w)};
+        const float2 S0[H] = {make_float2(st.x, st.y), make_float2(st.z, st.w)};
+        const float2 nS0[H] = {make_float2(-st.x, -st.y), make_float2(-st.z, -st.w)};
         const float2 CL[H] = {make_float2(cl[j].x, cl[j].y), make_float2(cl[j].z, cl[j].w)};
         const float2 SL[H] = {make_float2(sl[j].x, sl[j].y), make_float2(sl[j].z, sl[j].w)};
 #pragma unroll
         for (int h = 0; h < H; ++h) {
-          const float2 cc = __ffma2_rn(nS0[h], SL[h], __fmul2_rn(C0[h], CL[h]));  // cos(base + lane offset)
-          const float2 ss = __ffma2_rn(C0[h], SL[h], __fmul2_rn(S0[h], CL[h]));   // sin(base + lane offset)
+          const float2 cc = TABLE ? C0[h] : __ffma2_rn(nS0[h], SL[h], __fmul2_rn(C0[h], CL[h]));  // cos(base + offset)
+          const float2 ss = TABLE ? S0[h] : __ffma2_rn(C0[h], SL[h], __fmul2_rn(S0[h], CL[h]));   // sin(base + offset)
           // transposed rotation of the incoming gradient: d1 = w (g1 cc + g2 ss), d2 = w (g2 cc - g1 ss)
           const float2 d1 = __fmul2_rn(w2, __ffma2_rn(gg2[h], ss, __fmul2_rn(gg1[h], cc)));
           const float2 d2 = __fmul2_rn(nw2, __ffma2_rn(gg1[h], ss, __fmul2_rn(make_float2(-gg2[h].x, -gg2[h].y), cc)));
@@ -1158,8 +1167,9 @@ bool stream_bwd_rope_eligible(const pom_agg_bwd_args* a) {
   if (a->rope.kind == POM_ROPE_NONE)
     return a->ldx % 8 == 0 && a->ld_dx % 8 == 0 && aligned16(a->x) && aligned16(a->dx);
   if (a->rope.pos_stride != sp.sections || a->rope.len0 < 1 || (sp.sections == 2 && a->rope.len1 < 1)) return false;
-  if ((a->rope.step0 != 0 && a->rope.step0 != 1) || (sp.sections == 2 && a->rope.step1 != 0 && a->rope.step1 != 1))
-    return false;  // arbitrary positions: the chunked kernel reads a table row per token
+  const int most = a->causal == 3 ? 1 : 2;  // the token-causal layer takes shared and consecutive positions only
+  if (a->rope.step0 < 0 || a->rope.step0 > most || (sp.sections == 2 && (a->rope.step1 < 0 || a->rope.step1 > most)))
+    return false;
   if (a->ldx % 8 || a->ld_dx % 8 || !aligned16(a->x) || !aligned16(a->dx)) return false;
   for (const void* t : {static_cast<const void*>(a->rope.cos0), static_cast<const void*>(a->rope.sin0),
                         static_cast<const void*>(a->rope.cos1), static_cast<const void*>(a->rope.sin1)})
@@ -1902,9 +1912,9 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
                      static_cast<unsigned>(a->B));
     static std::atomic<uint64_t> attr_done_rope{0};
     (void)once_per_device(attr_done_rope, [] {
-      cudaFuncSetAttribute(agg_bwd_stream_pair_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemBytes);
-      cudaFuncSetAttribute(agg_bwd_stream_pair_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemBytes);
-      cudaFuncSetAttribute(agg_bwd_stream_pair_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemBytes);
+      for (const auto f : {agg_bwd_stream_pair_kernel<2, false, false>, agg_bwd_stream_pair_kernel<2, false, true>,
+                           agg_bwd_stream_pair_kernel<2, true, false>, agg_bwd_stream_pair_kernel<4, true, false>})
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kStSmemBytes);
       return static_cast<int>(POM_OK);
     });
     const int bps = sp.col_blocks / pr.sections;
@@ -1912,15 +1922,11 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
     if ((rc = stream_tile_map(&tmx, a->x, a->P, a->N, a->B, a->ldx, kStHalf, tt))) return rc;
     tms = tmx;
     if (fused_causal && (rc = stream_tile_map(&tms, a->dout, a->P, a->N, a->B, a->ld_dout, kStHalf, tt))) return rc;
-    if (!fused_causal)
-      (void)launch_pdl(agg_bwd_stream_pair_kernel<2, false>, sgrid, dim3(256), kStSmemBytes, st, tmx, tms, d,
-                       sp.tiles_per_cta, sp.splits, pr.q, bps, status);
-    else if (a->K <= 2)
-      (void)launch_pdl(agg_bwd_stream_pair_kernel<2, true>, sgrid, dim3(256), kStSmemBytes, st, tmx, tms, d,
-                       sp.tiles_per_cta, sp.splits, pr.q, bps, status);
-    else
-      (void)launch_pdl(agg_bwd_stream_pair_kernel<4, true>, sgrid, dim3(256), kStSmemBytes, st, tmx, tms, d,
-                       sp.tiles_per_cta, sp.splits, pr.q, bps, status);
+    const bool table = a->rope.kind != POM_ROPE_NONE && (a->rope.step0 == 2 || (pr.sections == 2 && a->rope.step1 == 2));
+    const auto kern = fused_causal ? (a->K <= 2 ? agg_bwd_stream_pair_kernel<2, true, false> : agg_bwd_stream_pair_kernel<4, true, false>)
+                      : table      ? agg_bwd_stream_pair_kernel<2, false, true>
+                                   : agg_bwd_stream_pair_kernel<2, false, false>;
+    (void)launch_pdl(kern, sgrid, dim3(256), kStSmemBytes, st, tmx, tms, d, sp.tiles_per_cta, sp.splits, pr.q, bps, status);
     count_launch();
     return check_launch();
   }

@@ -331,7 +331,7 @@ class _PoMLayer(torch.autograd.Function):
         # rotary embedding rides in the GEMM epilogues when the positions of every aligned 32-token group are
         # constant or consecutive (RopeSpec.steps) and the degree is at most 4; otherwise on the operator path
         rotary = spec.rope_ctx is not None or spec.rope_qry is not None
-        rope_ok = not rotary or (K <= 4 and all(r is None or r.fusable(P) for r in (spec.rope_ctx, spec.rope_qry)))
+        rope_ok = not rotary or (K <= 4 and all(r is None or r.fusable(P, causal) for r in (spec.rope_ctx, spec.rope_qry)))
         fused = (bf16 and not heads and (not rotary or rope_ok) and not causal and not full
                  and P % 8 == 0 and D % 8 == 0)
         # token-causal: the prefix means ride in the same epilogues (running sums per 32-token group + a scan over

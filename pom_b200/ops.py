@@ -78,8 +78,8 @@ class RopeSpec:
     cos1: Optional[torch.Tensor] = None
     sin1: Optional[torch.Tensor] = None
     # per position column, how the positions of every aligned group of 32 tokens look: 0 = one shared position,
-    # 1 = consecutive positions, -1 = anything else / unknown (see rope_pos_info); the fused tensor-core phases
-    # need 0 or 1, the stand-alone operators take any positions
+    # 1 = consecutive positions, 2 = at most 61 apart, -1 = anything else / unknown (see rope_pos_info); the fused
+    # tensor-core phases need 0 to 2 (token-causal: 0 or 1), the stand-alone operators take any positions
     steps: Tuple[int, int] = (-1, -1)
 
     def to_c(self) -> Rope:
@@ -94,12 +94,14 @@ class RopeSpec:
         r.step0, r.step1 = self.steps
         return r
 
-    def fusable(self, p: int) -> bool:
+    def fusable(self, p: int, causal: bool = False) -> bool:
         """Whether the rotary GEMM epilogues can take this description for p channels."""
+        if causal and 2 in self.steps:
+            return False
         if self.kind == _abi.ROPE_1D:
-            return p % 16 == 0 and self.cos0.shape[1] == p // 2 and self.steps[0] in (0, 1)
+            return p % 16 == 0 and self.cos0.shape[1] == p // 2 and self.steps[0] >= 0
         return (p % 64 == 0 and self.cos0.shape[1] == p // 4 and self.cos1.shape[1] == p // 4
-                and self.steps[0] in (0, 1) and self.steps[1] in (0, 1))
+                and self.steps[0] >= 0 and self.steps[1] >= 0)
 
 
 _pos_info_cache = {}
@@ -126,7 +128,7 @@ def rope_pos_info(pos: torch.Tensor):
     _abi.check(_abi.lib().pom_rope_pos_info(ptr(pos), pos.shape[0], stride, ptr(info), _abi.stream_ptr()),
                "pom_rope_pos_info")
     vals = info.cpu().tolist()
-    out = tuple((vals[4 * c], vals[4 * c + 1], 0 if vals[4 * c + 2] else (1 if vals[4 * c + 3] else -1))
+    out = tuple((vals[4 * c], vals[4 * c + 1], 0 if vals[4 * c + 2] else (vals[4 * c + 3] or -1))
                 for c in range(stride))
     if cacheable:
         _pos_info_cache[key] = (weakref.ref(pos), pos._version, out)
