@@ -155,6 +155,13 @@ uint64_t pom_gemm_f32_planes_scratch(int64_t M, int64_t N, int64_t K, int32_t ou
 int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_planes, int b_ready, void* scratch,
                         int* status, void* stream);
 
+/* A float32 projection C = A·Bmᵀ (both K-major, alpha 1, F32 out) whose columns feed the activation (columns below
+ * gate_col0) or, after gate_bias, the gate: pom_gemm_f32_planes, and then the value of pom_gemm_f32, bit for bit, for
+ * every element that lies close enough to a kink for the order of additions to decide on its side.  `norms`: M + N
+ * floats of scratch. */
+int pom_project_f32(const pom_gemm_args* a, void* a_planes, void* b_planes, float* norms, int64_t gate_col0,
+                    const float* gate_bias, int* status, void* stream);
+
 /* ------------------------------------------------------------------------------------------
  * Context phase, fused (bf16): hp = X·Wpoᵀ on tensor cores; the epilogue rounds hp to bf16,
  * optionally saves it, applies act + polynomial (+ per-token weight) and reduces over each

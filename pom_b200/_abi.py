@@ -216,6 +216,8 @@ _SIGNATURES = {
     "pom_gemm_f32_planes_scratch": (C.c_uint64, [C.c_int64, C.c_int64, C.c_int64, C.c_int32]),
     "pom_gemm_f32_planes": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p,
                                       C.c_void_p, C.c_void_p]),
+    "pom_project_f32": (C.c_int, [C.POINTER(GemmArgs), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p,
+                                  C.c_void_p, C.c_void_p]),
     "pom_ctx_gemm": (C.c_int, [C.POINTER(CtxArgs), C.c_void_p, C.c_void_p]),
     "pom_reduce_partials": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_float, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     "pom_gate_gemm": (C.c_int, [C.POINTER(GateArgs), C.c_void_p, C.c_void_p]),

@@ -17,6 +17,8 @@
 // Infinities, NaN and magnitudes of 2^56 or more (whose plane products could meet with opposite signs) do not go
 // through the planes: the split marks them and the FMA kernel (sgemm_kernel) computes that product instead, on the
 // device, without a host decision.
+#include <cfloat>
+#include <cmath>
 #include <cudaTypedefs.h>
 #include "common.cuh"
 #include "gemm_launch.cuh"
@@ -38,6 +40,10 @@ inline int split_blocks(int64_t rows, int64_t cols) {
   const int64_t n = ceil_div(rows * (plane_ld(cols) / 8), kSplitThreads);
   return static_cast<int>(n < kFlagWords ? n : kFlagWords);
 }
+inline int row_blocks(int64_t rows) {  // a warp per row
+  const int64_t n = ceil_div(rows, kSplitThreads / 32);
+  return static_cast<int>(n < kFlagWords ? n : kFlagWords);
+}
 inline __nv_bfloat16* planes_of(void* buf) {
   return reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(buf) + kFlagBytes);
 }
@@ -50,6 +56,17 @@ struct SplitMat {
   long long rows, cols, ld, groups;  // groups of 8 columns per row
   int blocks;
 };
+
+// Eight values of a row, zero past its end.
+__device__ __forceinline__ void load8(const float* s, long long left, bool vec, float (&v)[8]) {
+  if (vec && left >= 8) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(s)), y = __ldg(reinterpret_cast<const float4*>(s) + 1);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = e < left ? __ldg(s + e) : 0.f;
+  }
+}
 
 __device__ __forceinline__ void split_pair(float a, float b, uint32_t (&o)[3]) {
   o[0] = pack_bf16x2(a, b);
@@ -71,15 +88,8 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
   bool bad = false;
   for (long long i = blockIdx.x * 1ll * kSplitThreads + threadIdx.x; i < total; i += 1ll * m.blocks * kSplitThreads) {
     const long long r = i / m.groups, c = (i - r * m.groups) * 8;
-    const float* s = m.src + r * m.ld + c;
     float v[8];
-    if (vec && c + 8 <= m.cols) {
-      const float4 x = __ldg(reinterpret_cast<const float4*>(s)), y = __ldg(reinterpret_cast<const float4*>(s) + 1);
-      v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) v[e] = c + e < m.cols ? __ldg(s + e) : 0.f;
-    }
+    load8(m.src + r * m.ld + c, m.cols - c, vec, v);
     uint32_t p[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -91,6 +101,125 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
   }
   const int any = __syncthreads_or(bad);
   if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
+}
+
+// The same with a warp per row, which also leaves the row's 2-norm (pom_project_f32).
+__global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMat m0, const SplitMat m1,
+                                                                   float* __restrict__ norms) {
+  griddep_wait();
+  griddep_launch();
+  const SplitMat& m = blockIdx.y ? m1 : m0;
+  if (static_cast<int>(blockIdx.x) >= m.blocks) return;
+  float* norm = norms + (blockIdx.y ? m0.rows : 0);
+  const int lane = threadIdx.x & 31, warps = kSplitThreads / 32;
+  const bool vec = (m.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0;
+  const long long plane = m.rows * m.groups;
+  bool bad = false;
+  for (long long r = blockIdx.x * 1ll * warps + (threadIdx.x >> 5); r < m.rows; r += 1ll * m.blocks * warps) {
+    float sq = 0.f;
+    for (long long g = lane; g < m.groups; g += 32) {
+      float v[8];
+      load8(m.src + r * m.ld + g * 8, m.cols - g * 8, vec, v);
+      uint32_t p[4][3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        bad |= !(fabsf(v[2 * e]) < 0x1p56f) || !(fabsf(v[2 * e + 1]) < 0x1p56f);
+        sq = fmaf(v[2 * e], v[2 * e], fmaf(v[2 * e + 1], v[2 * e + 1], sq));
+        split_pair(v[2 * e], v[2 * e + 1], p[e]);
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        m.dst[k * plane + r * m.groups + g] = make_uint4(p[0][k], p[1][k], p[2][k], p[3][k]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (lane == 0) norm[r] = sqrtf(sq);
+  }
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
+}
+
+// ---------------------------------------------------------------------------- chain values beside the kinks
+struct NearArgs {
+  const float* A;
+  const float* B;
+  float* C;
+  const float* norms;  // 2-norms of the M rows of A, then of the N rows of B
+  const float* bias;   // of the gate columns
+  long long lda, ldb, ldc;
+  int M, N, K;
+  int gate0;           // columns from here on are gate columns
+  float factor;
+};
+
+// C = A·Bᵀ as the planes gave it -> elements so close to a kink (activation: 0, 6, -10; gate: -3 and 3 after its bias)
+// that the FMA chain's rounding could put them on the other side get the chain's own value, bit for bit that of
+// sgemm_kernel.  Both sums are within factor * |a| |b| of one another, factor = 8 sqrt(K) 2^-24: a chain's error stays
+// below lambda sqrt(K) 2^-24 sum |a_k b_k| but for a probability of 2 exp(-lambda^2 / 2) (Higham and Mary, 2019; 8: 3e-14),
+// the planes' is a fifth of it, and sum |a_k b_k| <= |a| |b|.  One element in about 3000 is that close.
+// The float32 training step at 4 x 1020 x 1152 takes 1429 us with this and 1952 with the FMA chain for every element.
+__global__ void __launch_bounds__(256) near_kinks_kernel(const NearArgs a) {
+  griddep_wait();
+  griddep_launch();
+  const int lane = threadIdx.x & 31;
+  const int per_row = (a.N + 3) / 4;
+  const long long total = 1ll * a.M * per_row, stride = gridDim.x * 256ll;
+  for (long long base = blockIdx.x * 256ll + (threadIdx.x - lane); base < total; base += stride) {
+    const long long i = base + lane;
+    const bool on = i < total;
+    const long long r = on ? i / per_row : 0;
+    const int c0 = on ? static_cast<int>(i - r * per_row) * 4 : 0;
+    float* row = a.C + r * a.ldc + c0;
+    float v[4];
+    if (c0 + 4 <= a.N && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+      const float4 q = *reinterpret_cast<const float4*>(row);
+      v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = c0 + e < a.N ? row[e] : 0.f;
+    }
+    const float na = a.factor * __ldg(a.norms + r);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int c = min(c0 + e, a.N - 1);
+      const float eps = na * __ldg(a.norms + a.M + c);
+      const bool gate = c >= a.gate0;
+      const float x = gate ? fabsf(v[e] + __ldg(a.bias + c - a.gate0)) : v[e];
+      const bool near = gate ? fabsf(x - 3.f) <= eps
+                             : fabsf(x) <= eps || fabsf(x - 6.f) <= eps || fabsf(x + 10.f) <= eps;
+      // (a sum that is not finite has come from the FMA kernel already)
+      uint32_t todo = __ballot_sync(0xffffffffu, on && c0 + e < a.N && near && eps < FLT_MAX);
+      while (todo) {  // the whole warp brings the element's two rows, 128 k ahead; every lane runs the chain
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const float* pa = a.A + __shfl_sync(0xffffffffu, r, src) * a.lda;
+        const float* pb = a.B + static_cast<long long>(__shfl_sync(0xffffffffu, c, src)) * a.ldb;
+        float acc = 0.f, xa[4], xb[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int k = 32 * q + lane;
+          xa[q] = k < a.K ? __ldg(pa + k) : 0.f, xb[q] = k < a.K ? __ldg(pb + k) : 0.f;
+        }
+        for (int k0 = 0; k0 < a.K; k0 += 128) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float ca = xa[q], cb = xb[q];
+            const int k = k0 + 128 + 32 * q + lane, left = a.K - k0 - 32 * q;
+            xa[q] = k < a.K ? __ldg(pa + k) : 0.f, xb[q] = k < a.K ? __ldg(pb + k) : 0.f;
+            if (left >= 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                acc = fmaf(__shfl_sync(0xffffffffu, ca, j), __shfl_sync(0xffffffffu, cb, j), acc);
+            } else {
+              for (int j = 0; j < left; ++j)
+                acc = fmaf(__shfl_sync(0xffffffffu, ca, j), __shfl_sync(0xffffffffu, cb, j), acc);
+            }
+          }
+        }
+        if (lane == src) row[e] = acc;
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------- the GEMM
@@ -448,39 +577,27 @@ SplitMat split_mat(const void* src, int64_t rows, int64_t cols, int64_t ld, void
   return m;
 }
 
-}  // namespace
-
-extern "C" {
-
-uint64_t pom_f32_planes_bytes(int64_t rows, int64_t cols) {
-  if (rows <= 0 || cols <= 0) return 0;
-  return kFlagBytes + 3ull * static_cast<uint64_t>(rows) * static_cast<uint64_t>(plane_ld(cols)) * 2ull;
-}
-
-uint64_t pom_gemm_f32_planes_scratch(int64_t M, int64_t N, int64_t K, int32_t out_mode) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const F32Plan p = pick_f32_plan(M, N, K, out_mode);
-  return p.split > 1 ? static_cast<uint64_t>(p.split) * M * ((N + 3) / 4 * 4) * 4 : 0;
-}
-
-int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_planes, int b_ready, void* scratch,
-                        int* status, void* stream) {
+// `norms` != NULL: the 2-norms of the rows of both operands (K-major, neither ready) are written there.
+int planes_product(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_planes, int b_ready, float* norms,
+                   void* scratch, int* status, cudaStream_t st) {
   if (!a || !a->A || !a->Bm || !a->C || !a_planes || !b_planes) return POM_ERR_NULL;
   if (a->M <= 0 || a->N <= 0 || a->K <= 0) return POM_ERR_BAD_SHAPE;
   if (a->out_mode != POM_OUT_F32 && a->out_mode != POM_OUT_F32_ACCUM) return POM_ERR_UNSUPPORTED;
   if (a->batches != 1) return POM_ERR_UNSUPPORTED;
   if (ceil_div(a->M, 64) > 65535 || a->N > INT32_MAX || a->K > INT32_MAX) return POM_ERR_TOO_LARGE;  // as pom_gemm_f32
   if (!aligned16(a_planes) || !aligned16(b_planes) || !aligned16(scratch)) return POM_ERR_BAD_ALIGN;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t ar = a->a_mn_major ? a->K : a->M, ac = a->a_mn_major ? a->M : a->K;
   const int64_t br = a->b_mn_major ? a->K : a->N, bc = a->b_mn_major ? a->N : a->K;
   SplitMat ma = split_mat(a->A, ar, ac, a->lda, a_planes), mb = split_mat(a->Bm, br, bc, a->ldb, b_planes);
+  if (norms) ma.blocks = row_blocks(ar), mb.blocks = row_blocks(br);
   const SgemmFlags flags{ma.flags, ma.blocks, mb.flags, mb.blocks};
   if (!a_ready || !b_ready) {
     const SplitMat& first = a_ready ? mb : ma;
     const int two = !a_ready && !b_ready;
     const int blocks = two && mb.blocks > ma.blocks ? mb.blocks : first.blocks;
-    if (launch_pdl(split_planes_kernel, dim3(blocks, 1 + two), dim3(kSplitThreads), 0, st, first, mb) != cudaSuccess) {
+    if ((norms ? launch_pdl(split_rows_kernel, dim3(blocks, 1 + two), dim3(kSplitThreads), 0, st, first, mb, norms)
+               : launch_pdl(split_planes_kernel, dim3(blocks, 1 + two), dim3(kSplitThreads), 0, st, first, mb)) !=
+        cudaSuccess) {
       (void)cudaGetLastError();
       return POM_ERR_CUDA;
     }
@@ -513,4 +630,50 @@ int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, voi
   return launch_sgemm(a, flags, st);
 }
 
+}  // namespace
+
+extern "C" {
+
+uint64_t pom_f32_planes_bytes(int64_t rows, int64_t cols) {
+  if (rows <= 0 || cols <= 0) return 0;
+  return kFlagBytes + 3ull * static_cast<uint64_t>(rows) * static_cast<uint64_t>(plane_ld(cols)) * 2ull;
+}
+
+uint64_t pom_gemm_f32_planes_scratch(int64_t M, int64_t N, int64_t K, int32_t out_mode) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const F32Plan p = pick_f32_plan(M, N, K, out_mode);
+  return p.split > 1 ? static_cast<uint64_t>(p.split) * M * ((N + 3) / 4 * 4) * 4 : 0;
+}
+
+int pom_gemm_f32_planes(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_planes, int b_ready, void* scratch,
+                        int* status, void* stream) {
+  return planes_product(a, a_planes, a_ready, b_planes, b_ready, nullptr, scratch, status,
+                        static_cast<cudaStream_t>(stream));
+}
+
+int pom_project_f32(const pom_gemm_args* a, void* a_planes, void* b_planes, float* norms, int64_t gate_col0,
+                    const float* gate_bias, int* status, void* stream) {
+  if (!a || !norms) return POM_ERR_NULL;
+  if (a->a_mn_major || a->b_mn_major || a->out_mode != POM_OUT_F32 || a->alpha != 1.f) return POM_ERR_UNSUPPORTED;
+  if (gate_col0 < 0 || gate_col0 > a->N) return POM_ERR_BAD_SHAPE;
+  if (gate_col0 < a->N && !gate_bias) return POM_ERR_NULL;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int rc = planes_product(a, a_planes, 0, b_planes, 0, norms, nullptr, status, st);
+  if (rc) return rc;
+  NearArgs n;
+  n.A = static_cast<const float*>(a->A), n.B = static_cast<const float*>(a->Bm), n.C = static_cast<float*>(a->C);
+  n.norms = norms, n.bias = gate_bias;
+  n.lda = a->lda, n.ldb = a->ldb, n.ldc = a->ldc;
+  n.M = static_cast<int>(a->M), n.N = static_cast<int>(a->N), n.K = static_cast<int>(a->K);
+  n.gate0 = static_cast<int>(gate_col0);
+  n.factor = 8.f * sqrtf(static_cast<float>(a->K)) * 0x1p-24f;
+  const int64_t want = ceil_div(a->M * ((a->N + 3) / 4), 256), cap = 8ll * sm_count();
+  if (launch_pdl(near_kinks_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0, st, n) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return POM_ERR_CUDA;
+  }
+  count_launch();
+  return check_launch();
+}
 }  // extern "C"

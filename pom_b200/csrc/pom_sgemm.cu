@@ -1,9 +1,7 @@
 // float32 GEMM with FMA instructions: every output is one chain of fused multiply-adds over k = 0, 1, 2, ... from zero.
 //
-// The projections that feed the layer's kinks (activation, hardsigmoid) run here: the chain's rounding decides on which
-// side of a kink a value that all but touches it falls, and with it a whole term of the gradients, so its order is part
-// of the result.  It does not depend on the tile, the batch or the operands' storage order.  Small products and those
-// that the three-plane form (pom_gemm_f32.cu) cannot carry come here too.
+// The order does not depend on the tile, the batch or the operands' storage order.  Products with a short K, and those
+// that the three-plane form (pom_gemm_f32.cu) cannot carry, come here.
 //
 // What bounds it: FMA issue (74 TFLOP/s at 1.965 GHz; 48 reached at 4080 x 4608 x 1152, 22 with the 4 x 4
 // outputs per thread and single buffer it had before; 8 x 16 outputs at one block per SM reach 47, scalar FMAs 44).  A thread keeps TM x TN outputs, so that 4 (or 3) shared-memory

@@ -7,11 +7,11 @@ order (reference pom/pom.py:52-135) for callers that hold pre-projected features
 
 Execution paths inside ``pom_layer`` (all CUDA, chosen from dtype / mask / rotary kind):
 
-* fused     bf16, no rotary, mask None or (B, N): tcgen05 GEMMs whose epilogues do the
-            activation, polynomial, token reduction and gating (pom_ctx_gemm, pom_gate_gemm,
-            pom_gate_bwd_gemm);
-* operator  everything else (causal, rotary, fp32): plain GEMMs (tcgen05 for bf16, SIMT for
-            fp32) around the stand-alone aggregation / selection kernels.
+* fused     bf16, mask None, (B, N) or "causal", with or without rotary embedding: tcgen05 GEMMs whose
+            epilogues do the activation, polynomial, rotation, token reduction and gating
+            (pom_ctx_gemm, pom_gate_gemm, pom_gate_bwd_gemm);
+* operator  everything else (fp32, (B, T, N) masks, positions and degrees the epilogues do not take):
+            plain GEMMs on tcgen05 around the stand-alone aggregation / selection kernels.
 
 Token sharding over several GPUs (``SeqShard``) inserts the only collectives: an all-reduce
 of the (B, P) partial sums for non-causal masks, an all-gather of per-rank totals followed
@@ -395,14 +395,14 @@ class _PoMLayer(torch.autograd.Function):
                                        rope=spec.rope_ctx)
             S_part = partial  # per-tile sums; reduced (and normalised, when no exchange is needed) below
         else:
-            # float32: the projections feed the kinks of the activation and of the gate, where the rounding of a sum
-            # picks the side and with it a whole gradient term: they keep the FMA chain's order of additions
             if spec.self_mixing:
-                hs = ops.gemm(xq.view(B * T, D), w_qc, fma=True).view(B, T, P + S)
+                hs = (ops.gemm(xq.view(B * T, D), w_qc) if bf16
+                      else ops.project_f32(xq.view(B * T, D), w_qc, P, bias32)).view(B, T, P + S)
                 hp, z = hs[..., :P], hs[..., P:]
             else:
-                hp = ops.gemm(xc.view(B * N, D), w_po, fma=True).view(B, N, P)
-                z = ops.gemm(xq.view(B * T, D), w_se, fma=True).view(B, T, S)
+                hp = (ops.gemm(xc.view(B * N, D), w_po) if bf16 else ops.project_f32(xc.view(B * N, D), w_po, P)).view(B, N, P)
+                z = (ops.gemm(xq.view(B * T, D), w_se) if bf16
+                     else ops.project_f32(xq.view(B * T, D), w_se, 0, bias32)).view(B, T, S)
             if not causal and not full:
                 S_part = ops.poly_agg_fwd(hp, coeff32, row_weight=maskf, rope=spec.rope_ctx)  # per-chunk sums
         if fused_causal:

@@ -233,16 +233,53 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     else:
         if a.dtype != torch.float32 or out.dtype != torch.float32:
             raise TypeError("fp32 GEMM needs float32 operands and output")
-        if not fma and f32_planes_pay(K):
+        planes = not fma and f32_planes_pay(K)
+        if planes:
             pa, pb = a_planes or F32Planes(), b_planes or F32Planes()
             nbytes = int(L.pom_gemm_f32_planes_scratch(M, N, K, g.out_mode))
-            scratch = torch.empty((nbytes,), dtype=torch.uint8, device=dev) if nbytes else None
-            _abi.check(L.pom_gemm_f32_planes(C.byref(g), ptr(pa.take(a)), pa.ready, ptr(pb.take(b)), pb.ready,
-                                             ptr(scratch), ptr(_abi.status_word(dev)), _abi.stream_ptr()),
-                       "pom_gemm_f32_planes")
+            try:
+                bufs = pa.take(a), pb.take(b), torch.empty((nbytes,), dtype=torch.uint8, device=dev) if nbytes else None
+            except torch.OutOfMemoryError:  # a product whose operands fill the GPU: the FMA kernel needs no planes
+                planes = False
+        if planes:
+            _abi.check(L.pom_gemm_f32_planes(C.byref(g), ptr(bufs[0]), pa.ready, ptr(bufs[1]), pb.ready, ptr(bufs[2]),
+                                             ptr(_abi.status_word(dev)), _abi.stream_ptr()), "pom_gemm_f32_planes")
             pa.ready = pb.ready = 1
         else:
             _abi.check(L.pom_gemm_f32(C.byref(g), _abi.stream_ptr()), "pom_gemm_f32")
+    return out
+
+
+# float32 projections with fewer weights run on the FMA kernel alone: its one launch takes 18 us for 512 tokens at
+# 1024 x 256, the four of the tensor-core form 30.  (The tokens do not enter: see f32_planes_pay.)
+F32_PROJECT_MIN_WEIGHTS = 1 << 19
+
+
+def project_f32(x: torch.Tensor, w: torch.Tensor, ctx_cols: int, gate_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x (M, K) · wᵀ (w (N, K)), float32: columns below ``ctx_cols`` feed the activation, the others, after
+    ``gate_bias``, the gate.  On the tensor cores, with the FMA chain's own value for elements that lie next to a kink:
+    there the rounding of the sum picks the side, and with it a whole term of the gradients."""
+    M, K = x.shape
+    N = w.shape[0]
+    if N * K < F32_PROJECT_MIN_WEIGHTS or not f32_planes_pay(K):
+        return gemm(x, w, fma=True)
+    dev = _require_cuda(x, w, gate_bias)
+    out = torch.empty((M, N), dtype=torch.float32, device=dev)
+    g = GemmArgs()
+    g.A, g.Bm, g.C = ptr(x), ptr(w), ptr(out)
+    g.M, g.N, g.K = M, N, K
+    g.lda, g.ldb, g.ldc = _row_stride(x), _row_stride(w), N
+    g.batches, g.out_mode, g.split_k, g.alpha = 1, _abi.OUT_F32, 1, 1.0
+    L = _abi.lib()
+    na = (int(L.pom_f32_planes_bytes(M, K)) + 255) // 256 * 256
+    nb = (int(L.pom_f32_planes_bytes(N, K)) + 255) // 256 * 256
+    try:
+        ws = torch.empty((na + nb + 4 * (M + N),), dtype=torch.uint8, device=dev)
+    except torch.OutOfMemoryError:
+        return gemm(x, w, out=out, fma=True)
+    base = ws.data_ptr()
+    _abi.check(L.pom_project_f32(C.byref(g), base, base + na, base + na + nb, ctx_cols, ptr(gate_bias),
+                                 ptr(_abi.status_word(dev)), _abi.stream_ptr()), "pom_project_f32")
     return out
 
 

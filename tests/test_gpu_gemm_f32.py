@@ -106,3 +106,42 @@ def test_shared_planes_and_repeated_runs_give_the_same_bits():
     pl = ops.F32Planes()
     first, second = _planes(a, b, a_planes=pl), _planes(a, w, a_mn=True, a_planes=pl)
     assert torch.equal(first, _planes(a, b)) and torch.equal(second, _planes(a, w, a_mn=True))
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 128), (130, 258, 129), (500, 1000, 256), (1021, 2304, 1152)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_projection_takes_the_chain_beside_the_kinks(shape, monkeypatch):
+    """Every comparison that a derivative makes (activation at 0, 6, -10; gate at +-3) falls as the FMA chain's does, and
+    the elements closest to a kink carry the chain's bits; wide weights reach all five kinks."""
+    from pom_b200 import ops
+
+    monkeypatch.setattr(ops, "F32_PROJECT_MIN_WEIGHTS", 0)
+    M, N, K = shape
+    g = torch.Generator().manual_seed(M)
+    x = torch.randn(M, K, generator=g).cuda()
+    w = (torch.randn(N, K, generator=g) * 6 / K ** 0.5).cuda()
+    P = N // 2
+    bias = torch.randn(N - P, generator=g).cuda()
+    got, chain = ops.project_f32(x, w, P, bias), _planes(x, w, use=False, fma=True)
+    want = _gemm64(x, w, False, False)
+    assert ((got.double() - want).norm() / want.norm()).item() <= BOUND
+    eps = 2.0 ** -24 * K ** 0.5 * x.norm(dim=1)[:, None] * w.norm(dim=1)[None]  # an eighth of the kernel's own bound
+    for v, c, cut, e in ((got[:, :P], chain[:, :P], (0.0, 6.0, -10.0), eps[:, :P]),
+                         (got[:, P:] + bias, chain[:, P:] + bias, (3.0, -3.0), eps[:, P:])):
+        for k in cut:
+            assert torch.equal(v > k, c > k) and torch.equal(v < k, c < k)
+            near = (c - k).abs() <= 4 * e
+            assert torch.equal(v[near], c[near])
+    assert M * N < 100000 or bool((chain[:, :P].abs() <= 4 * eps[:, :P]).any())  # the test meets such elements
+
+
+def test_projection_of_values_that_are_not_finite(monkeypatch):
+    from pom_b200 import ops
+
+    monkeypatch.setattr(ops, "F32_PROJECT_MIN_WEIGHTS", 0)
+    x, w = _operands(70, 90, 200, False, False, 8)
+    for value in (float("inf"), float("nan"), 3e38):
+        y = x.clone()
+        y[3, 5] = value
+        a, b = ops.project_f32(y, w, 90), _planes(y, w, use=False, fma=True)
+        assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
