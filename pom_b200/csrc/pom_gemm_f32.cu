@@ -3,11 +3,11 @@
 // Every float32 operand is first written as three bf16 planes (round to nearest, then the remainders), which hold all
 // 24 bits of it: x = hi + mid + lo, |mid| <= 2^-9 |x|, |lo| <= 2^-18 |x|.  Of the nine plane products the six largest
 // are formed (hi·hi, hi·mid, mid·hi, mid·mid, hi·lo, lo·hi); the three left out are below 2^-26 of the product.
-// tcgen05 adds in fp32 but truncates, so a long sum in tensor memory drifts by about half a unit in the last place per
-// instruction.  Two measures keep the result at least as close to the exact sum as a chain of float32 FMAs:
+// A long sum in a tensor-memory accumulator is taken to lose up to a unit in its last place per instruction (how tcgen05
+// rounds is not documented).  Two measures keep the result at least as close to the exact sum as a chain of float32 FMAs:
 //   * hi·hi is summed in tensor memory over one 64-deep k-block only (four instructions); the epilogue warps add each
 //     block into registers with correctly rounded float32 additions while the next products run;
-//   * the five small products go into an accumulator of their own, whose drift is 2^-8 of the other's.
+//   * the five small products go into an accumulator of their own, whose losses are 2^-8 of the other's.
 //
 // What bounds it: the tensor pipe, six bf16 products per float32 product (229 TFLOP/s of float32 work at this card's
 // sustained bf16 rate; 4080 x 4608 x 1152 takes 193 us = 224 TFLOP/s, 1969 us with FMAs; error against 64 bits 1.1e-7,
