@@ -70,6 +70,10 @@ inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cud
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// pom_gemm_bf16 for a product whose A has zeros in the first 64 * dead_k columns of every 128-row tile that
+// `tile_weight` gives 0 (one batch, no K split): those k-blocks are left out (pom_gemm.cu).
+int gemm_bf16_dead_k(const pom_gemm_args* a, const float* tile_weight, int dead_k, int* status, cudaStream_t st);
+
 // Rotary forms of the fused tensor-core phases (pom_gemm_rope.cu), reached through pom_ctx_gemm,
 // pom_gate_gemm and pom_gate_bwd_gemm when their `rope` member names a rotary kind.
 int ctx_gemm_rope(const pom_ctx_args* a, int* status, cudaStream_t st);

@@ -105,6 +105,7 @@ struct Operands {
   int batches;
   bool a_mn, b_mn;
   const float* tile_weight = nullptr;  // optional per (batch, 128-row tile) weights: 0 skips the tile
+  int dead_k = 0;                      // ... or, > 0, starts it at this k-block
   // strided batches: element offsets between consecutive batches (0 = the matrices follow one another);
   // b_batched: the B operand has one matrix per batch too
   int64_t a_batch_stride = 0, b_batch_stride = 0;
@@ -186,6 +187,7 @@ inline GemmGeom make_geom(const Operands& o, int bn, int split_k) {
   g.split_k = static_cast<int>(ceil_div(g.k_blocks, g.kb_per_split));
   g.group_m = 8;
   g.tile_weight = o.tile_weight;
+  g.dead_k = o.dead_k;
   g.b_batched = o.b_batched ? 1 : 0;
   return g;
 }

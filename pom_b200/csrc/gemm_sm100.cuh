@@ -57,6 +57,9 @@ struct GemmGeom {
   // Optional (batches * m_tiles_per_batch) fp32: a tile whose entry is 0 is not computed (no loads, no MMAs; its
   // epilogue sees t.live == false).  Used by the context phase to skip 128-token tiles that a mask empties.
   const float* tile_weight;
+  // > 0: a tile of weight 0 is computed all the same, but from this k-block on (the blocks before it are zero in its
+  // rows of A): the data gradient of tokens that a mask empties, whose half of [dhp | dz] is zero.
+  int dead_k;
   int b_batched;          // 1: the B operand has one matrix per batch (third tensor-map coordinate = batch)
   // Rotary column pairing (0 = off): the N columns are one or two sections of 2 * pair_q channels, pair_q first
   // channels followed by their pair_q rotation partners.  The pairs of all sections, laid end to end, are cut into
@@ -80,7 +83,13 @@ struct TileCtx {
   int gp0;         // paired: index of the tile's first pair among the pairs of all sections laid end to end
   int split;       // K split index
   bool live;       // false: the main loop is skipped for this tile (see GemmGeom::tile_weight)
+  int kb_first;    // first k-block (see GemmGeom::dead_k)
 };
+
+__device__ __forceinline__ void set_tile_live(const GemmGeom& g, TileCtx& t, bool dead) {
+  t.live = !dead || g.dead_k > 0;
+  t.kb_first = dead ? g.dead_k : 0;
+}
 
 // Where pair j of a paired tile sits: its section, its index inside the section's run of first channels, the global
 // column of its first channel (the partner is pair_q columns further), and whether it exists at all.
@@ -147,7 +156,7 @@ __device__ __forceinline__ TileCtx decode_tile(const GemmGeom& g, int unit, int 
   t.row0 = t.mt * kBM;
   t.rows_valid = min(kBM, g.rows_per_batch - t.row0);
   set_tile_cols(g, t, n, bn);
-  t.live = !g.tile_weight || __ldg(g.tile_weight + m) != 0.f;
+  set_tile_live(g, t, g.tile_weight && __ldg(g.tile_weight + m) == 0.f);
   return t;
 }
 
@@ -385,8 +394,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       bool alive = true;
       for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x) {
         const TileCtx t = decode_tile(geom, unit, BN);
-        const int kb0 = t.split * geom.kb_per_split;
-        const int kb1 = t.live ? min(geom.k_blocks, kb0 + geom.kb_per_split) : kb0;
+        const int kb0 = max(t.split * geom.kb_per_split, t.kb_first);
+        const int kb1 = t.live ? min(geom.k_blocks, (t.split + 1) * geom.kb_per_split) : kb0;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag, status, kStatusProducerTimeout)) {
             alive = false;
@@ -436,8 +445,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       bool alive = true;
       for (int unit = blockIdx.x; unit < total_units && alive; unit += gridDim.x, ++iter) {
         const TileCtx t = decode_tile(geom, unit, BN);
-        const int kb0 = t.split * geom.kb_per_split;
-        const int kb1 = t.live ? min(geom.k_blocks, kb0 + geom.kb_per_split) : kb0;
+        const int kb0 = max(t.split * geom.kb_per_split, t.kb_first);
+        const int kb1 = t.live ? min(geom.k_blocks, (t.split + 1) * geom.kb_per_split) : kb0;
         const int acc = iter & 1;
         const uint32_t acc_phase = (iter >> 1) & 1u;
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1u, abort_flag, status, kStatusMmaTimeout)) {

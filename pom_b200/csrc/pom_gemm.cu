@@ -14,15 +14,16 @@ std::atomic<long long> g_launches{0};
 std::atomic<int> g_gemm_mode{0};
 }
 
-// =========================================================================== C ABI
-extern "C" {
+namespace pomh {
 
-int pom_gemm_bf16(const pom_gemm_args* a, int* status, void* stream) {
+int gemm_bf16_dead_k(const pom_gemm_args* a, const float* tile_weight, int dead_k, int* status, cudaStream_t st) {
   if (!a || !a->C) return POM_ERR_NULL;
   Operands o{a->A, a->Bm, a->M, a->N, a->K, a->lda, a->ldb, a->batches, a->a_mn_major != 0, a->b_mn_major != 0};
   o.a_batch_stride = a->a_batch_stride;
   o.b_batch_stride = a->b_batch_stride;
   o.b_batched = a->b_batched != 0;
+  o.tile_weight = dead_k > 0 ? tile_weight : nullptr;
+  o.dead_k = dead_k;
   if (a->a_batch_stride % 8 || a->b_batch_stride % 8 || a->a_batch_stride < 0 || a->b_batch_stride < 0 ||
       a->c_batch_stride < 0)
     return POM_ERR_BAD_STRIDE;
@@ -55,7 +56,16 @@ int pom_gemm_bf16(const pom_gemm_args* a, int* status, void* stream) {
   if (a->out_mode == POM_OUT_BF16 &&
       (rc = make_io_map(&maps.out0, a->C, a->N, a->M, a->batches, a->ldc, a->c_batch_stride)))
     return rc;
-  return run_plan_any_major<EpiStore>(plan, o, split, maps, ep, status, static_cast<cudaStream_t>(stream));
+  return run_plan_any_major<EpiStore>(plan, o, split, maps, ep, status, st);
+}
+
+}  // namespace pomh
+
+// =========================================================================== C ABI
+extern "C" {
+
+int pom_gemm_bf16(const pom_gemm_args* a, int* status, void* stream) {
+  return gemm_bf16_dead_k(a, nullptr, 0, status, static_cast<cudaStream_t>(stream));
 }
 
 int pom_set_gemm_mode(int mode) {

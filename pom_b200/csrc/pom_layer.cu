@@ -29,6 +29,7 @@ struct Workspace {
   uint64_t scan;          // (B, ceil(groups/32), P) fp32: scratch of pom_group_scan (both calls)
   uint64_t suf;           // (B, N, P) bf16: running sums of the gradient of the prefix means (backward)
   uint64_t gsum;          // (B, groups, P) fp32: their group totals, then carries (backward)
+  uint64_t tile_flat;     // fp32: mask weight of every 128 rows of the flattened tokens (backward, self-mixing)
   uint64_t total;
 };
 
@@ -59,6 +60,9 @@ Workspace carve(const pom_layer_args* a) {
   off = align_up(off + bp);
   w.dh2 = off;
   off = align_up(off + bp);
+  w.tile_flat = off;
+  if (a->mask && a->self_mixing)
+    off = align_up(off + (static_cast<uint64_t>(a->B) * a->N + 127) / 128 * sizeof(float));
   w.suf = w.gsum = off;
   if (a->causal) {
     if (off < fwd_end) off = fwd_end;  // past the scan scratch
@@ -104,7 +108,8 @@ const __nv_bfloat16* bf(const void* p) { return static_cast<const __nv_bfloat16*
   } while (0)
 
 int gemm(const void* A, const void* Bm, void* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc,
-         bool a_mn, bool b_mn, int out_mode, const void* residual, int64_t ldr, int* status, void* stream) {
+         bool a_mn, bool b_mn, int out_mode, const void* residual, int64_t ldr, int* status, void* stream,
+         const float* tile_weight = nullptr, int dead_k = 0) {
   pom_gemm_args g{};
   g.A = A;
   g.Bm = Bm;
@@ -123,17 +128,19 @@ int gemm(const void* A, const void* Bm, void* C, int64_t M, int64_t N, int64_t K
   g.alpha = 1.f;
   g.residual = residual;
   g.ldr = ldr;
-  return pom_gemm_bf16(&g, status, stream);
+  return gemm_bf16_dead_k(&g, tile_weight, dead_k, status, static_cast<cudaStream_t>(stream));
 }
 
 // dX (and dXc) = G·Wqc, dWqc += Gᵀ·X: the last launches of the backward call, whatever produced G = [dhp | dz].
+// `tile_flat`: a mask's weight of every 128 rows of G; rows of weight 0 have dhp = 0, and their dX is formed from the dz
+// half alone.
 int input_and_weight_grads(const pom_layer_args* a, __nv_bfloat16* G, __nv_bfloat16* g_hp, __nv_bfloat16* g_z,
-                           float* d_wqc, int* status, void* stream) {
+                           float* d_wqc, const float* tile_flat, int* status, void* stream) {
   const int D = a->D, P = a->P;
   const int64_t rows_q = static_cast<int64_t>(a->B) * a->T, rows_c = static_cast<int64_t>(a->B) * a->N;
   if (a->self_mixing) {
     POM_TRY(gemm(G, a->w_qc, a->dxq, rows_q, D, 2LL * P, 2LL * P, D, D, false, true, POM_OUT_BF16, nullptr, 0, status,
-                 stream));
+                 stream, tile_flat, tile_flat ? P / 64 : 0));
     return gemm(G, a->xq, d_wqc, 2LL * P, D, rows_q, 2LL * P, D, D, true, true, POM_OUT_F32_ACCUM, nullptr, 0, status,
                 stream);
   }
@@ -331,7 +338,7 @@ int pom_layer_bwd(const pom_layer_args* a, int* status, void* stream) {
     ab.causal = 3;
     POM_TRY(pom_poly_agg_bwd(&ab, stream));
     POM_TRY(pom_reduce_partials(ab.dcoeff_partial, d_coeff, nullptr, 1.f, 1, pom_poly_agg_bwd_slots(&ab), P * K, stream));
-    return input_and_weight_grads(a, G, g_hp, g_z, d_wqc, status, stream);
+    return input_and_weight_grads(a, G, g_hp, g_z, d_wqc, nullptr, status, stream);
   }
   POM_TRY(pom_gate_bwd_gemm(&gb, status, stream));
   float* dH = at<float>(a, w.dh);
@@ -366,7 +373,12 @@ int pom_layer_bwd(const pom_layer_args* a, int* status, void* stream) {
   ab.causal = 0;
   POM_TRY(pom_poly_agg_bwd(&ab, stream));
   POM_TRY(pom_reduce_partials(ab.dcoeff_partial, d_coeff, nullptr, 1.f, 1, pom_poly_agg_bwd_slots(&ab), P * K, stream));
-  return input_and_weight_grads(a, G, g_hp, g_z, d_wqc, status, stream);
+  const float* tile_flat = nullptr;
+  if (a->mask && a->self_mixing && rows_q <= INT32_MAX) {
+    POM_TRY(pom_tile_weights(a->mask, at<float>(a, w.tile_flat), 1, static_cast<int32_t>(rows_q), stream));
+    tile_flat = at<float>(a, w.tile_flat);
+  }
+  return input_and_weight_grads(a, G, g_hp, g_z, d_wqc, tile_flat, status, stream);
 }
 
 }  // extern "C"

@@ -708,9 +708,19 @@ agg_bwd_stream_kernel(const __grid_constant__ CUtensorMap tmx, const AggBwdDev a
   __nv_bfloat16* dxb = static_cast<__nv_bfloat16*>(a.dx) + static_cast<long long>(b) * a.N * a.ld_dx + p0;
   // One tiled bulk load brings the whole 64-token x 256-channel tile (rows and channels past the end are
   // zero-filled): per-row bulk copies were bound by the copy engine's per-request cost, not by bandwidth.
+  // A tile whose tokens all have weight 0 is neither loaded nor computed: its gradient is zero (whole warp).
+  auto dead = [&](int i) {
+    if (!a.row_weight) return false;
+    const float* w = a.row_weight + static_cast<long long>(b) * a.N;
+    const int n = (t_begin + i) * kStTok + lane;
+    const bool any = (n < a.N && __ldg(w + n) != 0.f) || (n + 32 < a.N && __ldg(w + n + 32) != 0.f);
+    return !__any_sync(0xffffffffu, any);
+  };
   auto issue = [&](int i) {  // producer warp
     const int stage = i % kStStages;
-    if (lane == 0) {
+    const bool skip = dead(i);
+    if (lane == 0 && skip) mbar_arrive(&full[stage]);
+    if (lane == 0 && !skip) {
       mbar_expect_tx(&full[stage], static_cast<uint32_t>(kStTileBytes));
       tma_load_3d(ring + stage * kStTok * kStCols, &tmx, &full[stage], p0, (t_begin + i) * kStTok, b);
     }
@@ -767,11 +777,18 @@ agg_bwd_stream_kernel(const __grid_constant__ CUtensorMap tmx, const AggBwdDev a
         issue(j);
       }
     }
+    const bool zero = dead(i);
     if (!mbar_wait(&full[stage], static_cast<uint32_t>(i / kStStages) & 1u, abort_flag, status, kStatusStreamTimeout))
       break;
     const int n0 = (t_begin + i) * kStTok;
     const int rows = min(kStTok, a.N - n0);
-    if (live) {
+    if (live && zero) {
+      for (int r = ty; r < rows; r += kGroups) {
+        __nv_bfloat16* dst = dxb + static_cast<long long>(n0 + r) * a.ld_dx + c;
+        if constexpr (VEC == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(0u, 0u);
+      }
+    } else if (live) {
 #pragma unroll 2
       for (int r = ty; r < rows; r += kGroups) {
         const int n = n0 + r;
@@ -1884,6 +1901,8 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
     (void)once_per_device(attr_done, [] {
       cudaFuncSetAttribute(agg_bwd_stream_kernel<2, kStVec, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kStSmemBytes);
+      cudaFuncSetAttribute(agg_bwd_stream_kernel<3, kStVec, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           kStSmemBytes);
       cudaFuncSetAttribute(agg_bwd_stream_kernel<4, kStVec, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kStSmemBytes);
       return static_cast<int>(POM_OK);
@@ -1895,8 +1914,8 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
       (void)launch_pdl(agg_bwd_stream_kernel<2, kStVec, true>, sgrid, dim3(threads + 32), kStSmemBytes, st, tmx, d,
                        sp.tiles_per_cta, sp.splits, status);
     else
-      (void)launch_pdl(agg_bwd_stream_kernel<4, kStVec, false>, sgrid, dim3(threads), kStSmemBytes, st, tmx, d,
-                       sp.tiles_per_cta, sp.splits, status);
+      (void)launch_pdl(a->K == 3 ? agg_bwd_stream_kernel<3, kStVec, false> : agg_bwd_stream_kernel<4, kStVec, false>, sgrid,
+                       dim3(threads), kStSmemBytes, st, tmx, d, sp.tiles_per_cta, sp.splits, status);
     count_launch();
     return check_launch();
   }
