@@ -443,17 +443,19 @@ class _PoMLayer(torch.autograd.Function):
             sh, z = ops.gate_gemm(xq, w_se, bias32, H, save_z=need_grad, rope=spec.rope_qry)
         elif heads:
             ones = _ones(B, heads, xq.device)
-            s32 = _f32(ops.select_fwd(z, bias32, ones, rope=spec.rope_qry))   # gate in head space (B, T, heads)
-            if full:  # the division by the mask's row sums rides on the (small) gate: s / rowsum, 0 for empty rows
-                s32 = s32 * _inv_rows(rowden).view(B, T, 1)
+            s32 = ops.select_fwd(z, bias32, ones, rope=spec.rope_qry)   # gate in head space (B, T, heads)
             # one aggregate per sample: the P-wide gated state and its output GEMM collapse to a (heads x D)
             # matrix per sample (pom_heads_*); per-token aggregates (causal) keep the explicit form
-            # (bf16: the batched tensor-core products of the collapsed form read rows of head_dim elements)
+            # (bf16: the batched tensor-core products of the collapsed form read rows of head_dim elements, and the gate
+            # as the selection kernel leaves it)
             collapsed = (not causal and not full and ops.heads_supported(heads, D, P)
                          and (not bf16 or (P // heads) % 8 == 0))
             if collapsed:
                 sh = ops.heads_mix(H, w_ag, heads)  # Mb (B, heads, D), kept in the slot of the gated state
             else:
+                s32 = _f32(s32)
+                if full:  # the division by the mask's row sums rides on the (small) gate: s / rowsum, 0 for empty rows
+                    s32 = s32 * _inv_rows(rowden).view(B, T, 1)
                 sh = ops.select_heads_fwd(s32, Hc if (causal or full) else H, xq.dtype)
         else:
             sh = ops.select_fwd(z, bias32, Hc if (causal or full) else H, rope=spec.rope_qry, row_denom=rowden)
@@ -577,9 +579,8 @@ class _PoMLayer(torch.autograd.Function):
                 dH = ops.reduce_partials(dh_p)
             ops.reduce_partials(db_p.view(1, -1, P), out=d_bias.view(1, P))
         elif ctx.collapsed:
-            ds32, dMb = ops.heads_out_bwd(dy, s32, sh)          # sh holds Mb here
+            ds, dMb = ops.heads_out_bwd(dy, s32, sh)            # sh holds Mb here
             dH = ops.heads_mix_bwd(dMb, H, w_ag, d_wag)         # also dWo
-            ds = ds32 if dt == torch.float32 else ops.to_bf16(ds32)
             ops.select_bwd(ds, z, bias32, _ones(B, heads, dev), g_z.view(B, T, heads), rope=spec.rope_qry,
                            dbias_out=d_bias)
         else:

@@ -808,12 +808,12 @@ def heads_mix(H: torch.Tensor, w_ag: torch.Tensor, heads: int) -> torch.Tensor:
 
 
 def heads_out_fwd(s: torch.Tensor, Mb: torch.Tensor, dtype: torch.dtype, residual: Optional[torch.Tensor] = None):
-    """y[b, t, :] = sum_h s[b, t, h] * Mb[b, h, :] (+ residual): s (B, T, heads) fp32 -> (B, T, D) of ``dtype``."""
+    """y[b, t, :] = sum_h s[b, t, h] * Mb[b, h, :] (+ residual): s (B, T, heads) and y (B, T, D) of ``dtype``."""
     dev = _require_cuda(s, Mb, residual)
     B, T, heads = s.shape
     D = Mb.shape[2]
     if dtype == torch.bfloat16:  # per sample: (T x heads) · (heads x D), the inner dimension zero-padded by TMA
-        return gemm_batched(to_bf16(s), Mb, b_mn=True, residual=residual)
+        return gemm_batched(s, Mb, b_mn=True, residual=residual)
     y = torch.empty((B, T, D), dtype=dtype, device=dev)
     a = _heads_common(B, T, D, heads, heads, dtype)  # P is not used by this call; any multiple of heads
     a.s, a.Mb, a.y, a.residual = ptr(s), ptr(Mb), ptr(y), ptr(residual)
@@ -822,14 +822,13 @@ def heads_out_fwd(s: torch.Tensor, Mb: torch.Tensor, dtype: torch.dtype, residua
 
 
 def heads_out_bwd(dy: torch.Tensor, s: torch.Tensor, Mb: torch.Tensor):
-    """Returns (ds (B, T, heads) fp32, dMb (B, heads, D) fp32)."""
+    """Returns (ds (B, T, heads), dMb (B, heads, D)) of dy's dtype (what their consumers read; the tensor-core products
+    round their fp32 sums once, as a cast behind them would)."""
     dev = _require_cuda(dy, s, Mb)
     B, T, heads = s.shape
     D = Mb.shape[2]
     if dy.dtype == torch.bfloat16:
-        ds = gemm_batched(dy, Mb, out_dtype=torch.float32)                              # (B, T, heads)
-        dMb = gemm_batched(to_bf16(s), dy, a_mn=True, b_mn=True, out_dtype=torch.float32)  # (B, heads, D)
-        return ds, dMb
+        return gemm_batched(dy, Mb), gemm_batched(s, dy, a_mn=True, b_mn=True)
     ds = torch.empty((B, T, heads), dtype=torch.float32, device=dev)
     dMb = torch.empty((B, heads, D), dtype=torch.float32, device=dev)
     part = torch.empty((B, (T + 127) // 128, heads, D), dtype=torch.float32, device=dev)
@@ -848,7 +847,7 @@ def heads_mix_bwd(dMb: torch.Tensor, H: torch.Tensor, w_ag: torch.Tensor, dwo_ac
     dH = torch.empty((B, P), dtype=torch.float32, device=dev)
     if w_ag.dtype == torch.bfloat16:
         hd = P // heads
-        g16 = to_bf16(dMb).transpose(0, 1)                       # (heads, B, D) view
+        g16 = dMb.transpose(0, 1)                                # (heads, B, D) view
         w3 = w_ag.view(D, heads, hd).transpose(0, 1)             # (heads, D, hd) view
         gemm_batched(g16, w3, b_mn=True, out=dH.view(B, heads, hd).transpose(0, 1))
         gemm_batched(g16, to_bf16(H).view(B, heads, hd).transpose(0, 1), a_mn=True, b_mn=True,
