@@ -1469,13 +1469,14 @@ __global__ void state_merge_kernel(const float* hp, const float* hc, float* hn, 
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < count) hn[i] = (n_past * hp[i] + hc[i]) / (n_past + 1.f);
 }
-// out[b, t] = sum of the 128 mask weights of tile t of sample b (one warp per tile).
+// out[b, t] = sum of the magnitudes of the 128 mask weights of tile t of sample b (one warp per tile): 0 only where
+// every weight is 0, whatever their signs.
 __global__ void tile_weights_kernel(const float* __restrict__ w, float* __restrict__ out, int N, int tiles) {
   const int t = blockIdx.x, b = blockIdx.y, lane = threadIdx.x;
   float s = 0.f;
   for (int r = lane; r < 128; r += 32) {
     const int n = t * 128 + r;
-    if (n < N) s += w[static_cast<long long>(b) * N + n];
+    if (n < N) s += fabsf(w[static_cast<long long>(b) * N + n]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);

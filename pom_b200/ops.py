@@ -358,7 +358,7 @@ def m_tiles(n_rows: int) -> int:
 
 # ---------------------------------------------------------------------------- fused GEMM phases (bf16)
 def tile_weights(mask: torch.Tensor) -> torch.Tensor:
-    """(B, N) fp32 key-padding weights -> (B, ceil(N/128)) sums per 128-token tile."""
+    """(B, N) fp32 key-padding weights -> (B, ceil(N/128)) sums of magnitudes per 128-token tile."""
     _require_cuda(mask)
     B, N = mask.shape
     out = torch.empty((B, m_tiles(N)), dtype=torch.float32, device=mask.device)

@@ -54,6 +54,36 @@ def test_skipped_tiles_change_nothing(B, N, D, E, kind, degree, monkeypatch):
         assert (a.double().cpu() - b.double()).norm() <= 2e-2 * b.double().norm()
 
 
+@pytest.mark.parametrize("kind", ["across samples", "inside a tile"])
+def test_weights_of_both_signs_that_cancel_in_a_tile(kind):
+    """A tile is left out where every weight is 0, not where the weights add up to 0."""
+    from pom_b200 import PoM
+
+    torch.manual_seed(3)
+    B, N, D = 2, (64 if kind == "across samples" else 300), 64
+    mask = torch.ones(B, N)
+    if kind == "across samples":  # 128 rows of the flattened tokens: 64 weights of 1, 64 of -1
+        mask[1] = -1
+    else:                         # the first tile of a sample
+        mask[0, :128:2] = -1
+        mask[1, 64:128] = -1
+    mod = PoM(D, 2, 2).cuda()
+    torch.nn.init.normal_(mod.po_coeff, std=0.2)
+    mod = mod.bfloat16()
+    x, dy = (torch.randn(B, N, D, device="cuda").bfloat16() for _ in range(2))
+    x.requires_grad_()
+    wrt = [x, mod.qc_proj.weight, mod.se_bias, mod.po_coeff, mod.ag_proj.weight]
+    y = mod(x, mask=mask.cuda())
+    got = [y, *torch.autograd.grad(y, wrt, dy)]
+    ps = {k: v.detach().float().cpu().requires_grad_() for k, v in mod.state_dict().items()}
+    xf = x.detach().float().cpu().requires_grad_()
+    y = O.OraclePoM(ps, 2, 2).forward(xf, None, mask)
+    names = ["qc_proj.weight", "se_bias", "po_coeff", "ag_proj.weight"]
+    want = [y, *torch.autograd.grad(y, [xf] + [ps[n] for n in names], dy.float().cpu())]
+    for a, b in zip(got, want):
+        assert (a.double().cpu() - b.double()).norm() <= 2e-2 * b.double().norm()
+
+
 def test_a_sample_without_any_valid_token():
     from pom_b200 import PoM
 
