@@ -74,6 +74,11 @@ inline cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, cud
 // `tile_weight` gives 0 (one batch, no K split): those k-blocks are left out (pom_gemm.cu).
 int gemm_bf16_dead_k(const pom_gemm_args* a, const float* tile_weight, int dead_k, int* status, cudaStream_t st);
 
+// The `tile_weight` of the data gradient: per 128 of the `rows` = B * N flattened tokens, 0 where the context half of the
+// gradient is zero because every mask weight is 0 (pom_ops.cu).
+int flat_tile_weights(const float* w, const float* dH, const float* denom, float scale, float* out, int rows, int N,
+                      int P, cudaStream_t st);
+
 // Rotary forms of the fused tensor-core phases (pom_gemm_rope.cu), reached through pom_ctx_gemm,
 // pom_gate_gemm and pom_gate_bwd_gemm when their `rope` member names a rotary kind.
 int ctx_gemm_rope(const pom_ctx_args* a, int* status, cudaStream_t st);

@@ -29,7 +29,7 @@ struct Workspace {
   uint64_t scan;          // (B, ceil(groups/32), P) fp32: scratch of pom_group_scan (both calls)
   uint64_t suf;           // (B, N, P) bf16: running sums of the gradient of the prefix means (backward)
   uint64_t gsum;          // (B, groups, P) fp32: their group totals, then carries (backward)
-  uint64_t tile_flat;     // fp32: mask weight of every 128 rows of the flattened tokens (backward, self-mixing)
+  uint64_t tile_flat;     // fp32: 0 for 128 rows of the flattened tokens that the mask empties (backward, self-mixing)
   uint64_t total;
 };
 
@@ -132,7 +132,7 @@ int gemm(const void* A, const void* Bm, void* C, int64_t M, int64_t N, int64_t K
 }
 
 // dX (and dXc) = G·Wqc, dWqc += Gᵀ·X: the last launches of the backward call, whatever produced G = [dhp | dz].
-// `tile_flat`: a mask's weight of every 128 rows of G; rows of weight 0 have dhp = 0, and their dX is formed from the dz
+// `tile_flat`: 0 for every 128 rows of G whose dhp half is zero (flat_tile_weights); their dX is formed from the dz
 // half alone.
 int input_and_weight_grads(const pom_layer_args* a, __nv_bfloat16* G, __nv_bfloat16* g_hp, __nv_bfloat16* g_z,
                            float* d_wqc, const float* tile_flat, int* status, void* stream) {
@@ -375,7 +375,8 @@ int pom_layer_bwd(const pom_layer_args* a, int* status, void* stream) {
   POM_TRY(pom_reduce_partials(ab.dcoeff_partial, d_coeff, nullptr, 1.f, 1, pom_poly_agg_bwd_slots(&ab), P * K, stream));
   const float* tile_flat = nullptr;
   if (a->mask && a->self_mixing && rows_q <= INT32_MAX) {
-    POM_TRY(pom_tile_weights(a->mask, at<float>(a, w.tile_flat), 1, static_cast<int32_t>(rows_q), stream));
+    POM_TRY(flat_tile_weights(a->mask, dH, a->denom, scale, at<float>(a, w.tile_flat), static_cast<int>(rows_q), N, P,
+                              static_cast<cudaStream_t>(stream)));
     tile_flat = at<float>(a, w.tile_flat);
   }
   return input_and_weight_grads(a, G, g_hp, g_z, d_wqc, tile_flat, status, stream);

@@ -708,7 +708,7 @@ agg_bwd_stream_kernel(const __grid_constant__ CUtensorMap tmx, const AggBwdDev a
   __nv_bfloat16* dxb = static_cast<__nv_bfloat16*>(a.dx) + static_cast<long long>(b) * a.N * a.ld_dx + p0;
   // One tiled bulk load brings the whole 64-token x 256-channel tile (rows and channels past the end are
   // zero-filled): per-row bulk copies were bound by the copy engine's per-request cost, not by bandwidth.
-  // A tile whose tokens all have weight 0 is neither loaded nor computed: its gradient is zero (whole warp).
+  // A tile whose tokens all have weight 0 is not loaded: its rows are those of one token of weight 0 (whole warp).
   auto dead = [&](int i) {
     if (!a.row_weight) return false;
     const float* w = a.row_weight + static_cast<long long>(b) * a.N;
@@ -783,10 +783,20 @@ agg_bwd_stream_kernel(const __grid_constant__ CUtensorMap tmx, const AggBwdDev a
     const int n0 = (t_begin + i) * kStTok;
     const int rows = min(kStTok, a.N - n0);
     if (live && zero) {
+      uint32_t pk[VEC / 2];
+      const float2 w2 = make_float2(0.f * wb, 0.f * wb);  // 0, or NaN where the arithmetic of a loaded tile gives NaN
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const float2 d = __fmul2_rn(w2, g[h]);
+        const float2 o = __fmul2_rn(d, pf[h][0]);
+        pk[h] = pack_bf16x2(o.x, o.y);
+#pragma unroll
+        for (int k = 0; k < KR; ++k) dc[h][k] = __ffma2_rn(d, make_float2(0.f, 0.f), dc[h][k]);
+      }
       for (int r = ty; r < rows; r += kGroups) {
         __nv_bfloat16* dst = dxb + static_cast<long long>(n0 + r) * a.ld_dx + c;
-        if constexpr (VEC == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-        else *reinterpret_cast<uint2*>(dst) = make_uint2(0u, 0u);
+        if constexpr (VEC == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        else *reinterpret_cast<uint2*>(dst) = make_uint2(pk[0], pk[1]);
       }
     } else if (live) {
 #pragma unroll 2
@@ -1483,6 +1493,24 @@ __global__ void tile_weights_kernel(const float* __restrict__ w, float* __restri
   if (lane == 0) out[static_cast<long long>(b) * tiles + t] = s;
 }
 
+// out[t] = 0 where every row of [128 t, 128 t + 128) of the flattened (B, N) tokens has weight 0 and a gradient through
+// the aggregate that is 0 for it: 0 * (scale / denom) * dH, NaN where the gradient of its sample is not finite.
+__global__ void __launch_bounds__(128) flat_tile_kernel(const float* __restrict__ w, const float* __restrict__ dH,
+                                                        const float* __restrict__ denom, float scale,
+                                                        float* __restrict__ out, int rows, int N, int P) {
+  const int r0 = blockIdx.x * 128, last = min(rows - r0, 128) - 1, tid = threadIdx.x;
+  int live = __syncthreads_or(tid <= last && w[r0 + tid] != 0.f);
+  if (!live) {
+    bool odd = false;
+    for (int b = r0 / N; b <= (r0 + last) / N; ++b) {
+      const float dn = denom[b], z = 0.f * (dn != 0.f ? scale / dn : 0.f);
+      for (int p = tid; p < P; p += 128) odd |= z * dH[static_cast<long long>(b) * P + p] != 0.f;  // NaN
+    }
+    live = __syncthreads_or(odd);
+  }
+  if (tid == 0) out[blockIdx.x] = live ? 1.f : 0.f;
+}
+
 // Rows of a mask (bool or uint8, bf16, fp32) -> the same values as rows of bf16 or fp32 `ld` apart, and the sum of every
 // row as it was given.  One pass, a warp per row and 8 values per lane and step; 6144 x 1536 bool to bf16: 7 us, where a copy to
 // bf16, one to fp32 and their row sums took 244 us.
@@ -1686,6 +1714,15 @@ int launch_reduce(const float* partial, float* out, const float* denom, float sc
 }
 
 }  // namespace
+
+namespace pomh {
+int flat_tile_weights(const float* w, const float* dH, const float* denom, float scale, float* out, int rows, int N,
+                      int P, cudaStream_t st) {
+  flat_tile_kernel<<<static_cast<unsigned>(ceil_div(rows, 128)), 128, 0, st>>>(w, dH, denom, scale, out, rows, N, P);
+  count_launch();
+  return check_launch();
+}
+}  // namespace pomh
 
 // =========================================================================== C ABI
 extern "C" {

@@ -84,6 +84,22 @@ def test_weights_of_both_signs_that_cancel_in_a_tile(kind):
         assert (a.double().cpu() - b.double()).norm() <= 2e-2 * b.double().norm()
 
 
+def test_a_gradient_that_is_not_finite_reaches_the_empty_tiles():
+    """0 times an infinite gradient of the aggregate is NaN, in a tile that the mask empties as in any other."""
+    from pom_b200 import PoM
+
+    torch.manual_seed(4)
+    B, N, D = 2, 640, 64
+    mod = PoM(D, 2, 2).cuda().bfloat16()
+    mask = torch.ones(B, N, device="cuda")
+    mask[:, 100:] = 0
+    x, dy = (torch.randn(B, N, D, device="cuda").bfloat16() for _ in range(2))
+    x.requires_grad_()
+    dy[0, 3] = float("inf")
+    dx, dcoeff = torch.autograd.grad(mod(x, mask=mask), [x, mod.po_coeff], dy)
+    assert bool(dx[0].isnan().all()) and bool(dx[1].isfinite().all()) and bool(dcoeff.isnan().any())
+
+
 def test_a_sample_without_any_valid_token():
     from pom_b200 import PoM
 
