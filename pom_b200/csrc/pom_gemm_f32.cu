@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
   if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
 }
 
-// The same with a warp per row, which also leaves the row's 2-norm (pom_project_f32).
+// The same with a warp per row, which also leaves the row's 2-norm (pom_project_f32): 0 only for a row of zeros, and never
+// too small where squares underflow (sqrt(cols) times the largest magnitude then).
 __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMat m0, const SplitMat m1,
                                                                    float* __restrict__ norms) {
   griddep_wait();
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
   const long long plane = m.rows * m.groups;
   bool bad = false;
   for (long long r = blockIdx.x * 1ll * warps + (threadIdx.x >> 5); r < m.rows; r += 1ll * m.blocks * warps) {
-    float sq = 0.f;
+    float sq = 0.f, top = 0.f;
     for (long long g = lane; g < m.groups; g += 32) {
       float v[8];
       load8(m.src + r * m.ld + g * 8, m.cols - g * 8, vec, v);
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
       for (int e = 0; e < 4; ++e) {
         bad |= !(fabsf(v[2 * e]) < 0x1p56f) || !(fabsf(v[2 * e + 1]) < 0x1p56f);
         sq = fmaf(v[2 * e], v[2 * e], fmaf(v[2 * e + 1], v[2 * e + 1], sq));
+        top = fmaxf(top, fmaxf(fabsf(v[2 * e]), fabsf(v[2 * e + 1])));
         split_pair(v[2 * e], v[2 * e + 1], p[e]);
       }
 #pragma unroll
@@ -132,8 +134,11 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
         m.dst[k * plane + r * m.groups + g] = make_uint4(p[0][k], p[1][k], p[2][k], p[3][k]);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (lane == 0) norm[r] = sqrtf(sq);
+    for (int o = 16; o > 0; o >>= 1) {
+      sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    if (lane == 0) norm[r] = sq < 0x1p-60f ? top * sqrtf(static_cast<float>(m.cols)) : sqrtf(sq);
   }
   const int any = __syncthreads_or(bad);
   if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
@@ -156,7 +161,8 @@ struct NearArgs {
 // that the FMA chain's rounding could put them on the other side get the chain's own value, bit for bit that of
 // sgemm_kernel.  Both sums are within factor * |a| |b| of one another, factor = 8 sqrt(K) 2^-24: a chain's error stays
 // below lambda sqrt(K) 2^-24 sum |a_k b_k| but for a probability of 2 exp(-lambda^2 / 2) (Higham and Mary, 2019; 8: 3e-14),
-// the planes' is a fifth of it, and sum |a_k b_k| <= |a| |b|.  One element in about 3000 is that close.
+// the planes' is a fifth of it, and sum |a_k b_k| <= |a| |b|.  Of dense inputs one element in about 3000 is that close.
+// Where a row of A or of B is all zeros (a padded token) both sums are exactly 0 and there is no chain to run.
 // The float32 training step at 4 x 1020 x 1152 takes 1429 us with this and 1952 with the FMA chain for every element.
 __global__ void __launch_bounds__(256) near_kinks_kernel(const NearArgs a) {
   griddep_wait();
@@ -178,17 +184,17 @@ __global__ void __launch_bounds__(256) near_kinks_kernel(const NearArgs a) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[e] = c0 + e < a.N ? row[e] : 0.f;
     }
-    const float na = a.factor * __ldg(a.norms + r);
+    const float na = __ldg(a.norms + r);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int c = min(c0 + e, a.N - 1);
-      const float eps = na * __ldg(a.norms + a.M + c);
+      const float nb = __ldg(a.norms + a.M + c), eps = fmaxf(a.factor * (na * nb), FLT_MIN);
       const bool gate = c >= a.gate0;
       const float x = gate ? fabsf(v[e] + __ldg(a.bias + c - a.gate0)) : v[e];
       const bool near = gate ? fabsf(x - 3.f) <= eps
                              : fabsf(x) <= eps || fabsf(x - 6.f) <= eps || fabsf(x + 10.f) <= eps;
       // (a sum that is not finite has come from the FMA kernel already)
-      uint32_t todo = __ballot_sync(0xffffffffu, on && c0 + e < a.N && near && eps < FLT_MAX);
+      uint32_t todo = __ballot_sync(0xffffffffu, on && c0 + e < a.N && near && eps < FLT_MAX && na > 0.f && nb > 0.f);
       while (todo) {  // the whole warp brings the element's two rows, 128 k ahead; every lane runs the chain
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;

@@ -145,3 +145,48 @@ def test_projection_of_values_that_are_not_finite(monkeypatch):
         y[3, 5] = value
         a, b = ops.project_f32(y, w, 90), _planes(y, w, use=False, fma=True)
         assert torch.equal(torch.nan_to_num(a, nan=7.0), torch.nan_to_num(b, nan=7.0))
+
+
+def _us(fn, runs=5):
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    times = []
+    for _ in range(runs):
+        ev[0].record()
+        fn()
+        ev[1].record()
+        torch.cuda.synchronize()
+        times.append(ev[0].elapsed_time(ev[1]) * 1e3)
+    return min(times[1:])
+
+
+def test_projection_of_zero_rows_runs_no_chains():
+    """Padded tokens and zero weight rows sit on the kink at 0 with all their elements: exactly 0 without a chain, the
+    other rows as they were, and the time of a product without them (a chain per element took a hundred times it)."""
+    from pom_b200 import ops
+
+    M, N, K = 2048, 1000, 1152
+    x, w = _operands(M, N, K, False, False, 9)
+    dense = ops.project_f32(x, w, N)
+    xz, wz = x.clone(), w.clone()
+    xz[M // 2:] = 0
+    wz[100:200] = 0
+    got = ops.project_f32(xz, wz, N)
+    keep = torch.ones(N, dtype=torch.bool, device="cuda")
+    keep[100:200] = False
+    assert torch.equal(got[:M // 2, keep], dense[:M // 2, keep])
+    assert not bool(got[M // 2:].any()) and not bool(got[:, 100:200].any())
+    assert _us(lambda: ops.project_f32(xz, wz, N)) <= 3 * _us(lambda: ops.project_f32(x, w, N))
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -75, 2.0 ** -100])
+def test_projection_beside_a_kink_where_squares_underflow(scale, monkeypatch):
+    """Rows whose 2-norm underflows in float32 still take the chain's side of the kink at 0."""
+    from pom_b200 import ops
+
+    monkeypatch.setattr(ops, "F32_PROJECT_MIN_WEIGHTS", 0)
+    x, w = _operands(256, 512, 300, False, False, 10)
+    got, chain = ops.project_f32(x * scale, w, 512), _planes(x * scale, w, use=False, fma=True)
+    assert torch.equal(got > 0, chain > 0)
+    eps = 2.0 ** -24 * 300 ** 0.5 * (x.norm(dim=1)[:, None].double() * scale * w.norm(dim=1)[None].double())
+    near = chain.abs().double() <= 4 * eps
+    assert bool(near.any()) and torch.equal(got[near], chain[near])
