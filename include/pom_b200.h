@@ -69,10 +69,12 @@ long long pom_launch_count(void);
  * no clamp).
  * step0 / step1 describe the positions that section 0 (1-D, or the row half of 2-D) and section 1 (the
  * column half) use, per aligned group of 32 tokens:  0 = the tokens of a group share one position,
- * 1 = they hold consecutive positions (base, base + 1, ...), 2 = their positions are at most 61 apart,
- * -1 = anything else.  The stand-alone operators take any positions; the fused tensor-core phases
- * (pom_ctx_gemm, pom_gate_gemm, pom_gate_bwd_gemm) need 0, 1 or 2 (token-causal: 0 or 1; they build every token's
- * angle from its group's base angle and an offset of at most 31 either way) and return POM_ERR_UNSUPPORTED otherwise.  pom_rope_pos_info computes both from the positions.
+ * 1 = they hold consecutive positions (base, base + 1, ...), 2 = their positions are at most 61 apart, 3 = as 2, and all
+ * positions lie in [0, 32), -1 = anything else.  The stand-alone operators take any positions; the fused tensor-core
+ * phases (pom_ctx_gemm, pom_gate_gemm, pom_gate_bwd_gemm) need 0 to 3 (token-causal: 0 or 1) and return
+ * POM_ERR_UNSUPPORTED otherwise.  Kinds 0, 2 and 3 rotate by each token's own table row.  Kind 1 forms the angle of token
+ * base + i from table rows `base` and i, so it needs tables of angles position * frequency (row 0 the identity): for any
+ * other table, say 2 or -1.  pom_rope_pos_info computes both from the positions.
  * ------------------------------------------------------------------------------------------ */
 typedef struct pom_rope {
   int32_t kind; /* POM_ROPE_* */
@@ -88,8 +90,9 @@ typedef struct pom_rope {
 
 /* Scans positions (n, pos_stride) int64 on the device and writes, for column c of the positions (c = 0, 1;
  * only c = 0 when pos_stride == 1), info[4c + 0] = min, info[4c + 1] = max, info[4c + 2] = 1 when every aligned
- * 32-token group is constant, info[4c + 3] = 1 when every aligned 32-token group is consecutive, else 2 when the positions
- * of every aligned 32-token group are at most 61 apart, else 0.  info is 8 int64
+ * 32-token group is constant, info[4c + 3] = 1 when every aligned 32-token group is consecutive, else 3 when the positions
+ * of every aligned 32-token group are at most 61 apart and all lie in [0, 32), else 2 when they are at most 61 apart,
+ * else 0.  info is 8 int64
  * in device memory; the call only enqueues work.  (Host helper of the rotary epilogues: no reference counterpart,
  * the reference indexes its tables with the positions directly, pom/pom_rope.py:171-172.) */
 int pom_rope_pos_info(const int64_t* pos, int64_t n, int32_t pos_stride, int64_t* info, void* stream);
@@ -168,7 +171,7 @@ int pom_project_f32(const pom_gemm_args* a, void* a_planes, void* b_planes, floa
  * 128-token tile.  partial is (B * ceil(N/128), P) fp32; reduce it with pom_reduce_partials.
  * With rope.kind != POM_ROPE_NONE the polynomial features of every token are rotated by its position before
  * the reduction (reference pom/pom_rope.py:513-515, pom_triton_rope.py:93-217): needs K <= 4, P % 16 == 0
- * (1-D) or P % 64 == 0 (2-D) and rope.step0/1 in {0, 1, 2}; otherwise POM_ERR_UNSUPPORTED (use pom_poly_agg_fwd).
+ * (1-D) or P % 64 == 0 (2-D) and rope.step0/1 in 0..3; otherwise POM_ERR_UNSUPPORTED (use pom_poly_agg_fwd).
  * Replaces: pom/pom.py:205-206 + pom/pom.py:83-91 / 35-38 (and pom_triton.py:68-153).
  * ------------------------------------------------------------------------------------------ */
 typedef struct pom_ctx_args {

@@ -131,7 +131,7 @@ struct EpiCtxCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
   }
   template <int BN>
   static __device__ __forceinline__ void prologue(const Params&, const EpiMaps&, const GemmGeom&, const TileCtx&, int,
@@ -165,7 +165,7 @@ struct EpiCtxCausal {
         for (int e = 0; e < 4; ++e) a1[e] = act_fast(v[i + e]), a2[e] = act_fast(v[16 + i + e]);
         poly4<KT, BN>(cst + 16 * su + i, p.K, a1, f1);
         poly4<KT, BN>(cst + BN / 2 + 16 * su + i, p.K, a2, f2);
-        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, false>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           v[i + e] = f1[e] * c[e] - f2[e] * s[e];
@@ -258,7 +258,7 @@ struct EpiGateCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_carry<BN>(sc.tile(slot), p.causal, g, t, lane);
   }
   // Each warp starts the load of its first `pre` blocks while the tile's main loop is still running.
@@ -320,7 +320,7 @@ struct EpiGateCausal {
         float pr1[4], pr2[4], c[4], s[4];
         read_block16_4(in, lane, i, pr1);
         read_block16_4(in + 1024, lane, i, pr2);
-        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, false>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float s1 = pom_hardsigmoid(v[i + e] + bb1[e]);
@@ -404,7 +404,7 @@ struct EpiGateBwdCausal {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, false>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_carry<BN>(sc.tile(slot), p.causal, g, t, lane);
   }
   // Each warp starts the load of its first input blocks while the tile's main loop is still running.
@@ -473,7 +473,7 @@ struct EpiGateBwdCausal {
         float pr1[4], pr2[4], c[4], s[4];
         read_block16_4(in + 2048, lane, i, pr1);
         read_block16_4(in + 3072, lane, i, pr2);
-        rope_cs4<BN, false>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, false>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float zz1 = z[i + e] + bb1[e], zz2 = z[16 + i + e] + bb2[e];

@@ -7,21 +7,21 @@
 // channels and its right half their partners, so both members of a pair sit in the same accumulator
 // rows of one CTA.  An epilogue warp walks the tile in sub-units of 16 pairs.
 //
-// cos/sin of (token, channel) never come from memory per element.  The tokens of a 32-row group (one
-// epilogue warp = one TMEM lane quarter) share one position, hold consecutive positions, or lie within 61 of one
-// another (RopeEpi::step, checked on the host), so
-//     angle(token, j) = angle(group base, j) + offset(token) * freq_j,     |offset| <= 31
-// and the epilogue combines, per pair,
-//     the table row of the group's base position (staged one tile ahead by the stager warp: 4 groups x BN/2
-//     channels), and
-//     row |offset| of the same table (cos/sin of |offset| * freq_j, the sine with the offset's sign; rows 0..31 as one
-//     32 x 16 block per sub-unit, bulk-loaded once per column block)
-// with the angle-addition formulas: 4 multiply-adds instead of two table reads per element.
-// Offsets that are not the lane number (2-D grids whose rows do not end on 32 tokens: 24 x 24, 28 x 28, ...) cost a
-// load of the token's position and two warp reductions per tile and section.  At 32 x 24 x 24 x 1152 the three
-// phases take 106 + 107 + 130 us; three plain GEMMs and the operator passes with table reads took 450.
+// cos/sin of (token, channel) are read from the tables per element only where nothing shorter is sound.  The tokens of a
+// 32-row group (one epilogue warp = one TMEM lane quarter) are of one kind per section (RopeEpi::step, found on the host):
+//   0  they share one position: the table row of that position, staged one tile ahead by the stager warp (4 groups x BN/2
+//      channels);
+//   1  they hold consecutive positions: angle(lane, j) = angle(group base, j) + lane * freq_j, formed from the staged base
+//      row and row `lane` of the same table (rows 0..31 as one 32 x 16 block per sub-unit, bulk-loaded once per column
+//      block) by the angle-addition formulas, 4 multiply-adds per pair.  This needs tables whose rows are the angles
+//      position * freq (row 0 is the identity);
+//   2  they span at most 61 positions: every token's own row, from global memory (a warp's rows stay in L1);
+//   3  all positions of the launch are below 32: every token's own row, from the blocks of rows 0..31.
+// Kinds 2 and 3 are 2-D grids whose rows do not end on 32 tokens (24 x 24, 28 x 28, ...); any table will do for them, and
+// a rounded one is used as it is.  A training step of 18 432 tokens x 1152 (bf16, degree 2, expansion 2), against the
+// operators: 24 x 24 (kind 3) 910 us and 1067, 14 x 40 (kind 2) 1004 and 1054, 9 x 61 992 and 1053; 32 x 32 (kinds 0
+// and 1) 879.  The line at 61 is where these were measured; wider groups read more rows and take the operators.
 #pragma once
-#include <climits>
 #include "epilogues.cuh"
 
 namespace pomk {
@@ -32,7 +32,7 @@ struct RopeEpi {
   const long long* pos;  // (rows, pos_stride) int64 token positions; section s reads column s (pos_stride 2)
   int pos_stride;
   int len[2];
-  int step[2];           // the tokens of an aligned 32-token group: 0 share one position; 1 consecutive; 2 span <= 61
+  int step[2];           // of an aligned 32-token group: 0 shared position; 1 consecutive; 2 span <= 61; 3 all below 32
   int rotate;            // 0: no rotation at all (cos = 1, sin = 0; tables and positions are not read)
   // selections by ternary keep the kernel parameters out of local memory (no dynamically indexed arrays)
   __device__ __forceinline__ int step_of(int sec) const { return sec ? step[1] : step[0]; }
@@ -78,40 +78,25 @@ __device__ __forceinline__ int rope_pos(const RopeEpi& r, int n, int sec) {
   const int len = r.len_of(sec);
   return p < 0 ? 0 : p >= len ? len - 1 : static_cast<int>(p);
 }
-// Base of the 32-token group that starts at token n0 (whole warp; `own` receives the lane's own position): the first
-// token's position, or, where they only span <= 61, the smallest from which none is more than 31 away.
-__device__ __forceinline__ int rope_group_base(const RopeEpi& r, int n0, int rows, int sec, int lane, int& own) {
-  const bool ok = n0 + lane < rows;
-  own = ok ? rope_pos(r, n0 + lane, sec) : 0;
-  const int lo = __reduce_min_sync(0xffffffffu, ok ? own : INT_MAX);
-  const int hi = __reduce_max_sync(0xffffffffu, ok ? own : 0);
-  const int base = max(lo, hi - 31);
-  if (!ok) own = base;
-  return base;
-}
 
-// What an epilogue warp needs of the rotary constants of its tile.  SPAN: offsets other than the lane number are
-// possible (the token-causal epilogues, which have no registers left for them, never see such positions).
-template <bool SPAN>
+// What an epilogue warp needs of the rotary constants of its tile.  OWN: kinds 2 and 3 of RopeEpi::step are possible (the
+// token-causal epilogues, which have no registers left for them, never see such positions).
+template <bool OWN>
 struct RopeView {
   const float* base_cos;  // [4 quarters][BN/2]
   const float* base_sin;
   const uint8_t* lane;
-  int row[2];        // per section: row of the lane tables that holds this token's offset
-  uint32_t flip[2];  // sign bit of a negative offset
+  int row[2];             // per section: the table row of this token (kinds 2, 3), else the lane
   __device__ __forceinline__ RopeView(const RopeEpi& r, const GemmGeom& g, const TileCtx& t, int quarter, int lane_id,
                                       const float* bc, const float* bs, const uint8_t* lt)
       : base_cos(bc), base_sin(bs), lane(lt) {
 #pragma unroll
     for (int sec = 0; sec < 2; ++sec) {
       row[sec] = lane_id;
-      flip[sec] = 0;
-      const int n0 = t.row0 + 32 * quarter;
-      if (SPAN && r.rotate && r.step_of(sec) == 2 && n0 < g.rows_per_batch && (sec == 0 || r.pos_stride == 2)) {
-        int own;
-        const int d = -rope_group_base(r, n0, g.rows_per_batch, sec, lane_id, own) + own;
-        row[sec] = abs(d);
-        flip[sec] = d < 0 ? 0x80000000u : 0u;
+      if (OWN && r.step_of(sec) >= 2 && (sec == 0 || r.pos_stride == 2)) {
+        const int n = t.row0 + 32 * quarter + lane_id;
+        row[sec] = n < g.rows_per_batch ? rope_pos(r, n, sec) : 0;
+        if (r.step_of(sec) == 3) row[sec] &= 31;  // the kind promises it: keeps a read inside the block
       }
     }
   }
@@ -125,7 +110,7 @@ __device__ __forceinline__ uint32_t rope_stage_lane(const RopeEpi& r, const EpiM
   uint32_t bytes = 0;
   for (int su = 0; su < BN / 32; ++su) {
     const PairPos pp = pair_pos(g, t, 16 * su);
-    if (!pp.ok || r.step_of(pp.sec) == 0) continue;  // no pairs, or one position per row group: no lane table
+    if (!pp.ok || !(r.step_of(pp.sec) & 1)) continue;  // no pairs, or no use for the first 32 rows
     if (lane == 0) {
       tma_load_2d(lane_tab + su * 4096, &maps.lane[2 * pp.sec], bar, pp.u, 0);
       tma_load_2d(lane_tab + su * 4096 + 2048, &maps.lane[2 * pp.sec + 1], bar, pp.u, 0);
@@ -138,7 +123,7 @@ __device__ __forceinline__ uint32_t rope_stage_lane(const RopeEpi& r, const EpiM
 // Stager warp: cos / sin of the base position of the tile's four 32-row groups for its BN/2 pairs, four pairs per
 // load (pair_q and the tile's first pair are multiples of 4, the tables 16-byte aligned: the lane-table tensor maps
 // have the same needs).
-template <int BN, bool SPAN>
+template <int BN>
 __device__ __forceinline__ void rope_stage_base(const RopeEpi& r, const GemmGeom& g, const TileCtx& t, int lane,
                                                 float* base_cos, float* base_sin) {
   constexpr int kHalf = BN / 2;
@@ -149,12 +134,8 @@ __device__ __forceinline__ void rope_stage_base(const RopeEpi& r, const GemmGeom
     const int n = t.row0 + 32 * quarter;
 #pragma unroll
     for (int sec = 0; sec < 2; ++sec) {
-      int p = 0;
-      if (r.rotate && n < g.rows_per_batch && (sec == 0 || r.pos_stride == 2)) {
-        int own;
-        p = SPAN && r.step_of(sec) == 2 ? rope_group_base(r, n, g.rows_per_batch, sec, lane, own) : rope_pos(r, n, sec);
-      }
-      pos[quarter][sec] = p;
+      pos[quarter][sec] =
+          r.rotate && n < g.rows_per_batch && (sec == 0 || r.pos_stride == 2) ? rope_pos(r, n, sec) : 0;
     }
   }
   static_assert((4 * kVec) % 32 == 0, "tile width");
@@ -194,31 +175,39 @@ __device__ __forceinline__ bool tail_last_warp(EpiIO& io, int parity, int lane) 
   return true;
 }
 
-// cos/sin of this lane's token for pairs [16 su + i, 16 su + i + 4) of the tile; `step`: RopeEpi::step of the
-// sub-unit's section `sec`.
-template <int BN, bool SPAN>
-__device__ __forceinline__ void rope_cs4(const RopeView<SPAN>& rs, int step, int sec, int quarter, int su, int i,
-                                         float (&c)[4], float (&s)[4]) {
-  const float4 C0 = *reinterpret_cast<const float4*>(rs.base_cos + quarter * (BN / 2) + 16 * su + i);
-  const float4 S0 = *reinterpret_cast<const float4*>(rs.base_sin + quarter * (BN / 2) + 16 * su + i);
-  if (step) {
-    const uint8_t* blk = rs.lane + su * 4096;
-    const int row = SPAN && sec ? rs.row[1] : rs.row[0];
-    const float4 cl = *reinterpret_cast<const float4*>(blk + swz64(row, i >> 2));
-    float4 sl = *reinterpret_cast<const float4*>(blk + 2048 + swz64(row, i >> 2));
-    if (SPAN && step == 2) {
-      const uint32_t f = sec ? rs.flip[1] : rs.flip[0];
-      sl.x = __uint_as_float(__float_as_uint(sl.x) ^ f), sl.y = __uint_as_float(__float_as_uint(sl.y) ^ f);
-      sl.z = __uint_as_float(__float_as_uint(sl.z) ^ f), sl.w = __uint_as_float(__float_as_uint(sl.w) ^ f);
+// cos/sin of this lane's token for pairs [16 su + i, 16 su + i + 4) of the tile, which start at pair pp.u + i of the
+// sub-unit's section; `step`: RopeEpi::step of that section.
+template <int BN, bool OWN>
+__device__ __forceinline__ void rope_cs4(const RopeEpi& r, const RopeView<OWN>& rs, const GemmGeom& g, const PairPos& pp,
+                                         int step, int quarter, int su, int i, float (&c)[4], float (&s)[4]) {
+  float4 cc, ss;
+  const int row = pp.sec ? rs.row[1] : rs.row[0];
+  if (OWN && step >= 2) {
+    if (step == 2) {
+      const long long o = static_cast<long long>(row) * g.pair_q + pp.u + i;
+      cc = __ldg(reinterpret_cast<const float4*>(r.cos_of(pp.sec) + o));
+      ss = __ldg(reinterpret_cast<const float4*>(r.sin_of(pp.sec) + o));
+    } else {
+      const uint8_t* blk = rs.lane + su * 4096;
+      cc = *reinterpret_cast<const float4*>(blk + swz64(row, i >> 2));
+      ss = *reinterpret_cast<const float4*>(blk + 2048 + swz64(row, i >> 2));
     }
-    c[0] = C0.x * cl.x - S0.x * sl.x, s[0] = S0.x * cl.x + C0.x * sl.x;
-    c[1] = C0.y * cl.y - S0.y * sl.y, s[1] = S0.y * cl.y + C0.y * sl.y;
-    c[2] = C0.z * cl.z - S0.z * sl.z, s[2] = S0.z * cl.z + C0.z * sl.z;
-    c[3] = C0.w * cl.w - S0.w * sl.w, s[3] = S0.w * cl.w + C0.w * sl.w;
   } else {
-    c[0] = C0.x, c[1] = C0.y, c[2] = C0.z, c[3] = C0.w;
-    s[0] = S0.x, s[1] = S0.y, s[2] = S0.z, s[3] = S0.w;
+    cc = *reinterpret_cast<const float4*>(rs.base_cos + quarter * (BN / 2) + 16 * su + i);
+    ss = *reinterpret_cast<const float4*>(rs.base_sin + quarter * (BN / 2) + 16 * su + i);
+    if (step) {
+      const uint8_t* blk = rs.lane + su * 4096;
+      const float4 C0 = cc, S0 = ss;
+      const float4 cl = *reinterpret_cast<const float4*>(blk + swz64(row, i >> 2));
+      const float4 sl = *reinterpret_cast<const float4*>(blk + 2048 + swz64(row, i >> 2));
+      cc = make_float4(C0.x * cl.x - S0.x * sl.x, C0.y * cl.y - S0.y * sl.y, C0.z * cl.z - S0.z * sl.z,
+                       C0.w * cl.w - S0.w * sl.w);
+      ss = make_float4(S0.x * cl.x + C0.x * sl.x, S0.y * cl.y + C0.y * sl.y, S0.z * cl.z + C0.z * sl.z,
+                       S0.w * cl.w + C0.w * sl.w);
+    }
   }
+  c[0] = cc.x, c[1] = cc.y, c[2] = cc.z, c[3] = cc.w;
+  s[0] = ss.x, s[1] = ss.y, s[2] = ss.z, s[3] = ss.w;
 }
 
 // Global column of tile column c (left half: first channels, right half: partners) and whether it exists.
@@ -306,7 +295,7 @@ struct EpiCtxRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
   }
   template <int BN>
   static __device__ __forceinline__ void prologue(const Params&, const EpiMaps&, const GemmGeom&, const TileCtx&, int,
@@ -363,7 +352,7 @@ struct EpiCtxRope {
         for (int e = 0; e < 4; ++e) a1[e] = act_fast(v[i + e]), a2[e] = act_fast(v[16 + i + e]);
         poly4<KT, BN>(cst + 16 * su + i, p.K, a1, f1);
         poly4<KT, BN>(cst + BN / 2 + 16 * su + i, p.K, a2, f2);
-        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, true>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float r1 = f1[e] * c[e] - f2[e] * s[e];
@@ -449,7 +438,7 @@ struct EpiGateRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_paired_vector<BN>(sc.tile(slot), p.H + static_cast<long long>(t.b) * p.h_batch_stride, g, t, lane);
   }
   template <int BN>
@@ -488,7 +477,7 @@ struct EpiGateRope {
         const float bb1[4] = {b1.x, b1.y, b1.z, b1.w}, bb2[4] = {b2.x, b2.y, b2.z, b2.w};
         const float hh1[4] = {h1.x, h1.y, h1.z, h1.w}, hh2[4] = {h2.x, h2.y, h2.z, h2.w};
         float c[4], s[4];
-        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, true>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float s1 = pom_hardsigmoid(v[i + e] + bb1[e]);
@@ -573,7 +562,7 @@ struct EpiGateBwdRope {
   static __device__ __forceinline__ void stage_tile(const Params& p, const EpiMaps&, const GemmGeom& g,
                                                     const TileCtx& t, int lane, float* scratch, int slot) {
     const Scratch<BN> sc(scratch);
-    rope_stage_base<BN, true>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
+    rope_stage_base<BN>(p.rope, g, t, lane, sc.base_cos(slot), sc.base_sin(slot));
     stage_paired_vector<BN>(sc.tile(slot), p.H + static_cast<long long>(t.b) * p.h_batch_stride, g, t, lane);
   }
   // Each warp starts the load of its first z blocks while the tile's main loop is still running.
@@ -636,7 +625,7 @@ struct EpiGateBwdRope {
         const float bb1[4] = {b1.x, b1.y, b1.z, b1.w}, bb2[4] = {b2.x, b2.y, b2.z, b2.w};
         const float hh1[4] = {h1.x, h1.y, h1.z, h1.w}, hh2[4] = {h2.x, h2.y, h2.z, h2.w};
         float c[4], s[4];
-        rope_cs4<BN, true>(rs, step, pp.sec, quarter, su, i, c, s);
+        rope_cs4<BN, true>(p.rope, rs, g, pp, step, quarter, su, i, c, s);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float zz1 = z[i + e] + bb1[e], zz2 = z[16 + i + e] + bb2[e];

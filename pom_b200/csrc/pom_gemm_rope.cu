@@ -44,7 +44,7 @@ int make_rope(const pom_rope& r, const PairShape& ps, RopeEpi* e, EpiMaps* maps)
   e->step[0] = r.step0, e->step[1] = ps.sections == 2 ? r.step1 : r.step0;
   for (int s = 0; s < ps.sections; ++s) {
     if (e->len[s] < 1) return POM_ERR_BAD_SHAPE;
-    if (e->step[s] < 0 || e->step[s] > 2) return POM_ERR_UNSUPPORTED;
+    if (e->step[s] < 0 || e->step[s] > 3) return POM_ERR_UNSUPPORTED;
     int rc;
     if ((rc = make_lane_table_map(&maps->lane[2 * s], e->cos[s], ps.q, e->len[s]))) return rc;
     if ((rc = make_lane_table_map(&maps->lane[2 * s + 1], e->sin[s], ps.q, e->len[s]))) return rc;
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(1024) rope_pos_info_kernel(const long long* __
       flat &= s_flat[c][w];
       step &= s_step[c][w];
     }
-    info[4 * c + 0] = mn, info[4 * c + 1] = mx, info[4 * c + 2] = flat, info[4 * c + 3] = (step & 1) ? 1 : step;
+    info[4 * c + 0] = mn, info[4 * c + 1] = mx, info[4 * c + 2] = flat, info[4 * c + 3] = (step & 1) ? 1 : step == 2 && mn >= 0 && mx < 32 ? 3 : step;
   }
 }
 

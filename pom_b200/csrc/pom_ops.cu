@@ -880,8 +880,9 @@ agg_bwd_stream_kernel(const __grid_constant__ CUtensorMap tmx, const AggBwdDev a
 // their 4 partners.  The gradient reaching token n is the transposed rotation of dH by that token's angle
 // (reference pom/pom_rope.py:171-180, 208-235; backward of pom_triton_rope.py:227-475).
 //
-// No table row is read per token.  The positions of every aligned group of 32 tokens are constant or consecutive
-// (pom_rope::step0/1), so angle(token) = angle(group base) + lane * step * freq: a thread visits rows ty, ty + 8,
+// TABLE (positions of kind 2 or 3, pom_rope::step0/1): every token's own table row is read; the rows of the block's 128
+// channels stay in L1.  Otherwise no table row is read per token: the positions of every aligned group of 32 tokens are
+// constant or consecutive, so angle(token) = angle(group base) + lane * step * freq: a thread visits rows ty, ty + 8,
 // ... of each 64-token tile, i.e. four lane offsets that never change, whose cos/sin it keeps in registers for the
 // whole run; per tile it fetches the table rows of the two group bases (two 16-byte loads each) while the tile is
 // still landing, and combines both with the angle-addition formulas.
@@ -890,8 +891,6 @@ constexpr int kStHalf = kStCols / 2;
 // CAUSAL (the fused token-causal layer): tiles are one 32-token group; beside hp the ring carries `suf`, the
 // running sums (up the group's rows) of the gradient of the prefix means written by the causal gate-backward
 // epilogue, and the gradient of token n's features is suf[n] + carry[group] instead of w[n]·dH.
-// TABLE: positions of any order; every token's table row is read (the rows of the block's 128 channels stay in L1)
-// instead of being built from its group's base row.
 template <int KR, bool CAUSAL, bool TABLE>
 __global__ void __launch_bounds__(256, 2)
 agg_bwd_stream_pair_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tms,
@@ -1194,7 +1193,7 @@ bool stream_bwd_rope_eligible(const pom_agg_bwd_args* a) {
   if (a->rope.kind == POM_ROPE_NONE)
     return a->ldx % 8 == 0 && a->ld_dx % 8 == 0 && aligned16(a->x) && aligned16(a->dx);
   if (a->rope.pos_stride != sp.sections || a->rope.len0 < 1 || (sp.sections == 2 && a->rope.len1 < 1)) return false;
-  const int most = a->causal == 3 ? 1 : 2;  // the token-causal layer takes shared and consecutive positions only
+  const int most = a->causal == 3 ? 1 : 3;  // the token-causal layer takes shared and consecutive positions only
   if (a->rope.step0 < 0 || a->rope.step0 > most || (sp.sections == 2 && (a->rope.step1 < 0 || a->rope.step1 > most)))
     return false;
   if (a->ldx % 8 || a->ld_dx % 8 || !aligned16(a->x) || !aligned16(a->dx)) return false;
@@ -1979,7 +1978,7 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
     if ((rc = stream_tile_map(&tmx, a->x, a->P, a->N, a->B, a->ldx, kStHalf, tt))) return rc;
     tms = tmx;
     if (fused_causal && (rc = stream_tile_map(&tms, a->dout, a->P, a->N, a->B, a->ld_dout, kStHalf, tt))) return rc;
-    const bool table = a->rope.kind != POM_ROPE_NONE && (a->rope.step0 == 2 || (pr.sections == 2 && a->rope.step1 == 2));
+    const bool table = a->rope.kind != POM_ROPE_NONE && (a->rope.step0 >= 2 || (pr.sections == 2 && a->rope.step1 >= 2));
     const auto kern = fused_causal ? (a->K <= 2 ? agg_bwd_stream_pair_kernel<2, true, false> : agg_bwd_stream_pair_kernel<4, true, false>)
                       : table      ? agg_bwd_stream_pair_kernel<2, false, true>
                                    : agg_bwd_stream_pair_kernel<2, false, false>;

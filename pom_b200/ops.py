@@ -78,8 +78,9 @@ class RopeSpec:
     cos1: Optional[torch.Tensor] = None
     sin1: Optional[torch.Tensor] = None
     # per position column, how the positions of every aligned group of 32 tokens look: 0 = one shared position,
-    # 1 = consecutive positions, 2 = at most 61 apart, -1 = anything else / unknown (see rope_pos_info); the fused
-    # tensor-core phases need 0 to 2 (token-causal: 0 or 1), the stand-alone operators take any positions
+    # 1 = consecutive positions, 2 = at most 61 apart, 3 = as 2 and all in [0, 32), -1 = anything else / unknown (see
+    # rope_pos_info); the fused tensor-core phases need 0 to 3 (token-causal: 0 or 1), the stand-alone operators take any
+    # positions.  Kind 1 expects tables of angles position * frequency: token base + i is rotated by rows base and i
     steps: Tuple[int, int] = (-1, -1)
 
     def to_c(self) -> Rope:
@@ -96,7 +97,7 @@ class RopeSpec:
 
     def fusable(self, p: int, causal: bool = False) -> bool:
         """Whether the rotary GEMM epilogues can take this description for p channels."""
-        if causal and 2 in self.steps:
+        if causal and max(self.steps) >= 2:
             return False
         if self.kind == _abi.ROPE_1D:
             return p % 16 == 0 and self.cos0.shape[1] == p // 2 and self.steps[0] >= 0
