@@ -149,9 +149,9 @@ int pom_gemm_f32(const pom_gemm_args* a, void* stream);
  * that hold all its bits, and the six largest plane products are summed (batches must be 1; any strides, sizes and
  * alignment).  `a_planes` / `b_planes`: 16-byte aligned buffers of pom_f32_planes_bytes(rows, cols) of the operand as
  * it is stored; *_ready != 0 when an earlier call with the same operand (whichever major it was read in) has filled
- * them.  `scratch`: pom_gemm_f32_planes_scratch bytes (0: may be NULL).  Operands with infinities, NaN or magnitudes of
- * 2^56 and more are computed by the FMA kernel, which is always enqueued behind the product and returns at once
- * otherwise.  Results are the same bits on every run; K is split (partial sums in `scratch`) in accumulate mode only, so
+ * them.  `scratch`: pom_gemm_f32_planes_scratch bytes (0: may be NULL).  Operands with infinities or NaN, with
+ * magnitudes whose largest product times K reaches 2^78, or whose smallest product (of two nonzero values) is below
+ * 2^-148, are computed by the FMA kernel, which is always enqueued behind the product and returns at once otherwise.  Results are the same bits on every run; K is split (partial sums in `scratch`) in accumulate mode only, so
  * that a row of a plain product does not depend on how many rows there are. */
 uint64_t pom_f32_planes_bytes(int64_t rows, int64_t cols);
 uint64_t pom_gemm_f32_planes_scratch(int64_t M, int64_t N, int64_t K, int32_t out_mode);

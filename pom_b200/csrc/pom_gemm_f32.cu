@@ -1,8 +1,10 @@
 // float32 GEMM on the tensor cores: C[m, n] = alpha * sum_k A[m, k] * B[n, k] with the accuracy of float32 sums.
 //
-// Every float32 operand is first written as three bf16 planes (round to nearest, then the remainders), which hold all
-// 24 bits of it: x = hi + mid + lo, |mid| <= 2^-9 |x|, |lo| <= 2^-18 |x|.  Of the nine plane products the six largest
-// are formed (hi·hi, hi·mid, mid·hi, mid·mid, hi·lo, lo·hi); the three left out are below 2^-26 of the product.
+// Every float32 operand is first written as three bf16 planes of 2^24 x (round to nearest, then the remainders), which
+// hold all 24 bits of it: 2^24 x = hi + mid + lo, |mid| <= 2^-9 |hi|, |lo| <= 2^-18 |hi| (without the factor the last
+// bits of |x| < 2^-110 would fall under bf16's range).  Of the nine plane products the six largest are formed (hi·hi,
+// hi·mid, mid·hi, mid·mid, hi·lo, lo·hi); the three left out are below 2^-26 of the product.  The sum times 2^-48 is the
+// result.
 // A long sum in a tensor-memory accumulator is taken to lose up to a unit in its last place per instruction (how tcgen05
 // rounds is not documented).  Two measures keep the result at least as close to the exact sum as a chain of float32 FMAs:
 //   * hi·hi is summed in tensor memory over one 64-deep k-block only (four instructions); the epilogue warps add each
@@ -14,9 +16,11 @@
 // 6.1e-7 with FMAs).  A pair tile of 256 x 256 loads 96 KB per SM and k-block for 3072 tensor cycles (32 B/clk/SM,
 // half of what the bf16 kernels ask of L2), so two stages of three planes are enough.
 //
-// Infinities, NaN and magnitudes of 2^56 or more (whose plane products could meet with opposite signs) do not go
-// through the planes: the split marks them and the FMA kernel (sgemm_kernel) computes that product instead, on the
-// device, without a host decision.
+// Operands whose products could leave the range in which all of this holds do not go through the planes.  The split notes
+// the exponents of the largest and the smallest magnitude (but zero) of either operand.  The largest product times K has to
+// stay below 2^78 (2^126 with the factors: no sum overflows), the smallest at or above 2^-148 (2^-100 with the factors:
+// no plane product that counts falls under 2^-126, where a tensor core may take it for zero).  Otherwise, and for
+// infinities and NaN, the FMA kernel (sgemm_kernel) computes the product, decided on the device without the host.
 #include <cfloat>
 #include <cmath>
 #include <cudaTypedefs.h>
@@ -33,6 +37,7 @@ constexpr int kFlagWords = 1024;                // one word per block of the spl
 constexpr int kFlagBytes = kFlagWords * 4;
 constexpr int kSplitThreads = 256;
 constexpr int kF32Threads = 32 * 10;            // producer, MMA issuer, eight epilogue warps
+constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;  // of an operand's planes, of a product of two
 constexpr int kMinSplitBlocks = 2;              // k-blocks that a K split keeps at least
 
 inline int64_t plane_ld(int64_t cols) { return (cols + 7) / 8 * 8; }
@@ -52,7 +57,7 @@ inline __nv_bfloat16* planes_of(void* buf) {
 struct SplitMat {
   const float* src;
   uint4* dst;       // three planes of rows x ldp bf16
-  int* flags;       // word of every block: 1 when it met a value the planes cannot carry
+  int* flags;       // word of every block: exponents of its largest and smallest magnitudes (SgemmFlags)
   long long rows, cols, ld, groups;  // groups of 8 columns per row
   int blocks;
 };
@@ -68,7 +73,32 @@ __device__ __forceinline__ void load8(const float* s, long long left, bool vec, 
   }
 }
 
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&o)[3]) {
+// Largest and smallest magnitude (but zero) of the values a thread splits, as bits.
+struct Extremes {
+  uint32_t hi = 0, lo = 0x7f800000u;
+  __device__ __forceinline__ void see(float x) {
+    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+    hi = max(hi, u);
+    lo = min(lo, u ? u : lo);
+  }
+  // The word of the block (every thread calls it once).
+  __device__ __forceinline__ void store(int* word) const {
+    __shared__ uint32_t sh[2][kSplitThreads / 32];
+    const uint32_t h = __reduce_max_sync(0xffffffffu, hi), l = __reduce_min_sync(0xffffffffu, lo);
+    if ((threadIdx.x & 31) == 0) sh[0][threadIdx.x >> 5] = h, sh[1][threadIdx.x >> 5] = l;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t a = sh[0][0], b = sh[1][0];
+      for (int w = 1; w < kSplitThreads / 32; ++w) a = max(a, sh[0][w]), b = min(b, sh[1][w]);
+      *word = static_cast<int>(a >> 23 << 16 | b >> 23);
+    }
+  }
+};
+
+// Planes of 2^24 a and 2^24 b.
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t (&o)[3], Extremes& x) {
+  a *= kScale, b *= kScale;
+  x.see(a), x.see(b);
   o[0] = pack_bf16x2(a, b);
   a -= __uint_as_float(o[0] << 16), b -= __uint_as_float(o[0] & 0xffff0000u);
   o[1] = pack_bf16x2(a, b);
@@ -85,7 +115,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
   if (static_cast<int>(blockIdx.x) >= m.blocks) return;
   const long long total = m.rows * m.groups, plane = total;
   const bool vec = (m.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0;
-  bool bad = false;
+  Extremes seen;
   for (long long i = blockIdx.x * 1ll * kSplitThreads + threadIdx.x; i < total; i += 1ll * m.blocks * kSplitThreads) {
     const long long r = i / m.groups, c = (i - r * m.groups) * 8;
     float v[8];
@@ -93,14 +123,12 @@ __global__ void __launch_bounds__(kSplitThreads) split_planes_kernel(const Split
     uint32_t p[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      bad |= !(fabsf(v[2 * e]) < 0x1p56f) || !(fabsf(v[2 * e + 1]) < 0x1p56f);
-      split_pair(v[2 * e], v[2 * e + 1], p[e]);
+      split_pair(v[2 * e], v[2 * e + 1], p[e], seen);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) m.dst[k * plane + i] = make_uint4(p[0][k], p[1][k], p[2][k], p[3][k]);
   }
-  const int any = __syncthreads_or(bad);
-  if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
+  seen.store(m.flags + blockIdx.x);
 }
 
 // The same with a warp per row, which also leaves the row's 2-norm (pom_project_f32): 0 only for a row of zeros, and never
@@ -115,7 +143,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
   const int lane = threadIdx.x & 31, warps = kSplitThreads / 32;
   const bool vec = (m.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(m.src) & 15) == 0;
   const long long plane = m.rows * m.groups;
-  bool bad = false;
+  Extremes seen;
   for (long long r = blockIdx.x * 1ll * warps + (threadIdx.x >> 5); r < m.rows; r += 1ll * m.blocks * warps) {
     float sq = 0.f, top = 0.f;
     for (long long g = lane; g < m.groups; g += 32) {
@@ -124,10 +152,9 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
       uint32_t p[4][3];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        bad |= !(fabsf(v[2 * e]) < 0x1p56f) || !(fabsf(v[2 * e + 1]) < 0x1p56f);
         sq = fmaf(v[2 * e], v[2 * e], fmaf(v[2 * e + 1], v[2 * e + 1], sq));
         top = fmaxf(top, fmaxf(fabsf(v[2 * e]), fabsf(v[2 * e + 1])));
-        split_pair(v[2 * e], v[2 * e + 1], p[e]);
+        split_pair(v[2 * e], v[2 * e + 1], p[e], seen);
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k)
@@ -140,8 +167,7 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
     }
     if (lane == 0) norm[r] = sq < 0x1p-60f ? top * sqrtf(static_cast<float>(m.cols)) : sqrtf(sq);
   }
-  const int any = __syncthreads_or(bad);
-  if (threadIdx.x == 0) m.flags[blockIdx.x] = any;
+  seen.store(m.flags + blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------- chain values beside the kinks
@@ -451,8 +477,8 @@ gemm_f32_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         if (left >= 32 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float4 v = make_float4(out.alpha * acc[c][4 * j], out.alpha * acc[c][4 * j + 1],
-                                   out.alpha * acc[c][4 * j + 2], out.alpha * acc[c][4 * j + 3]);
+            float4 v = make_float4(out.alpha * (kUnscale * acc[c][4 * j]), out.alpha * (kUnscale * acc[c][4 * j + 1]),
+                                   out.alpha * (kUnscale * acc[c][4 * j + 2]), out.alpha * (kUnscale * acc[c][4 * j + 3]));
             float4* q = reinterpret_cast<float4*>(d) + j;
             if (out.accumulate) {
               const float4 o = *q;
@@ -463,7 +489,10 @@ gemm_f32_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (i < left) d[i] = out.accumulate ? d[i] + out.alpha * acc[c][i] : out.alpha * acc[c][i];
+            if (i < left) {
+              const float v = out.alpha * (kUnscale * acc[c][i]);
+              d[i] = out.accumulate ? d[i] + v : v;
+            }
         }
       }
     }
@@ -596,7 +625,10 @@ int planes_product(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_
   const int64_t br = a->b_mn_major ? a->K : a->N, bc = a->b_mn_major ? a->N : a->K;
   SplitMat ma = split_mat(a->A, ar, ac, a->lda, a_planes), mb = split_mat(a->Bm, br, bc, a->ldb, b_planes);
   if (norms) ma.blocks = row_blocks(ar), mb.blocks = row_blocks(br);
-  const SgemmFlags flags{ma.flags, ma.blocks, mb.flags, mb.blocks};
+  int log_k = 0;
+  while ((1ll << log_k) < a->K) ++log_k;
+  // exponent fields are 127 above the exponents of values times 2^24; a magnitude is below 2^(its exponent + 1)
+  const SgemmFlags flags{ma.flags, ma.blocks, mb.flags, mb.blocks, 2 * 127 + 126 - 2 - log_k, 2 * 127 - 100};
   if (!a_ready || !b_ready) {
     const SplitMat& first = a_ready ? mb : ma;
     const int two = !a_ready && !b_ready;

@@ -206,5 +206,5 @@ extern "C" int pom_gemm_f32(const pom_gemm_args* a, void* stream) {
   const long long Mtot = a->M * a->batches;
   if (Mtot > INT32_MAX || a->N > INT32_MAX || a->K > INT32_MAX) return POM_ERR_TOO_LARGE;
   if (ceil_div(Mtot, 64) > 65535) return POM_ERR_TOO_LARGE;
-  return launch_sgemm(a, SgemmFlags{nullptr, 0, nullptr, 0}, static_cast<cudaStream_t>(stream));
+  return launch_sgemm(a, SgemmFlags{nullptr, 0, nullptr, 0, 0, 0}, static_cast<cudaStream_t>(stream));
 }

@@ -5,20 +5,48 @@
 
 namespace pomk {
 
-// Marks that the split of two operands into planes left behind (pom_gemm_f32.cu); no words: an unconditional product.
+// What the split of two operands into planes found out about them (pom_gemm_f32.cu); no words: an unconditional product.
+// A word holds, for a part of an operand, the float exponent field of the largest magnitude (254 and up: bf16 cannot
+// hold it) above bit 16 and that of the smallest one that is not zero (255: all zeros) below, both of value * 2^24.
 struct SgemmFlags {
   const int* a;
   int na;
   const int* b;
   int nb;
-  __device__ __forceinline__ bool scan(int first, int step) const {
-    int f = 0;
-    for (int i = first; i < na; i += step) f |= __ldcg(a + i);
-    for (int i = first; i < nb; i += step) f |= __ldcg(b + i);
-    return f != 0;
+  int max_sum;  // largest sum of the two operands' largest exponent fields, smallest sum of their smallest ones,
+  int min_sum;  // with which the plane products neither overflow nor lose bits
+  struct Range {
+    int hi, lo;
+  };
+  // Of the words first, first + step, ... and the other lanes' (whole warp).
+  __device__ __forceinline__ static Range scan(const int* w, int n, int first, int step) {
+    int hi = 0, lo = 255;
+#pragma unroll 8
+    for (int i = first; i < n; i += step) {
+      const int v = __ldcg(w + i);
+      hi = max(hi, v >> 16), lo = min(lo, v & 255);
+    }
+    return Range{__reduce_max_sync(0xffffffffu, hi), __reduce_min_sync(0xffffffffu, lo)};
   }
-  __device__ __forceinline__ bool any_in_warp(int lane) const { return __any_sync(0xffffffffu, scan(lane, 32)); }
-  __device__ __forceinline__ bool any_in_block() const { return __syncthreads_or(scan(threadIdx.x, blockDim.x)); }
+  __device__ __forceinline__ bool out_of_range(const Range& x, const Range& y) const {
+    return x.hi >= 254 || y.hi >= 254 || x.hi + y.hi > max_sum || x.lo + y.lo < min_sum;
+  }
+  // Whether the planes cannot carry the product.
+  __device__ __forceinline__ bool any_in_warp(int lane) const {
+    return out_of_range(scan(a, na, lane, 32), scan(b, nb, lane, 32));
+  }
+  __device__ __forceinline__ bool any_in_block() const {
+    __shared__ int sh[4];
+    if (threadIdx.x < 4) sh[threadIdx.x] = threadIdx.x < 2 ? 0 : 255;
+    __syncthreads();
+    const Range x = scan(a, na, threadIdx.x, blockDim.x), y = scan(b, nb, threadIdx.x, blockDim.x);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(sh, x.hi), atomicMax(sh + 1, y.hi);
+      atomicMin(sh + 2, x.lo), atomicMin(sh + 3, y.lo);
+    }
+    __syncthreads();
+    return out_of_range(Range{sh[0], sh[2]}, Range{sh[1], sh[3]});
+  }
 };
 
 }  // namespace pomk

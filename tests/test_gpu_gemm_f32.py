@@ -65,6 +65,30 @@ def test_sums_of_one_sign_and_far_scales_keep_float32_accuracy(scale):
     assert err <= 1e-6  # a chain of 6000 float32 FMAs is 5e-6 off on these inputs
 
 
+@pytest.mark.parametrize("a_scale,b_scale", [(1e-34, 1), (1e-38, 1), (1e-41, 1e3), (1, 1e-38), (1e-20, 1e-15), (1e-19, 1e-19),
+                                             (1e-22, 1e-22), (1e-30, 1e20), (1e12, 1e12), (1e25, 1e-25), (1e31, 1e-20)])
+def test_small_and_large_magnitudes_are_no_further_off_than_a_chain(a_scale, b_scale):
+    """Operands near either end of float32's range, subnormal ones among them, and products near it: the error, as a
+    share of the sum of magnitudes, is at most that of the FMA chain (or, where results are subnormal, one of their
+    steps)."""
+    g = torch.Generator().manual_seed(4)
+    a, b = (torch.randn(256, 512, generator=g).cuda() * s for s in (a_scale, b_scale))
+    a[:, ::7] *= 1e-3
+    want, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
+    err = [((_planes(a, b, use=u).double() - want).abs() - 2.0 ** -149).clamp(min=0).div(mag).max().item()
+           for u in (True, False)]
+    assert err[0] <= max(err[1], BOUND), err
+
+
+def test_values_outside_the_range_of_the_planes_move_the_product_to_the_fma_kernel():
+    a, b = _operands(300, 290, 260, False, False, 5)
+    b = b.sign() * (1 + b.abs())
+    for x, y, carried in ((1e-30, 1e-20, False), (1e24, 1e22, False), (1e-44, 1.0, True)):
+        p, q = a.clone(), b.clone()
+        p[17], q[5, 9] = x, y
+        assert torch.equal(_planes(p, q), _planes(p, q, use=False)) != carried, (x, y)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1), (63, 65, 17), (200, 1000, 40), (129, 257, 100), (2049, 2500, 33)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_fma_kernel_is_one_chain_over_k(shape):
