@@ -41,12 +41,10 @@ constexpr float kScale = 0x1p24f, kUnscale = 0x1p-48f;  // of an operand's plane
 constexpr int kMinSplitBlocks = 2;              // k-blocks that a K split keeps at least
 
 inline int64_t plane_ld(int64_t cols) { return (cols + 7) / 8 * 8; }
+// Blocks of either split kernel, and words in the buffer: a function of the operand alone, so that planes filled by one
+// call are read rightly by another.
 inline int split_blocks(int64_t rows, int64_t cols) {
   const int64_t n = ceil_div(rows * (plane_ld(cols) / 8), kSplitThreads);
-  return static_cast<int>(n < kFlagWords ? n : kFlagWords);
-}
-inline int row_blocks(int64_t rows) {  // a warp per row
-  const int64_t n = ceil_div(rows, kSplitThreads / 32);
   return static_cast<int>(n < kFlagWords ? n : kFlagWords);
 }
 inline __nv_bfloat16* planes_of(void* buf) {
@@ -624,7 +622,6 @@ int planes_product(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_
   const int64_t ar = a->a_mn_major ? a->K : a->M, ac = a->a_mn_major ? a->M : a->K;
   const int64_t br = a->b_mn_major ? a->K : a->N, bc = a->b_mn_major ? a->N : a->K;
   SplitMat ma = split_mat(a->A, ar, ac, a->lda, a_planes), mb = split_mat(a->Bm, br, bc, a->ldb, b_planes);
-  if (norms) ma.blocks = row_blocks(ar), mb.blocks = row_blocks(br);
   int log_k = 0;
   while ((1ll << log_k) < a->K) ++log_k;
   // exponent fields are 127 above the exponents of values times 2^24; a magnitude is below 2^(its exponent + 1)

@@ -132,6 +132,41 @@ def test_shared_planes_and_repeated_runs_give_the_same_bits():
     assert torch.equal(first, _planes(a, b)) and torch.equal(second, _planes(a, w, a_mn=True))
 
 
+@pytest.mark.parametrize("rows,cols", [(512, 1152), (1000, 72)], ids=["wide", "narrow"])
+@pytest.mark.parametrize("value", [None, float("inf")])
+def test_planes_of_a_projection_serve_a_later_product(rows, cols, value):
+    """pom_gemm_f32_planes with an operand that pom_project_f32 has split, through the C ABI: the words that say which
+    kernel computes the product are found whichever split wrote them."""
+    import ctypes as C
+
+    from pom_b200 import _abi, ops
+
+    x, w = _operands(rows, 96, cols, False, False, 11)
+    if value is not None:
+        x[rows - 1, 0] = value
+    dy = torch.randn(rows, 40, device="cuda")
+    L, status, st = _abi.lib(), _abi.ptr(_abi.status_word(x.device)), _abi.stream_ptr()
+    # what words that no call writes hold: "not finite", or "all zeros"
+    for junk in (255 << 16, 255):
+        bufs = []
+        for t in (x, w, dy):
+            bufs.append(torch.zeros(int(L.pom_f32_planes_bytes(*t.shape)), dtype=torch.uint8, device="cuda"))
+            bufs[-1][:4096].view(torch.int32).fill_(junk)
+        norms, out = torch.empty(rows + 96, device="cuda"), torch.empty(rows, 96, device="cuda")
+        g = _abi.GemmArgs()
+        g.A, g.Bm, g.C, g.M, g.N, g.K = x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, 96, cols
+        g.lda, g.ldb, g.ldc, g.batches, g.out_mode, g.split_k, g.alpha = cols, cols, 96, 1, _abi.OUT_F32, 1, 1.0
+        _abi.check(L.pom_project_f32(C.byref(g), bufs[0].data_ptr(), bufs[1].data_ptr(), norms.data_ptr(), 96, None,
+                                     status, st), "pom_project_f32")
+        got = torch.zeros(cols, 40, device="cuda")  # xT . dy, x read in the other major
+        g.A, g.Bm, g.C, g.M, g.N, g.K = x.data_ptr(), dy.data_ptr(), got.data_ptr(), cols, 40, rows
+        g.lda, g.ldb, g.ldc, g.a_mn_major, g.b_mn_major = cols, 40, 40, 1, 1
+        _abi.check(L.pom_gemm_f32_planes(C.byref(g), bufs[0].data_ptr(), 1, bufs[2].data_ptr(), 0, None, status, st),
+                   "pom_gemm_f32_planes")
+        fresh = _planes(x, dy, a_mn=True, b_mn=True)
+        assert torch.equal(got.nan_to_num(nan=7.0), fresh.nan_to_num(nan=7.0)), junk
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 128), (130, 258, 129), (500, 1000, 256), (1021, 2304, 1152)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_projection_takes_the_chain_beside_the_kinks(shape, monkeypatch):
