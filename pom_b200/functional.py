@@ -544,16 +544,16 @@ class _PoMLayer(torch.autograd.Function):
         d_bias = flat[n_qc + n_ag:n_qc + n_ag + S]
         d_coeff = flat[n_qc + n_ag + S:n_flat].view(P, K)
         # dWo[d, p] = sum_t dY[t, d] * SH[t, p]   (collapsed multi-head path: formed from dMb further down)
-        dy_pl = ops.F32Planes()  # float32: the planes of dY and G serve two products each
+        dy_pl = ops.F32Planes()  # float32: the planes of dY and G serve two products each, and go behind the second
         if not ctx.collapsed:
             ops.gemm(dy2, sh.view(B * T, P), a_mn=True, b_mn=True, out=d_wag, accumulate=True, a_planes=dy_pl)
 
         if spec.self_mixing:
-            G = torch.empty((B * T, P + S), dtype=dt, device=dev)
+            G = ops.empty_or_drop((B * T, P + S), dt, dev, (dy_pl,))
             g_hp, g_z = G[:, :P], G[:, P:]
         else:
-            g_hp = torch.empty((B * N, P), dtype=dt, device=dev)
-            g_z = torch.empty((B * T, S), dtype=dt, device=dev)
+            g_hp = ops.empty_or_drop((B * N, P), dt, dev, (dy_pl,))
+            g_z = ops.empty_or_drop((B * T, S), dt, dev, (dy_pl,))
 
         # ---------------------------------------------------------------- query phase backward
         dH_reduced = False  # True once dH already holds the sum over all ranks
@@ -585,6 +585,7 @@ class _PoMLayer(torch.autograd.Function):
                            dbias_out=d_bias)
         else:
             dsh = ops.gemm(dy2, w_ag, b_mn=True, a_planes=dy_pl).view(B, T, P)
+            dy_pl.drop()
             if heads:
                 ds32 = ops.zeros_f32(B * T * heads, dev).view(B, T, heads)
                 dH = ops.select_heads_bwd(dsh, s32, Hc if (causal or full) else H, ds32)
@@ -665,8 +666,10 @@ class _PoMLayer(torch.autograd.Function):
             dxq = ops.gemm(G, w_qc, b_mn=True, a_planes=g_pl).view(B, T, D)
             dxc = None
         else:
-            dxc = ops.gemm(g_hp, w_qc[:P], b_mn=True, a_planes=g_pl).view(B, N, D)
-            dxq = ops.gemm(g_z, w_qc[P:], b_mn=True, a_planes=z_pl).view(B, T, D)
+            dxc = ops.gemm(g_hp, w_qc[:P], b_mn=True, a_planes=g_pl, spare=(z_pl,)).view(B, N, D)
+            dxq = ops.gemm(g_z, w_qc[P:], b_mn=True, a_planes=z_pl, spare=(g_pl,)).view(B, T, D)
+        g_pl.drop()
+        z_pl.drop()
         if overlap:
             main.wait_stream(side)
             f16.record_stream(main)

@@ -171,6 +171,23 @@ class F32Planes:
             self.buf = torch.empty((nbytes,), dtype=torch.uint8, device=t.device)
         return self.buf
 
+    def drop(self) -> None:
+        self.buf, self.ready = None, 0
+
+
+def empty_or_drop(shape, dtype, device, planes=()) -> torch.Tensor:
+    """``torch.empty``; where it does not fit, once more without the planes that are only kept for a later product (which
+    makes them again, or runs on the FMA kernel)."""
+    try:
+        return torch.empty(shape, dtype=dtype, device=device)
+    except torch.OutOfMemoryError:
+        held = [p for p in planes if p is not None and p.buf is not None]
+        if not held:
+            raise
+        for p in held:
+            p.drop()
+        return torch.empty(shape, dtype=dtype, device=device)
+
 
 def f32_planes_pay(K: int) -> bool:
     """Whether a float32 product runs on the tensor cores (``pom_gemm_f32_planes``) or on the FMA kernel.  At K = 64 and
@@ -184,14 +201,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
          out: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
          accumulate: bool = False, split_k: int = 0, alpha: float = 1.0, act: Optional[str] = None,
          residual: Optional[torch.Tensor] = None, a_planes: Optional[F32Planes] = None,
-         b_planes: Optional[F32Planes] = None, fma: bool = False) -> torch.Tensor:
+         b_planes: Optional[F32Planes] = None, fma: bool = False, spare: Tuple[F32Planes, ...] = ()) -> torch.Tensor:
     """C[m, n] = alpha * sum_k A[m, k] * B[n, k].
 
     ``a`` is (M, K) — or (K, M) when ``a_mn`` — and ``b`` is (N, K) — or (K, N) when ``b_mn``;
     both row-major with a contiguous last dimension.  bf16 inputs run on the tcgen05 kernel,
     fp32 inputs on its three-plane form (``a_planes`` / ``b_planes``: see :class:`F32Planes`) or, with ``fma`` or a short
-    K, on the FMA kernel, which sums every output as one chain over k.  ``accumulate`` adds into a fp32 ``out``.  For bf16 outputs the epilogue can
-    apply ``act="gelu"`` and add a bf16 ``residual`` of the output's shape.
+    K, on the FMA kernel, which sums every output as one chain over k.  Where memory is short, ``a_planes``, ``b_planes`` and ``spare`` (planes
+    kept for other products) give way to the output, and the planes to the FMA kernel.  ``accumulate`` adds into a fp32
+    ``out``.  For bf16 outputs the epilogue can apply ``act="gelu"`` and add a bf16 ``residual`` of the output's shape.
     """
     dev = _require_cuda(a, b, out)
     if a.dtype != b.dtype:
@@ -205,7 +223,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if accumulate:
             raise ValueError("accumulate needs an output tensor")
         odt = out_dtype or (torch.bfloat16 if is_bf16 else torch.float32)
-        out = torch.empty((M, N), dtype=odt, device=dev)
+        out = empty_or_drop((M, N), odt, dev, (a_planes, b_planes, *spare))
     if out.shape != (M, N):
         raise ValueError("output shape mismatch")
     if accumulate and out.dtype != torch.float32:
@@ -242,6 +260,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
                 bufs = pa.take(a), pb.take(b), torch.empty((nbytes,), dtype=torch.uint8, device=dev) if nbytes else None
             except torch.OutOfMemoryError:  # a product whose operands fill the GPU: the FMA kernel needs no planes
                 planes = False
+                pa.drop()
+                pb.drop()
         if planes:
             _abi.check(L.pom_gemm_f32_planes(C.byref(g), ptr(bufs[0]), pa.ready, ptr(bufs[1]), pb.ready, ptr(bufs[2]),
                                              ptr(_abi.status_word(dev)), _abi.stream_ptr()), "pom_gemm_f32_planes")

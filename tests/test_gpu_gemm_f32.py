@@ -249,3 +249,69 @@ def test_projection_beside_a_kink_where_squares_underflow(scale, monkeypatch):
     eps = 2.0 ** -24 * 300 ** 0.5 * (x.norm(dim=1)[:, None].double() * scale * w.norm(dim=1)[None].double())
     near = chain.abs().double() <= 4 * eps
     assert bool(near.any()) and torch.equal(got[near], chain[near])
+
+
+class _Budget:
+    """Stands in for a GPU that has ``cap`` bytes: torch.empty raises beyond it, as the caching allocator would."""
+
+    def __init__(self, monkeypatch, cap):
+        self.refused = 0
+        empty = torch.empty
+
+        def limited(*size, dtype=torch.float32, device=None, **kw):
+            t = empty(*size, dtype=dtype, device=device, **kw)
+            if t.is_cuda and torch.cuda.memory_allocated() > cap:
+                self.refused += 1
+                del t
+                raise torch.OutOfMemoryError("no room")
+            return t
+
+        monkeypatch.setattr(torch, "empty", limited)
+
+
+@pytest.mark.parametrize("cross", [False, True], ids=["self", "cross"])
+def test_a_step_that_fits_without_planes_fits_with_them(cross, monkeypatch):
+    """Planes are there when memory is: a training step runs in the memory that the FMA kernel alone needs, and the
+    result is the same but for the order of additions."""
+    from unittest import mock
+
+    from pom_b200 import PoM, ops
+
+    torch.manual_seed(2)
+    mod = PoM(384, 2, 2).cuda()
+    x, xc, dy = (torch.randn(4, 500, 384, device="cuda") for _ in range(3))
+    ins = [x.requires_grad_()] + ([xc.requires_grad_()] if cross else [])
+    wrt = ins + [mod.qc_proj.weight, mod.se_bias, mod.po_coeff, mod.ag_proj.weight]
+
+    def step():
+        return torch.autograd.grad(mod(*ins), wrt, dy)
+
+    with mock.patch.object(ops, "f32_planes_pay", lambda *_: False):
+        step()  # caches of the layer
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        want = step()
+        needs = torch.cuda.max_memory_allocated() - base
+    with monkeypatch.context() as m:
+        budget = _Budget(m, torch.cuda.memory_allocated() + needs)
+        got = step()
+    assert budget.refused > 0
+    for a, b in zip(got, want):
+        assert ((a - b).norm() / b.norm()).item() <= 1e-5  # float32 sums in another order
+
+
+def test_planes_give_way_to_an_output_that_does_not_fit(monkeypatch):
+    from pom_b200 import ops
+
+    a, b = _operands(512, 300, 256, False, False, 12)
+    pl, spare = ops.F32Planes(), ops.F32Planes()
+    want = _planes(a, b, a_planes=pl)
+    spare.take(a)
+    with monkeypatch.context() as m:
+        _Budget(m, torch.cuda.memory_allocated() + 4096)  # the output takes more, and less than the planes
+        got = ops.gemm(a, b, a_planes=pl, spare=(spare,))
+    assert pl.buf is None and spare.buf is None
+    assert ((got - want).norm() / want.norm()).item() <= 1e-6
+    with pytest.raises(torch.OutOfMemoryError), monkeypatch.context() as m:
+        _Budget(m, torch.cuda.memory_allocated())
+        ops.gemm(a, b)
