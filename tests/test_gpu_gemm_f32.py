@@ -110,16 +110,22 @@ def test_fma_kernel_is_one_chain_over_k(shape):
             assert torch.equal(_planes(a, b, use=False, a_mn=a_mn, b_mn=b_mn), want), (a_mn, b_mn, pad)
 
 
-def test_infinities_nan_and_huge_values_take_the_fma_kernel():
-    a, b = _operands(300, 290, 260, False, False, 5)
+@pytest.mark.parametrize("shape", [(300, 290, 260), (255, 513, 4100)], ids=["one pass", "split sums"])
+def test_infinities_nan_and_huge_values_take_the_fma_kernel(shape):
+    from pom_b200 import _abi
+
+    M, N, K = shape
+    assert bool(_abi.lib().pom_gemm_f32_planes_scratch(M, N, K, _abi.OUT_F32_ACCUM)) == (K > 4000)  # K is split
+    a, b = _operands(M, N, K, False, False, 5)
     for value in (float("inf"), float("-inf"), float("nan"), 1e30, -2e38):
         x = a.clone()
         x[17, 31] = value
         got = _planes(x, b)
         want = _planes(x, b, use=False)
         assert torch.equal(torch.nan_to_num(got, nan=7.0), torch.nan_to_num(want, nan=7.0))
-        acc = _planes(x, b, out=torch.ones_like(want), accumulate=True)
-        assert torch.equal(torch.isnan(acc), torch.isnan(want))
+        before = torch.randn(M, N, device="cuda")
+        acc = _planes(x, b, out=before.clone(), accumulate=True)
+        assert torch.equal(torch.nan_to_num(acc, nan=7.0), torch.nan_to_num(before + want, nan=7.0))
 
 
 def test_shared_planes_and_repeated_runs_give_the_same_bits():
