@@ -9,8 +9,8 @@
 // access is a coalesced 16-byte vector, several are in flight per thread, and every sum is formed in a fixed order
 // (deterministic, no float atomics).
 // Lanes: one keeps a thread's set-up (its coefficients above all) to one per 64 tokens; where that would leave the SMs
-// with a few warps each, more lanes shorten the walk.  Forward sums and causal walks keep one lane at every size: a
-// sample's result has the same bits whatever batch it came in.
+// with a few warps each, more lanes shorten the walk.  A sample's results have the same bits whatever batch it came in:
+// forward sums and causal walks keep one lane at every size, backward sums over a sample's tokens four.
 #include "common.cuh"
 #include "gemm_launch.cuh"
 #include "pom_math.cuh"
@@ -214,7 +214,7 @@ __device__ __forceinline__ float poly_grad_reg(float a, const float (&c)[KR]) {
 
 constexpr int kWalkThreads = 256;  // most threads of a block
 
-extern __shared__ float walk_sm[];  // blocks of more than one lane: see walk_smem
+extern __shared__ float walk_sm[];  // blocks of more than one lane (WalkLaunch::smem)
 
 // The tokens [n0, n1) of this thread in the c-th run of `span` tokens of a sequence of n tokens.
 __device__ __forceinline__ void lane_tokens(int c, int span, int n, bool on, int& n0, int& n1) {
@@ -1643,19 +1643,20 @@ struct WalkLaunch {
 // 32 threads across the channels (512 bytes of a row at 16 bytes each).  Where one 64-token walk per warp leaves the SMs
 // with fewer than kWalkWarps warps each, the walk is cut: into token lanes of a block if sums are formed over a chunk
 // (kLanes), into blocks of fewer tokens if not (kSpans; blocks of one warp run up to half as fast again as blocks of
-// two to four).  Channels that fill less than 32 threads take fewer threads and more lanes, up to one token per lane.
+// two to four).  Sums of one sample take four lanes whatever the batch (kFour): with one to eight by the batch their bits
+// would follow it.  Channels that fill less than 32 threads take fewer threads and more lanes, up to one token per lane.
 // Selection at 4 x 1536 x 2048, forward / backward: 33 / 80 us before, 12 / 27 us with 2 to 4 lanes; at
 // 32 x 1024 x 2304 157 / 263 and 74 / 126 us.
-enum WalkCut { kWhole, kLanes, kSpans };
+enum WalkCut { kWhole, kLanes, kFour, kSpans };
 constexpr int kWalkWarps = 24;
 WalkLaunch walk_launch(int P, int rope_kind, int vec, int N, int B, WalkCut cut) {
   const int units = static_cast<int>(ceil_div(first_channels(P, rope_kind), vec));
   const long long warps = ceil_div(units, 32) * ceil_div(N, kChunk) * B;
-  int nx = 32, parts = 1;
-  if (cut != kWhole)
+  int nx = 32, parts = cut == kFour ? 4 : 1;
+  if (cut == kLanes || cut == kSpans)
     while (parts < 8 && warps * parts < 1ll * kWalkWarps * sm_count()) parts *= 2;
   WalkLaunch w;
-  int ny = cut == kLanes ? parts : 1;
+  int ny = cut == kLanes || cut == kFour ? parts : 1;
   w.span = cut == kSpans ? kChunk / parts : kChunk;
   if (cut != kWhole && units < 32) {
     while (nx > 4 && nx / 2 >= units) nx /= 2;
@@ -2031,7 +2032,7 @@ static int select_common(SelDev& d, int dtype, bool bwd, std::initializer_list<l
   int rc = check_rope(d.rope, d.P);
   if (rc) return rc;
   const int vec = pick_vec(d.P, d.rope, dtype, 1, lds, ptrs);
-  const WalkLaunch wl = walk_launch(d.P, d.rope.kind, vec, d.T, d.B, bwd ? kLanes : kSpans);
+  const WalkLaunch wl = walk_launch(d.P, d.rope.kind, vec, d.T, d.B, bwd ? kFour : kSpans);
   d.span = wl.span;
   const bool has_rope = d.rope.kind != POM_ROPE_NONE;
   if (bwd) {
@@ -2136,7 +2137,7 @@ static int select_heads_common(const pom_select_heads_args* a, bool bwd, void* s
   int vec = pick_vec(d.head_dim, none, a->dtype, 1,
                      {a->h_per_token ? a->ld_h : 0, bwd ? a->ld_dsh : a->ld_sh, (bwd && a->h_per_token) ? a->ld_dh : 0},
                      {a->h_per_token ? a->H : nullptr, bwd ? a->dsh : a->sh, (bwd && a->h_per_token) ? a->dh_tok : nullptr});
-  const WalkLaunch wl = walk_launch(a->P, POM_ROPE_NONE, vec, a->T, a->B, kLanes);
+  const WalkLaunch wl = walk_launch(a->P, POM_ROPE_NONE, vec, a->T, a->B, kFour);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (bwd) {
 #define CALL_HB(T, V, KR) select_heads_kernel<T, V, true><<<wl.grid, wl.block, wl.smem, st>>>(d)

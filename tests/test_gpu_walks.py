@@ -42,6 +42,55 @@ def test_selection_and_per_token_features_at_every_cut(shape, dtype):
     assert close(dx, wx) and ((dc.double() - wc).norm() / wc.norm()).item() <= max(tol, 1e-4)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,P", [(1, 8), (63, 16), (65, 40), (300, 256), (1000, 1152), (77, 2304)])
+def test_a_samples_gradients_have_the_same_bits_in_every_batch(N, P, dtype):
+    """Launch shapes follow the batch; the order of a sample's sums, and every result, does not."""
+    from pom_b200 import ops
+
+    g = torch.Generator().manual_seed(N + P)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(dtype).cuda()
+    z, dsh = rnd(64, N, P), rnd(64, N, P)
+    bias, h = torch.randn(P, generator=g).cuda(), torch.randn(64, P, generator=g).cuda()
+    s32, coeff = torch.rand(64, N, P // 8, generator=g).cuda(), torch.randn(P, 4, generator=g).cuda()
+    rope = None
+    if P % 16 == 0:
+        ang = torch.rand(N, P // 2, generator=g).cuda()
+        rope = ops.RopeSpec(1, ang.cos(), ang.sin(), torch.arange(N, device="cuda"))
+    want = None
+    for B in (64, 16, 4, 1):
+        got = []
+        for r in (None, rope):
+            dz = torch.empty_like(z[:B])
+            got += [ops.select_bwd(dsh[:B], z[:B], bias, h[:B], dz, rope=r)[0][0], dz[0]]
+            got.append(ops.select_fwd(z[:B], bias, h[:B], rope=r)[0])
+            for c in (coeff[:, :2].contiguous(), coeff):
+                got += [ops.poly_agg_fwd(z[:B], c, rope=r)[0], ops.poly_agg_fwd(z[:B], c, per_token=True, rope=r)[0],
+                        ops.poly_agg_fwd(z[:B], c, causal=True, rope=r)[0][0]]
+                for kw in (dict(dH=h[:B]), dict(dout=dsh[:B], causal=True), dict(dout=dsh[:B], per_token=True)):
+                    dx = torch.empty_like(z[:B])
+                    ops.poly_agg_bwd(z[:B], c, dx_out=dx, rope=r, **kw)
+                    got.append(dx[0])
+        got.append(ops.select_heads_bwd(dsh[:B], s32[:B], h[:B], torch.zeros_like(s32[:B]))[0])
+        want = want or got
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), B
+
+
+@pytest.mark.parametrize("B", [1, 3, 16, 64])
+def test_a_samples_input_gradient_has_the_same_bits_in_every_batch(B):
+    from pom_b200 import PoM
+
+    torch.manual_seed(0)
+    mod = PoM(256, 2, 2).cuda()
+    x, dy = torch.randn(64, 300, 256, device="cuda"), torch.randn(64, 300, 256, device="cuda")
+
+    def dx(n):
+        q = x[:n].clone().requires_grad_()
+        return torch.autograd.grad(mod(q), q, dy[:n])[0][0]
+
+    assert torch.equal(dx(B), dx(64))
+
+
 @pytest.mark.parametrize("n", [1, 31, 1000, 4096, 4097, 70001])
 @pytest.mark.parametrize("rows", [1, 7, 40])
 def test_row_sums_of_one_column(rows, n):
