@@ -359,14 +359,19 @@ def reduce_partials(partial: torch.Tensor, *, denom: Optional[torch.Tensor] = No
     assert partial.dtype == torch.float32 and partial.is_contiguous()
     if out is None:
         out = torch.empty((B, P), dtype=torch.float32, device=partial.device)
-    # Few samples and very many chunks (one long sequence): the kernel's grid is (P/32, B), so first fold groups of
-    # chunks into (B*G, P) with G times as many CTAs, then finish over the G group sums.
-    if P > 1 and chunks >= 1024 and B * ((P + 31) // 32) < 256:
+    # Very many chunks (a long sequence): the kernel's grid is (P/32, B), so first fold groups of chunks into (B*G, P) with
+    # G times as many CTAs, then finish over the G group sums.  B does not enter (a sample's sum has the same bits whatever
+    # batch it came in); the samples of one launch are limited by its grid.
+    if P > 1 and chunks >= 1024 and (P + 31) // 32 < 256:
         G = next((g for g in (32, 16, 8, 4) if chunks % g == 0), 0)
         if G:
-            part = torch.empty((B * G, P), dtype=torch.float32, device=partial.device)
-            _abi.check(_abi.lib().pom_reduce_partials(ptr(partial), ptr(part), None, 1.0, B * G, chunks // G, P,
-                                                      _abi.stream_ptr()), "pom_reduce_partials")
+            part = torch.empty((B, G, P), dtype=torch.float32, device=partial.device)
+            per = 65535 // G
+            for lo in range(0, B, per):
+                n = min(per, B - lo)
+                _abi.check(_abi.lib().pom_reduce_partials(ptr(partial[lo:lo + n]), ptr(part[lo:lo + n]), None, 1.0,
+                                                          n * G, chunks // G, P, _abi.stream_ptr()),
+                           "pom_reduce_partials")
             partial, chunks = part, G
     _abi.check(_abi.lib().pom_reduce_partials(ptr(partial), ptr(out), ptr(denom), scale, B, chunks, P,
                                               _abi.stream_ptr()), "pom_reduce_partials")

@@ -76,6 +76,18 @@ def test_a_samples_gradients_have_the_same_bits_in_every_batch(N, P, dtype):
         assert all(torch.equal(a, b) for a, b in zip(got, want)), B
 
 
+@pytest.mark.parametrize("chunks", [64, 1023, 1024, 4100])
+def test_a_samples_partial_sums_have_the_same_bits_in_every_batch(chunks):
+    from pom_b200 import ops
+
+    x = torch.randn(40, chunks, 264, device="cuda")
+    want = ops.reduce_partials(x)
+    for B in (1, 7, 33):
+        assert torch.equal(ops.reduce_partials(x[:B]), want[:B])
+    many = torch.ones(2100, 1024, 8, device="cuda")  # more groups than a launch's grid takes
+    assert bool((ops.reduce_partials(many) == 1024).all())
+
+
 @pytest.mark.parametrize("B", [1, 3, 16, 64])
 def test_a_samples_input_gradient_has_the_same_bits_in_every_batch(B):
     from pom_b200 import PoM
