@@ -1254,7 +1254,9 @@ struct SelDev {
   pom_rope rope;
 };
 
-template <typename T, int VEC, bool BWD, bool ROPE>
+// HT: one aggregate per token (a.H is of T), else one per sample (fp32).  As a choice at run time it held registers for both:
+// 80 instead of 57 in the float32 backward, two waves instead of one at 64 x 577 x 768 (86 us, now 65).
+template <typename T, int VEC, bool BWD, bool ROPE, bool HT>
 __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_kernel(const SelDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
@@ -1269,7 +1271,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
     b1[e] = a.activated || !on ? 0.f : a.bias[m.p1 + e];
     b2[e] = (rope && !a.activated && on) ? a.bias[m.p2 + e] : 0.f;
     hb1[e] = hb2[e] = 0.f;
-    if (!a.h_per_token && on) {
+    if (!HT && on) {
       const float* H = static_cast<const float*>(a.H) + static_cast<long long>(b) * a.P;
       hb1[e] = H[m.p1 + e];
       if (rope) hb2[e] = H[m.p2 + e];
@@ -1294,7 +1296,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
         rz2[q].ld(z + t * a.ld_z + m.p2);
         rope_coeffs<VEC>(a.rope, m, t, cs[q], sn[q]);
       }
-      if (a.h_per_token) {
+      if (HT) {
         const T* __restrict__ H = static_cast<const T*>(a.H) + (rowb + t) * a.ld_h;
         rh1[q].ld(H + m.p1);
         if (rope) rh2[q].ld(H + m.p2);
@@ -1316,7 +1318,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
       float z1[VEC], z2[VEC], h1[VEC], h2[VEC], g1[VEC], g2[VEC];
       rz1[q].get(z1);
       if (rope) rz2[q].get(z2);
-      if (a.h_per_token) {
+      if (HT) {
         rh1[q].get(h1);
         if (rope) rh2[q].get(h2);
 #pragma unroll
@@ -1379,7 +1381,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
         }
         Vec<T, VEC>::st(dz + m.p1, o1);
         if (rope) Vec<T, VEC>::st(dz + m.p2, o2);
-        if (a.h_per_token) {
+        if (HT) {
           T* __restrict__ dh = static_cast<T*>(a.dh_tok) + (rowb + t) * a.ld_dh;
 #pragma unroll
           for (int e = 0; e < VEC; ++e) dh1[e] *= rs[q], dh2[e] *= rs[q];  // gradient of the un-normalised H
@@ -1393,7 +1395,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
     const long long o = (static_cast<long long>(b) * a.chunks + c) * a.P;
     sum_lanes<VEC>(accB1, on, [&](int e, float v) { a.dbias_partial[o + m.p1 + e] = v; });
     if (rope) sum_lanes<VEC>(accB2, on, [&](int e, float v) { a.dbias_partial[o + m.p2 + e] = v; });
-    if (!a.h_per_token) {
+    if (!HT) {
       sum_lanes<VEC>(accH1, on, [&](int e, float v) { a.dh_partial[o + m.p1 + e] = v; });
       if (rope) sum_lanes<VEC>(accH2, on, [&](int e, float v) { a.dh_partial[o + m.p2 + e] = v; });
     }
@@ -2036,15 +2038,19 @@ static int select_common(SelDev& d, int dtype, bool bwd, std::initializer_list<l
   d.span = wl.span;
   const bool has_rope = d.rope.kind != POM_ROPE_NONE;
   if (bwd) {
-#define CALL_SB(T, V, KR)                                                          \
-  if (has_rope) select_kernel<T, V, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);   \
-  else select_kernel<T, V, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_SB(T, V, KR)                                                                                   \
+  if (has_rope && d.h_per_token) select_kernel<T, V, true, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);    \
+  else if (has_rope) select_kernel<T, V, true, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);               \
+  else if (d.h_per_token) select_kernel<T, V, true, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else select_kernel<T, V, true, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SB);
 #undef CALL_SB
   } else {
-#define CALL_SF(T, V, KR)                                                          \
-  if (has_rope) select_kernel<T, V, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);  \
-  else select_kernel<T, V, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_SF(T, V, KR)                                                                                   \
+  if (has_rope && d.h_per_token) select_kernel<T, V, false, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);    \
+  else if (has_rope) select_kernel<T, V, false, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);               \
+  else if (d.h_per_token) select_kernel<T, V, false, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else select_kernel<T, V, false, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SF);
 #undef CALL_SF
   }
