@@ -269,6 +269,9 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : KR <= 2 ? 4 : 3) agg_
   const int c = blockIdx.y, b = blockIdx.z;
   constexpr bool rope = ROPE;
   constexpr bool PREFIX = MODE != kAggSum, per_token = MODE == kAggToken;
+  // Per-token results: a test of the end between the tokens of a batch keeps their loads from running ahead (float32
+  // 64 x 577 x 768 55 us with it, 40 without).  Rotated bf16 has no registers for that (58 us without, 45 with it).
+  constexpr bool kAhead = per_token && !(ROPE && VEC == 8);
   const ColMap m = map_unit(u, a.P, a.rope.kind);
   if (!m.valid) return;
   Coefs<VEC, KR> cf;
@@ -300,7 +303,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : KR <= 2 ? 4 : 3) agg_
 #pragma unroll
     for (int q = 0; q < kTB; ++q) {
       const int n = nb + q;
-      if (n >= n1) break;
+      if (!kAhead && n >= n1) break;
       if (per_token) {
 #pragma unroll
         for (int e = 0; e < VEC; ++e) acc1[e] = acc2[e] = 0.f;
@@ -324,11 +327,11 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : KR <= 2 ? 4 : 3) agg_
         float o[VEC];
 #pragma unroll
         for (int e = 0; e < VEC; ++e) o[e] = acc1[e] * inv;
-        Vec<T, VEC>::st(out + n * a.ld_out + m.p1, o);
+        if (!kAhead || n < n1) Vec<T, VEC>::st(out + n * a.ld_out + m.p1, o);
         if (rope) {
 #pragma unroll
           for (int e = 0; e < VEC; ++e) o[e] = acc2[e] * inv;
-          Vec<T, VEC>::st(out + n * a.ld_out + m.p2, o);
+          if (!kAhead || n < n1) Vec<T, VEC>::st(out + n * a.ld_out + m.p2, o);
         }
       }
     }
@@ -1643,23 +1646,25 @@ struct WalkLaunch {
 };
 
 // 32 threads across the channels (512 bytes of a row at 16 bytes each).  Where one 64-token walk per warp leaves the SMs
-// with fewer than kWalkWarps warps each, the walk is cut: into token lanes of a block if sums are formed over a chunk
-// (kLanes), into blocks of fewer tokens if not (kSpans; blocks of one warp run up to half as fast again as blocks of
-// two to four).  Sums of one sample take four lanes whatever the batch (kFour): with one to eight by the batch their bits
-// would follow it.  Channels that fill less than 32 threads take fewer threads and more lanes, up to one token per lane.
-// Selection at 4 x 1536 x 2048, forward / backward: 33 / 80 us before, 12 / 27 us with 2 to 4 lanes; at
-// 32 x 1024 x 2304 157 / 263 and 74 / 126 us.
-enum WalkCut { kWhole, kLanes, kFour, kSpans };
-constexpr int kWalkWarps = 24;
+// with too few warps each, the walk is cut: into token lanes of a block if sums are formed over a chunk (kLanes), into
+// blocks of fewer tokens if not (kSpans, kTokens; blocks of one warp run up to half as fast again as blocks of two to four).
+// Sums of one sample take four lanes whatever the batch (kFour): with one to eight by the batch their bits would follow it.
+// Channels that fill less than 32 threads take fewer threads and more lanes, up to one token per lane.
+// The lines, us at 12, 16 and 24 warps: selection of 16 x 512 x 1024 float32 16, 12, 12, of 8 x 1364 x 1672 38, 38, 35;
+// per-token features (which load coefficients in every block) of 8 x 1364 x 1672 bf16, degree 4, 26, 26, 33, of
+// 64 x 577 x 768 29, 23, 23.
+enum WalkCut { kWhole, kLanes, kFour, kSpans, kTokens };
 WalkLaunch walk_launch(int P, int rope_kind, int vec, int N, int B, WalkCut cut) {
   const int units = static_cast<int>(ceil_div(first_channels(P, rope_kind), vec));
   const long long warps = ceil_div(units, 32) * ceil_div(N, kChunk) * B;
+  const long long enough = (cut == kTokens ? 16ll : 24ll) * sm_count();
+  const bool spans = cut == kSpans || cut == kTokens;
   int nx = 32, parts = cut == kFour ? 4 : 1;
-  if (cut == kLanes || cut == kSpans)
-    while (parts < 8 && warps * parts < 1ll * kWalkWarps * sm_count()) parts *= 2;
+  if (cut == kLanes || spans)
+    while (parts < 8 && warps * parts < enough) parts *= 2;
   WalkLaunch w;
-  int ny = cut == kLanes || cut == kFour ? parts : 1;
-  w.span = cut == kSpans ? kChunk / parts : kChunk;
+  int ny = spans ? 1 : parts;
+  w.span = spans ? kChunk / parts : kChunk;
   if (cut != kWhole && units < 32) {
     while (nx > 4 && nx / 2 >= units) nx /= 2;
     ny = kWalkThreads / nx;
@@ -1768,7 +1773,7 @@ int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
   d.rope = a->rope;
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx, a->causal ? a->ld_out : 0},
                            {a->x, a->causal ? a->out : nullptr});
-  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 2 ? kSpans : kWhole);
+  const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 2 ? kTokens : kWhole);
   d.span = wl.span;
   const bool has_rope = a->rope.kind != POM_ROPE_NONE;
   if (a->causal != 2) {  // per-token features (causal == 2) need neither the sums nor the scan
