@@ -473,9 +473,8 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kWalkThreads) causal_bwd_sum_kernel(const AggBwdDev a) {
   const int p = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  const bool on = p < a.P;
-  int n0, n1;
-  lane_tokens(c, kChunk, a.N, on, n0, n1);
+  if (p >= a.P) return;
+  const int n0 = c * kChunk, n1 = min(a.N, n0 + kChunk);
   const T* __restrict__ g = static_cast<const T*>(a.dout) + static_cast<long long>(b) * a.N * a.ld_dout + p;
   float acc[VEC];
 #pragma unroll
@@ -493,14 +492,23 @@ __global__ void __launch_bounds__(kWalkThreads) causal_bwd_sum_kernel(const AggB
     }
   }
   float* part = a.partial + (static_cast<long long>(b) * a.chunks + c) * a.P + p;
-  sum_lanes<VEC>(acc, on, [&](int e, float v) { part[e] = v; });
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) part[e] = acc[e];
 }
 
 // CAUSAL == false: the gradient reaching every token is w[b,n] * dH[b, :].
 // CAUSAL == true : walk the chunk backwards; W[n] = suffix + sum_{m >= n} dout[m]/(m+1+offset).
 // Either way: un-rotate, then dx = g * poly'(a) * act'(x) and the coefficient gradient sums.
-template <typename T, int VEC, int KR, bool CAUSAL, bool ROPE>
-__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : 2) agg_bwd_kernel(const AggBwdDev a) {
+// Whole batches of tokens run without a test of the end between them, which would keep their loads from running ahead
+// (float32 mean of 32 x 1024 x 2304: 158 us with it, 114 without), where registers allow: not with rotation, not bf16 of
+// degree 3 and up.  DEEP: the causal walk, whose one lane wants more tokens in flight; bf16 of degree 3 and 4 takes it for
+// grids of a few warps per SM only (1 x 1529 x 1776, degree 4: 50 us without, 47 with it; 8 x 2047 x 2304: 87 and 101).
+template <typename T, int VEC, int KR, bool CAUSAL, bool ROPE, bool DEEP>
+__global__ void __launch_bounds__(kWalkThreads, ROPE || (DEEP && VEC == 8) ? 1 : 2) agg_bwd_kernel(const AggBwdDev a) {
+  constexpr bool kTight = VEC == 8 && KR > 2;
+  constexpr bool kFull = !ROPE && KR <= 4 && (!kTight || DEEP);
+  constexpr int TBW = KR > 4 || (ROPE && CAUSAL && VEC > 2) ? 2 : !ROPE && !kTight && (DEEP || (CAUSAL && VEC == 4)) ? 8 : kTB;
+
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
   constexpr bool rope = ROPE;
@@ -540,13 +548,13 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : 2) agg_bwd_kernel(con
     const float dn = a.denom[b];
     wb = dn != 0.f ? wb / dn : 0.f;
   }
-  constexpr int TBW = (ROPE && VEC > 2) || KR > 4 ? 2 : kTB;  // tokens in flight, as registers allow
-  for (int ib = 0; ib < cnt; ib += TBW) {
+  const auto batch = [&](int ib, auto full) {  // `full`: all TBW tokens exist
+    constexpr bool kAll = decltype(full)::value;
     Raw<T, VEC> r1[TBW], r2[TBW], go1[TBW], go2[TBW];
     float cs[TBW][VEC], sn[TBW][VEC], w[TBW];
 #pragma unroll
     for (int q = 0; q < TBW; ++q) {
-      const int i = min(ib + q, cnt - 1);
+      const int i = kAll ? ib + q : min(ib + q, cnt - 1);
       const int n = CAUSAL ? (n1 - 1 - i) : (n0 + i);
       r1[q].ld(x + n * a.ldx + m.p1);
       if (rope) {
@@ -564,7 +572,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : 2) agg_bwd_kernel(con
 #pragma unroll
     for (int q = 0; q < TBW; ++q) {
       const int i = ib + q;
-      if (i >= cnt) break;
+      if (!kAll && i >= cnt) break;
       const int n = CAUSAL ? (n1 - 1 - i) : (n0 + i);
       float x1[VEC], x2[VEC];
       if (CAUSAL) {
@@ -615,7 +623,11 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : 2) agg_bwd_kernel(con
       Vec<T, VEC>::st(dx + n * a.ld_dx + m.p1, o1);
       if (rope) Vec<T, VEC>::st(dx + n * a.ld_dx + m.p2, o2);
     }
-  }
+  };
+  int ib = 0;
+  if constexpr (kFull)
+    for (; ib + TBW <= cnt; ib += TBW) batch(ib, std::true_type{});
+  for (; ib < cnt; ib += TBW) batch(ib, std::false_type{});
   float* dcp = a.dcoeff_partial + (static_cast<long long>(b) * a.chunks + c) * a.P * a.K;
 #pragma unroll
   for (int k = 0; k < KR; ++k) {
@@ -2014,15 +2026,18 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
       count_launch();
       if (a->phase == 1) return check_launch();  // totals only
     }
-#define CALL_BC(T, V, KR)                                                                    \
-  if (has_rope) agg_bwd_kernel<T, V, KR, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
-  else agg_bwd_kernel<T, V, KR, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+    const bool deep = a->causal == 1 && (!(a->dtype == POM_BF16 && a->K > 2) ||
+                                         1ll * wl.grid.x * wl.grid.y * wl.grid.z < 6ll * sm_count());
+#define CALL_BC(T, V, KR)                                                                                     \
+  if (has_rope) agg_bwd_kernel<T, V, KR, true, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);           \
+  else if (deep) agg_bwd_kernel<T, V, KR, true, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else agg_bwd_kernel<T, V, KR, true, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BC);
 #undef CALL_BC
   } else {
-#define CALL_BN(T, V, KR)                                                                    \
-  if (has_rope) agg_bwd_kernel<T, V, KR, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);       \
-  else agg_bwd_kernel<T, V, KR, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_BN(T, V, KR)                                                                                     \
+  if (has_rope) agg_bwd_kernel<T, V, KR, false, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else agg_bwd_kernel<T, V, KR, false, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BN);
 #undef CALL_BN
   }
