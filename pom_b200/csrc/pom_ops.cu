@@ -213,6 +213,14 @@ __device__ __forceinline__ float poly_grad_reg(float a, const float (&c)[KR]) {
 }
 
 constexpr int kWalkThreads = 256;  // most threads of a block
+// Kernels with rotation (ROPE > 0) hold 120 to 250 registers, and an SM has room for 16 warps up to 128, for 12 up to 168
+// and for 8 beyond.  ROPE 1: as many as the compiler likes, for grids of up to 8 warps per SM.  ROPE 2: held to 168 (float32 of
+// degree 1 and 2: 128) for larger ones, which would run in one more wave (causal mean of 64 x 577 x 768: bf16 128 us with
+// ROPE 1, 98 with 2; float32 129 and 89; but bf16 of 1 x 1024 x 2304 45 and 51).  Degrees 3 and 4 only in the float32
+// backward pass (8 x 1364 x 1664, degree 4: 88 and 71; the others spill).
+constexpr int kRopeThreads = 128;
+template <int VEC, int KR>
+constexpr int rope_blocks(int rope) { return rope == 1 ? 1 : VEC <= 4 && KR <= 2 ? 4 : 3; }
 
 extern __shared__ float walk_sm[];  // blocks of more than one lane (WalkLaunch::smem)
 
@@ -263,15 +271,17 @@ struct AggDev {
 // PREFIX: partial holds the exclusive prefix per chunk; writes out[b, n, :].
 // TOKEN : writes each token's own (rotated) features.
 enum AggMode { kAggSum, kAggPrefix, kAggToken };
-template <typename T, int VEC, int KR, AggMode MODE, bool ROPE>
-__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : KR <= 2 ? 4 : 3) agg_fwd_kernel(const AggDev a) {
+template <typename T, int VEC, int KR, AggMode MODE, int ROPE>
+__global__ void __launch_bounds__(ROPE ? kRopeThreads : kWalkThreads, ROPE ? rope_blocks<VEC, KR>(ROPE) : KR <= 2 ? 4 : 3)
+agg_fwd_kernel(const AggDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  constexpr bool rope = ROPE;
+  constexpr bool rope = ROPE > 0;
   constexpr bool PREFIX = MODE != kAggSum, per_token = MODE == kAggToken;
   // Per-token results: a test of the end between the tokens of a batch keeps their loads from running ahead (float32
-  // 64 x 577 x 768 55 us with it, 40 without).  Rotated bf16 has no registers for that (58 us without, 45 with it).
-  constexpr bool kAhead = per_token && !(ROPE && VEC == 8);
+  // 64 x 577 x 768 55 us with it, 40 without).  With rotation there are registers for that only in float32 of degree 1 and 2
+  // (57 us with it, 50 without; bf16 45 and 58).
+  constexpr bool kAhead = per_token && (!ROPE || (VEC <= 4 && KR <= 2));
   const ColMap m = map_unit(u, a.P, a.rope.kind);
   if (!m.valid) return;
   Coefs<VEC, KR> cf;
@@ -503,15 +513,16 @@ __global__ void __launch_bounds__(kWalkThreads) causal_bwd_sum_kernel(const AggB
 // (float32 mean of 32 x 1024 x 2304: 158 us with it, 114 without), where registers allow: not with rotation, not bf16 of
 // degree 3 and up.  DEEP: the causal walk, whose one lane wants more tokens in flight; bf16 of degree 3 and 4 takes it for
 // grids of a few warps per SM only (1 x 1529 x 1776, degree 4: 50 us without, 47 with it; 8 x 2047 x 2304: 87 and 101).
-template <typename T, int VEC, int KR, bool CAUSAL, bool ROPE, bool DEEP>
-__global__ void __launch_bounds__(kWalkThreads, ROPE || (DEEP && VEC == 8) ? 1 : 2) agg_bwd_kernel(const AggBwdDev a) {
+template <typename T, int VEC, int KR, bool CAUSAL, int ROPE, bool DEEP>
+__global__ void __launch_bounds__(ROPE ? kRopeThreads : kWalkThreads, ROPE ? rope_blocks<VEC, KR>(ROPE) : DEEP && VEC == 8 ? 1 : 2)
+agg_bwd_kernel(const AggBwdDev a) {
   constexpr bool kTight = VEC == 8 && KR > 2;
   constexpr bool kFull = !ROPE && KR <= 4 && (!kTight || DEEP);
   constexpr int TBW = KR > 4 || (ROPE && CAUSAL && VEC > 2) ? 2 : !ROPE && !kTight && (DEEP || (CAUSAL && VEC == 4)) ? 8 : kTB;
 
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  constexpr bool rope = ROPE;
+  constexpr bool rope = ROPE > 0;
   const ColMap m = map_unit(u, a.P, a.rope.kind);
   const bool on = m.valid;
   Coefs<VEC, KR> cf;
@@ -1271,11 +1282,14 @@ struct SelDev {
 
 // HT: one aggregate per token (a.H is of T), else one per sample (fp32).  As a choice at run time it held registers for both:
 // 80 instead of 57 in the float32 backward, two waves instead of one at 64 x 577 x 768 (86 us, now 65).
-template <typename T, int VEC, bool BWD, bool ROPE, bool HT>
-__global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_kernel(const SelDev a) {
+// (Rotated float32 forward keeps the choice at run time: 53 us at 64 x 577 x 768, 59 without.)
+template <typename T, int VEC, bool BWD, int ROPE, bool HT>
+__global__ void __launch_bounds__(ROPE ? kRopeThreads : kWalkThreads, ROPE ? rope_blocks<VEC, 1>(ROPE) : BWD ? 2 : 4)
+select_kernel(const SelDev a) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int c = blockIdx.y, b = blockIdx.z;
-  constexpr bool rope = ROPE;
+  constexpr bool rope = ROPE > 0;
+  const bool ht = ROPE && !BWD && VEC == 4 ? a.h_per_token != 0 : HT;
   const ColMap m = map_unit(u, a.P, a.rope.kind);
   const bool on = m.valid;
   const long long rowb = static_cast<long long>(b) * a.T;
@@ -1286,7 +1300,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
     b1[e] = a.activated || !on ? 0.f : a.bias[m.p1 + e];
     b2[e] = (rope && !a.activated && on) ? a.bias[m.p2 + e] : 0.f;
     hb1[e] = hb2[e] = 0.f;
-    if (!HT && on) {
+    if (!ht && on) {
       const float* H = static_cast<const float*>(a.H) + static_cast<long long>(b) * a.P;
       hb1[e] = H[m.p1 + e];
       if (rope) hb2[e] = H[m.p2 + e];
@@ -1311,7 +1325,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
         rz2[q].ld(z + t * a.ld_z + m.p2);
         rope_coeffs<VEC>(a.rope, m, t, cs[q], sn[q]);
       }
-      if (HT) {
+      if (ht) {
         const T* __restrict__ H = static_cast<const T*>(a.H) + (rowb + t) * a.ld_h;
         rh1[q].ld(H + m.p1);
         if (rope) rh2[q].ld(H + m.p2);
@@ -1333,7 +1347,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
       float z1[VEC], z2[VEC], h1[VEC], h2[VEC], g1[VEC], g2[VEC];
       rz1[q].get(z1);
       if (rope) rz2[q].get(z2);
-      if (HT) {
+      if (ht) {
         rh1[q].get(h1);
         if (rope) rh2[q].get(h2);
 #pragma unroll
@@ -1396,7 +1410,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
         }
         Vec<T, VEC>::st(dz + m.p1, o1);
         if (rope) Vec<T, VEC>::st(dz + m.p2, o2);
-        if (HT) {
+        if (ht) {
           T* __restrict__ dh = static_cast<T*>(a.dh_tok) + (rowb + t) * a.ld_dh;
 #pragma unroll
           for (int e = 0; e < VEC; ++e) dh1[e] *= rs[q], dh2[e] *= rs[q];  // gradient of the un-normalised H
@@ -1410,7 +1424,7 @@ __global__ void __launch_bounds__(kWalkThreads, ROPE ? 1 : BWD ? 2 : 4) select_k
     const long long o = (static_cast<long long>(b) * a.chunks + c) * a.P;
     sum_lanes<VEC>(accB1, on, [&](int e, float v) { a.dbias_partial[o + m.p1 + e] = v; });
     if (rope) sum_lanes<VEC>(accB2, on, [&](int e, float v) { a.dbias_partial[o + m.p2 + e] = v; });
-    if (!HT) {
+    if (!ht) {
       sum_lanes<VEC>(accH1, on, [&](int e, float v) { a.dh_partial[o + m.p1 + e] = v; });
       if (rope) sum_lanes<VEC>(accH2, on, [&](int e, float v) { a.dh_partial[o + m.p2 + e] = v; });
     }
@@ -1655,6 +1669,9 @@ struct WalkLaunch {
   dim3 grid, block;
   size_t smem;
   int span;  // tokens per block
+  bool many() const {  // more warps than an SM holds of a kernel with ROPE 1
+    return 1ll * grid.x * grid.y * grid.z * ((block.x * block.y + 31) / 32) > 8ll * sm_count();
+  }
 };
 
 // 32 threads across the channels (512 bytes of a row at 16 bytes each).  Where one 64-token walk per warp leaves the SMs
@@ -1671,15 +1688,16 @@ WalkLaunch walk_launch(int P, int rope_kind, int vec, int N, int B, WalkCut cut)
   const long long warps = ceil_div(units, 32) * ceil_div(N, kChunk) * B;
   const long long enough = (cut == kTokens ? 16ll : 24ll) * sm_count();
   const bool spans = cut == kSpans || cut == kTokens;
+  const int threads = rope_kind == POM_ROPE_NONE ? kWalkThreads : kRopeThreads;
   int nx = 32, parts = cut == kFour ? 4 : 1;
   if (cut == kLanes || spans)
-    while (parts < 8 && warps * parts < enough) parts *= 2;
+    while (parts < (spans ? 8 : threads / 32) && warps * parts < enough) parts *= 2;
   WalkLaunch w;
   int ny = spans ? 1 : parts;
   w.span = spans ? kChunk / parts : kChunk;
   if (cut != kWhole && units < 32) {
     while (nx > 4 && nx / 2 >= units) nx /= 2;
-    ny = kWalkThreads / nx;
+    ny = threads / nx;
     w.span = kChunk;
   }
   w.block = dim3(static_cast<unsigned>(nx), static_cast<unsigned>(ny));
@@ -1787,11 +1805,12 @@ int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
                            {a->x, a->causal ? a->out : nullptr});
   const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 2 ? kTokens : kWhole);
   d.span = wl.span;
-  const bool has_rope = a->rope.kind != POM_ROPE_NONE;
+  const int rope = a->rope.kind == POM_ROPE_NONE ? 0 : wl.many() ? 2 : 1;
   if (a->causal != 2) {  // per-token features (causal == 2) need neither the sums nor the scan
-#define CALL_SUM(T, V, KR)                                                                    \
-  if (has_rope) agg_fwd_kernel<T, V, KR, kAggSum, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
-  else agg_fwd_kernel<T, V, KR, kAggSum, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_SUM(T, V, KR)                                                                                      \
+  if (rope == 2 && KR <= 2) agg_fwd_kernel<T, V, KR, kAggSum, KR <= 2 ? 2 : 1><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) agg_fwd_kernel<T, V, KR, kAggSum, 1><<<wl.grid, wl.block, wl.smem, st>>>(d);                    \
+  else agg_fwd_kernel<T, V, KR, kAggSum, 0><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_SUM);
 #undef CALL_SUM
     count_launch();
@@ -1802,15 +1821,17 @@ int pom_poly_agg_fwd(const pom_agg_args* a, void* stream) {
     count_launch();
   }
   if (a->causal == 2) {
-#define CALL_TOK(T, V, KR)                                                                            \
-  if (has_rope) agg_fwd_kernel<T, V, KR, kAggToken, true><<<wl.grid, wl.block, wl.smem, st>>>(d);      \
-  else agg_fwd_kernel<T, V, KR, kAggToken, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_TOK(T, V, KR)                                                                                      \
+  if (rope == 2 && KR <= 2) agg_fwd_kernel<T, V, KR, kAggToken, KR <= 2 ? 2 : 1><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) agg_fwd_kernel<T, V, KR, kAggToken, 1><<<wl.grid, wl.block, wl.smem, st>>>(d);                    \
+  else agg_fwd_kernel<T, V, KR, kAggToken, 0><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_TOK);
 #undef CALL_TOK
   } else {
-#define CALL_PFX(T, V, KR)                                                                            \
-  if (has_rope) agg_fwd_kernel<T, V, KR, kAggPrefix, true><<<wl.grid, wl.block, wl.smem, st>>>(d);     \
-  else agg_fwd_kernel<T, V, KR, kAggPrefix, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_PFX(T, V, KR)                                                                                      \
+  if (rope == 2 && KR <= 2) agg_fwd_kernel<T, V, KR, kAggPrefix, KR <= 2 ? 2 : 1><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) agg_fwd_kernel<T, V, KR, kAggPrefix, 1><<<wl.grid, wl.block, wl.smem, st>>>(d);                    \
+  else agg_fwd_kernel<T, V, KR, kAggPrefix, 0><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_PFX);
 #undef CALL_PFX
   }
@@ -1881,12 +1902,13 @@ int pom_poly_agg_mean_noalloc(const pom_agg_args* a, const float* denom, float s
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx}, {a->x});
   const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, kWhole);
   d.span = wl.span;
-  const bool has_rope = a->rope.kind != POM_ROPE_NONE;
+  const int rope = a->rope.kind == POM_ROPE_NONE ? 0 : wl.many() ? 2 : 1;
   // Every (sample, chunk, channel) slot that the reduction below reads is written by this launch first,
   // so nothing left in the workspace by an earlier call can leak into the result.
-#define CALL_NA(T, V, KR)                                                                      \
-  if (has_rope) agg_fwd_kernel<T, V, KR, kAggSum, true><<<wl.grid, wl.block, wl.smem, st>>>(d);        \
-  else agg_fwd_kernel<T, V, KR, kAggSum, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_NA(T, V, KR)                                                                                      \
+  if (rope == 2 && KR <= 2) agg_fwd_kernel<T, V, KR, kAggSum, KR <= 2 ? 2 : 1><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) agg_fwd_kernel<T, V, KR, kAggSum, 1><<<wl.grid, wl.block, wl.smem, st>>>(d);                    \
+  else agg_fwd_kernel<T, V, KR, kAggSum, 0><<<wl.grid, wl.block, wl.smem, st>>>(d)
   POM_DISPATCH_K(a->dtype, vec, a->K, CALL_NA);
 #undef CALL_NA
   count_launch();
@@ -2010,7 +2032,7 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
   const int vec = pick_vec(a->P, a->rope, a->dtype, a->K, {a->ldx, a->ld_dx, a->causal ? a->ld_dout : 0},
                            {a->x, a->dx, a->causal ? a->dout : nullptr});
   const WalkLaunch wl = walk_launch(a->P, a->rope.kind, vec, a->N, a->B, a->causal == 1 ? kWhole : kLanes);
-  const bool has_rope = a->rope.kind != POM_ROPE_NONE;
+  const int rope = a->rope.kind == POM_ROPE_NONE ? 0 : wl.many() ? 2 : 1;
   if (a->causal) {
     if (a->causal == 1) {
       // Plain column walk (no channel pairing) for the scaled chunk sums.
@@ -2028,16 +2050,21 @@ int pom_poly_agg_bwd(const pom_agg_bwd_args* a, void* stream) {
     }
     const bool deep = a->causal == 1 && (!(a->dtype == POM_BF16 && a->K > 2) ||
                                          1ll * wl.grid.x * wl.grid.y * wl.grid.z < 6ll * sm_count());
-#define CALL_BC(T, V, KR)                                                                                     \
-  if (has_rope) agg_bwd_kernel<T, V, KR, true, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);           \
-  else if (deep) agg_bwd_kernel<T, V, KR, true, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
-  else agg_bwd_kernel<T, V, KR, true, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_BC(T, V, KR)                                                                                           \
+  if (rope == 2 && (KR <= 2 || (KR <= 4 && V <= 4)))                                                                \
+    agg_bwd_kernel<T, V, KR, true, KR <= 2 || (KR <= 4 && V <= 4) ? 2 : 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);                  \
+  else if (rope) agg_bwd_kernel<T, V, KR, true, 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);                   \
+  else if (deep) agg_bwd_kernel<T, V, KR, true, 0, true><<<wl.grid, wl.block, wl.smem, st>>>(d);                    \
+  else agg_bwd_kernel<T, V, KR, true, 0, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BC);
 #undef CALL_BC
   } else {
-#define CALL_BN(T, V, KR)                                                                                     \
-  if (has_rope) agg_bwd_kernel<T, V, KR, false, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
-  else agg_bwd_kernel<T, V, KR, false, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+    // (bf16 means run best with their own registers at every size: 136 us at 32 x 1024 x 2304, 156 held to 168)
+#define CALL_BN(T, V, KR)                                                                                           \
+  if (rope == 2 && KR <= 4 && V <= 4)                                                                               \
+    agg_bwd_kernel<T, V, KR, false, KR <= 4 && V <= 4 ? 2 : 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);       \
+  else if (rope) agg_bwd_kernel<T, V, KR, false, 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);                  \
+  else agg_bwd_kernel<T, V, KR, false, 0, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH_K(a->dtype, vec, a->K, CALL_BN);
 #undef CALL_BN
   }
@@ -2056,21 +2083,23 @@ static int select_common(SelDev& d, int dtype, bool bwd, std::initializer_list<l
   const int vec = pick_vec(d.P, d.rope, dtype, 1, lds, ptrs);
   const WalkLaunch wl = walk_launch(d.P, d.rope.kind, vec, d.T, d.B, bwd ? kFour : kSpans);
   d.span = wl.span;
-  const bool has_rope = d.rope.kind != POM_ROPE_NONE;
+  const int rope = d.rope.kind == POM_ROPE_NONE ? 0 : wl.many() ? 2 : 1;
   if (bwd) {
-#define CALL_SB(T, V, KR)                                                                                   \
-  if (has_rope && d.h_per_token) select_kernel<T, V, true, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);    \
-  else if (has_rope) select_kernel<T, V, true, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);               \
-  else if (d.h_per_token) select_kernel<T, V, true, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
-  else select_kernel<T, V, true, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_SB(T, V, KR)                                                                              \
+  if (rope == 2 && d.h_per_token) select_kernel<T, V, true, 2, true><<<wl.grid, wl.block, wl.smem, st>>>(d);   \
+  else if (rope == 2) select_kernel<T, V, true, 2, false><<<wl.grid, wl.block, wl.smem, st>>>(d);              \
+  else if (rope && d.h_per_token) select_kernel<T, V, true, 1, true><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) select_kernel<T, V, true, 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);                  \
+  else if (d.h_per_token) select_kernel<T, V, true, 0, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else select_kernel<T, V, true, 0, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SB);
 #undef CALL_SB
   } else {
-#define CALL_SF(T, V, KR)                                                                                   \
-  if (has_rope && d.h_per_token) select_kernel<T, V, false, true, true><<<wl.grid, wl.block, wl.smem, st>>>(d);    \
-  else if (has_rope) select_kernel<T, V, false, true, false><<<wl.grid, wl.block, wl.smem, st>>>(d);               \
-  else if (d.h_per_token) select_kernel<T, V, false, false, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
-  else select_kernel<T, V, false, false, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
+#define CALL_SF(T, V, KR)                                                                              \
+  if (rope && d.h_per_token) select_kernel<T, V, false, 1, true><<<wl.grid, wl.block, wl.smem, st>>>(d); \
+  else if (rope) select_kernel<T, V, false, 1, false><<<wl.grid, wl.block, wl.smem, st>>>(d);                  \
+  else if (d.h_per_token) select_kernel<T, V, false, 0, true><<<wl.grid, wl.block, wl.smem, st>>>(d);          \
+  else select_kernel<T, V, false, 0, false><<<wl.grid, wl.block, wl.smem, st>>>(d)
     POM_DISPATCH(dtype, vec, CALL_SF);
 #undef CALL_SF
   }
