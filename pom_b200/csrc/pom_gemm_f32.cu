@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(256) near_kinks_kernel(const NearArgs a) {
 struct F32Out {
   float* C;
   long long ldc, split_stride;  // split_stride > 0: every K split stores its partial sums at C + split * stride
-  float alpha;
+  float alpha;   // times kUnscale
   int accumulate;
   SgemmFlags flags;
 };
@@ -475,8 +475,8 @@ gemm_f32_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
         if (left >= 32 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            float4 v = make_float4(out.alpha * (kUnscale * acc[c][4 * j]), out.alpha * (kUnscale * acc[c][4 * j + 1]),
-                                   out.alpha * (kUnscale * acc[c][4 * j + 2]), out.alpha * (kUnscale * acc[c][4 * j + 3]));
+            float4 v = make_float4(out.alpha * acc[c][4 * j], out.alpha * acc[c][4 * j + 1],
+                                   out.alpha * acc[c][4 * j + 2], out.alpha * acc[c][4 * j + 3]);
             float4* q = reinterpret_cast<float4*>(d) + j;
             if (out.accumulate) {
               const float4 o = *q;
@@ -488,7 +488,7 @@ gemm_f32_planes_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 #pragma unroll
           for (int i = 0; i < 32; ++i)
             if (i < left) {
-              const float v = out.alpha * (kUnscale * acc[c][i]);
+              const float v = out.alpha * acc[c][i];
               d[i] = out.accumulate ? d[i] + v : v;
             }
         }
@@ -641,10 +641,12 @@ int planes_product(const pom_gemm_args* a, void* a_planes, int a_ready, void* b_
   const F32Plan plan = pick_f32_plan(a->M, a->N, a->K, a->out_mode);
   const int ldp = static_cast<int>((a->N + 3) / 4 * 4);
   const bool accumulate = a->out_mode == POM_OUT_F32_ACCUM;
-  F32Out out{static_cast<float*>(a->C), a->ldc, 0, a->alpha, accumulate, flags};
+  // an alpha that the planes' factor would make subnormal: the FMA kernel (with the planes in place for a later product)
+  if (a->alpha != 0.f && fabsf(a->alpha) < 0x1p-78f) return launch_sgemm(a, SgemmFlags{nullptr, 0, nullptr, 0, 0, 0}, st);
+  F32Out out{static_cast<float*>(a->C), a->ldc, 0, a->alpha * kUnscale, accumulate, flags};
   if (plan.split > 1) {
     if (!scratch) return POM_ERR_NULL;
-    out = F32Out{static_cast<float*>(scratch), ldp, a->M * ldp, 1.f, 0, flags};
+    out = F32Out{static_cast<float*>(scratch), ldp, a->M * ldp, kUnscale, 0, flags};
   }
   const void *pa = planes_of(a_planes), *pb = planes_of(b_planes);
   const int rc = plan.bn == 256 ? launch_f32_any<256>(a, pa, pb, plan.split, out, status, st)

@@ -80,6 +80,16 @@ def test_small_and_large_magnitudes_are_no_further_off_than_a_chain(a_scale, b_s
     assert err[0] <= max(err[1], BOUND), err
 
 
+@pytest.mark.parametrize("alpha", [3.0, -2.0 ** -60, 2.0 ** -90, 0.0])
+def test_products_times_any_alpha(alpha):
+    """The factor of the planes is part of the epilogue's alpha, down to where that would be subnormal."""
+    a, b = _operands(300, 290, 260, False, False, 5)
+    got, want = _planes(a, b, alpha=alpha), alpha * _gemm64(a, b, False, False)
+    assert (got.double() - want).norm().item() <= BOUND * want.norm().item()
+    acc = _planes(a, b, alpha=alpha, out=torch.ones_like(got), accumulate=True)
+    assert (acc.double() - 1 - want).norm().item() <= BOUND * (1 + want).norm().item()
+
+
 def test_values_outside_the_range_of_the_planes_move_the_product_to_the_fma_kernel():
     a, b = _operands(300, 290, 260, False, False, 5)
     b = b.sign() * (1 + b.abs())
