@@ -546,7 +546,7 @@ typedef struct pom_layer_args {
   uint64_t workspace_bytes;
   /* Rotary embedding (pom/pom_rope.py:487-522) and the token-causal mask (pom/pom.py:92-95) inside the same two
    * calls, under the conditions of pom_ctx_gemm / pom_gate_gemm (degree <= 4, P % 16 == 0, 2-D: P % 64 == 0,
-   * positions constant or consecutive inside aligned 32-token groups); otherwise POM_ERR_UNSUPPORTED. */
+   * pom_rope::step0/1 in 0..3, token-causal 0 or 1); otherwise POM_ERR_UNSUPPORTED. */
   pom_rope rope_c;            /* positions of the N context tokens (kind POM_ROPE_NONE: no rotation) */
   pom_rope rope_q;            /* positions of the T query tokens */
   const void* w_ag_t;         /* backward with rope_q or causal: (P, D) bf16, the output weight transposed

@@ -1281,7 +1281,7 @@ struct SelDev {
 };
 
 // HT: one aggregate per token (a.H is of T), else one per sample (fp32).  As a choice at run time it held registers for both:
-// 80 instead of 57 in the float32 backward, two waves instead of one at 64 x 577 x 768 (86 us, now 65).
+// 80 instead of 57 in the float32 backward, two waves instead of one at 64 x 577 x 768 (86 us against 68).
 // (Rotated float32 forward keeps the choice at run time: 53 us at 64 x 577 x 768, 59 without.)
 template <typename T, int VEC, bool BWD, int ROPE, bool HT>
 __global__ void __launch_bounds__(ROPE ? kRopeThreads : kWalkThreads, ROPE ? rope_blocks<VEC, 1>(ROPE) : BWD ? 2 : 4)
@@ -1542,8 +1542,8 @@ __global__ void __launch_bounds__(128) flat_tile_kernel(const float* __restrict_
 }
 
 // Rows of a mask (bool or uint8, bf16, fp32) -> the same values as rows of bf16 or fp32 `ld` apart, and the sum of every
-// row as it was given.  One pass, a warp per row and 8 values per lane and step; 6144 x 1536 bool to bf16: 7 us, where a copy to
-// bf16, one to fp32 and their row sums took 244 us.
+// row as it was given.  One pass, a warp per row and 8 values per lane and step; 6144 x 1536 bool to bf16: 7 us (14 from
+// memory), where a copy to bf16, one to fp32 and their row sums took 244 us.
 template <typename S>
 __device__ __forceinline__ float mask_value(S v) { return static_cast<float>(v); }
 template <>

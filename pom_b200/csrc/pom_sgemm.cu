@@ -3,9 +3,9 @@
 // The order does not depend on the tile, the batch or the operands' storage order.  Products with a short K, and those
 // that the three-plane form (pom_gemm_f32.cu) cannot carry, come here.
 //
-// What bounds it: FMA issue (74 TFLOP/s at 1.965 GHz; 48 reached at 4080 x 4608 x 1152, 22 with the 4 x 4
-// outputs per thread and single buffer it had before; 8 x 16 outputs at one block per SM reach 47, scalar FMAs 44).  A thread keeps TM x TN outputs, so that 4 (or 3) shared-memory
-// reads feed 64 (or 32) FMAs; the next k-step is loaded into registers while the current one is computed from a
+// What bounds it: FMA issue (74 TFLOP/s at 1.965 GHz; 48 reached at 4080 x 4608 x 1152, where 4 x 4 outputs per thread
+// and a single buffer reach 22, 8 x 16 outputs at one block per SM 47, scalar FMAs 44).  A thread keeps TM x 8 outputs, so
+// that 4 (or 3) shared-memory reads feed 64 (or 32) FMAs; the next k-step is loaded into registers while the current one is computed from a
 // double-buffered tile, one barrier per step.
 #include "common.cuh"
 #include "sgemm.cuh"

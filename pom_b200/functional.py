@@ -328,8 +328,9 @@ class _PoMLayer(torch.autograd.Function):
             if tuple(mask.shape) != (B, N):
                 raise ValueError(f"expected a (B, N) = ({B}, {N}) mask, got {tuple(mask.shape)}")
             maskf = mask.to(device=xq.device, dtype=torch.float32).contiguous()
-        # rotary embedding rides in the GEMM epilogues when the positions of every aligned 32-token group are
-        # constant or consecutive (RopeSpec.steps) and the degree is at most 4; otherwise on the operator path
+        # rotary embedding rides in the GEMM epilogues when the positions of every aligned 32-token group are shared,
+        # consecutive or (not token-causal) at most 61 apart (RopeSpec.steps) and the degree is at most 4; otherwise on the
+        # operator path
         rotary = spec.rope_ctx is not None or spec.rope_qry is not None
         rope_ok = not rotary or (K <= 4 and all(r is None or r.fusable(P, causal) for r in (spec.rope_ctx, spec.rope_qry)))
         fused = (bf16 and not heads and (not rotary or rope_ok) and not causal and not full
@@ -340,7 +341,7 @@ class _PoMLayer(torch.autograd.Function):
         fused_causal = (causal and bf16 and not heads and (not rotary or rope_ok) and K <= 4 and D % 8 == 0
                         and P % (64 if two_d else 16) == 0)
 
-        hp = z = Hc = s32 = None
+        hp = z = Hc = gate = None
         collapsed = False
         ctx.collapsed = False
         ctx.fused_causal = fused_causal
@@ -443,7 +444,7 @@ class _PoMLayer(torch.autograd.Function):
             sh, z = ops.gate_gemm(xq, w_se, bias32, H, save_z=need_grad, rope=spec.rope_qry)
         elif heads:
             ones = _ones(B, heads, xq.device)
-            s32 = ops.select_fwd(z, bias32, ones, rope=spec.rope_qry)   # gate in head space (B, T, heads)
+            gate = ops.select_fwd(z, bias32, ones, rope=spec.rope_qry)  # in head space (B, T, heads)
             # one aggregate per sample: the P-wide gated state and its output GEMM collapse to a (heads x D)
             # matrix per sample (pom_heads_*); per-token aggregates (causal) keep the explicit form
             # (bf16: the batched tensor-core products of the collapsed form read rows of head_dim elements, and the gate
@@ -453,16 +454,16 @@ class _PoMLayer(torch.autograd.Function):
             if collapsed:
                 sh = ops.heads_mix(H, w_ag, heads)  # Mb (B, heads, D), kept in the slot of the gated state
             else:
-                s32 = _f32(s32)
+                gate = _f32(gate)
                 if full:  # the division by the mask's row sums rides on the (small) gate: s / rowsum, 0 for empty rows
-                    s32 = s32 * _inv_rows(rowden).view(B, T, 1)
-                sh = ops.select_heads_fwd(s32, Hc if (causal or full) else H, xq.dtype)
+                    gate = gate * _inv_rows(rowden).view(B, T, 1)
+                sh = ops.select_heads_fwd(gate, Hc if (causal or full) else H, xq.dtype)
         else:
             sh = ops.select_fwd(z, bias32, Hc if (causal or full) else H, rope=spec.rope_qry, row_denom=rowden)
         if residual is not None and not bf16:
             raise NotImplementedError("the fused residual add of the output projection is a bf16 feature")
         if collapsed:
-            y = ops.heads_out_fwd(s32, sh, xq.dtype, None if residual is None else residual.contiguous())
+            y = ops.heads_out_fwd(gate, sh, xq.dtype, None if residual is None else residual.contiguous())
         else:
             y = ops.gemm(sh.view(B * T, P), w_ag,
                          residual=None if residual is None else residual.contiguous().view(B * T, D)).view(B, T, D)
@@ -473,7 +474,7 @@ class _PoMLayer(torch.autograd.Function):
         ctx.collapsed = collapsed
         ctx.dims = (B, T, N, D, P, K, S, heads, n_glob, offset)
         ctx.h_past_dtype = None if h_past is None else h_past.dtype
-        ctx.save_for_backward(xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, Hc, sh, maskf, denom, s32, maskd, rowden)
+        ctx.save_for_backward(xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, Hc, sh, maskf, denom, gate, maskd, rowden)
         ctx.param_like = (w_qc, se_bias, coeff, w_ag)
         if spec.want_state:
             return y, H.view(B, 1, P)
@@ -483,7 +484,7 @@ class _PoMLayer(torch.autograd.Function):
     @on_tensor_device
     def backward(ctx, dy, dh_state):
         spec: LayerSpec = ctx.spec
-        xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, Hc, sh, maskf, denom, s32, maskd, rowden = ctx.saved_tensors
+        xq, xc, w_qc, w_ag, coeff32, bias32, hp, z, H, Hc, sh, maskf, denom, gate, maskd, rowden = ctx.saved_tensors
         B, T, N, D, P, K, S, heads, n_glob, offset = ctx.dims
         p_qc, p_bias, p_coeff, p_ag = ctx.param_like
         shard = spec.shard
@@ -579,7 +580,7 @@ class _PoMLayer(torch.autograd.Function):
                 dH = ops.reduce_partials(dh_p)
             ops.reduce_partials(db_p.view(1, -1, P), out=d_bias.view(1, P))
         elif ctx.collapsed:
-            ds, dMb = ops.heads_out_bwd(dy, s32, sh)            # sh holds Mb here
+            ds, dMb = ops.heads_out_bwd(dy, gate, sh)            # sh holds Mb here
             dH = ops.heads_mix_bwd(dMb, H, w_ag, d_wag)         # also dWo
             ops.select_bwd(ds, z, bias32, _ones(B, heads, dev), g_z.view(B, T, heads), rope=spec.rope_qry,
                            dbias_out=d_bias)
@@ -588,7 +589,7 @@ class _PoMLayer(torch.autograd.Function):
             dy_pl.drop()
             if heads:
                 ds32 = ops.zeros_f32(B * T * heads, dev).view(B, T, heads)
-                dH = ops.select_heads_bwd(dsh, s32, Hc if (causal or full) else H, ds32)
+                dH = ops.select_heads_bwd(dsh, gate, Hc if (causal or full) else H, ds32)
                 if full:
                     ds32 = ds32 * _inv_rows(rowden).view(B, T, 1)
                 ds = ds32 if dt == torch.float32 else ops.to_bf16(ds32)

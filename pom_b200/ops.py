@@ -193,7 +193,8 @@ def f32_planes_pay(K: int) -> bool:
     """Whether a float32 product runs on the tensor cores (``pom_gemm_f32_planes``) or on the FMA kernel.  At K = 64 and
     64 to 256 rows and columns the planes take 8 to 10 us (three launches) and the FMA kernel 5; at K = 128 11 and 8 to
     9.5; at K = 256 14 and 14 to 17, and from there on, or with more rows, the planes win by up to five times.  M and N
-    do not enter: a sample's result has the same bits whatever batch it came in."""
+    do not enter: a sample's result has the same bits whatever batch it came in (where memory has room for the planes, and
+    every value of the batch is in their range: one outside it moves the whole product to the FMA kernel)."""
     return K >= 128
 
 
@@ -271,8 +272,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
-# float32 projections with fewer weights run on the FMA kernel alone: its one launch takes 18 us for 512 tokens at
-# 1024 x 256, the four of the tensor-core form 30.  (The tokens do not enter: see f32_planes_pay.)
+# float32 projections with fewer weights run on the FMA kernel alone.  Tensor-core form (four launches) and FMA kernel (one)
+# at 128 / 512 / 2048 / 32768 tokens, us: 1024 x 256 (2^18 weights) 27 and 20, 27 and 20, 33 and 39, 244 and 369;
+# 1536 x 384 (2^19.2) 33 and 27, 35 and 37, 57 and 82, 434 and 799; 3072 x 768 53 and 49, 63 and 84, 139 and 244, 1249 and
+# 3098.  The line keeps the calls of a few hundred tokens, which the host bounds, at one launch.  (The tokens do not enter:
+# see f32_planes_pay.)
 F32_PROJECT_MIN_WEIGHTS = 1 << 19
 
 
