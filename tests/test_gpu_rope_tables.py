@@ -47,8 +47,8 @@ def _errors(mod, names, pos, x, dy, two_d, heights):
 
 
 @pytest.mark.parametrize("kind", ["centred", "cast"])
-@pytest.mark.parametrize("two_d,heights", [(True, (24, 24)), (True, (9, 40)), (True, (5, 62)), (False, (400,))],
-                         ids=["24x24", "9x40", "5x62", "1d"])
+@pytest.mark.parametrize("two_d,heights", [(True, (24, 24)), (True, (9, 40)), (True, (5, 62)), (False, (400,)), (False, (30,))],
+                         ids=["24x24", "9x40", "5x62", "1d", "1d_below_32"])
 @pytest.mark.parametrize("degree", [2, 4])
 def test_every_token_is_rotated_by_its_own_table_row(kind, two_d, heights, degree, monkeypatch):
     from pom_b200 import ops
@@ -61,10 +61,11 @@ def test_every_token_is_rotated_by_its_own_table_row(kind, two_d, heights, degre
         pos = torch.stack([torch.arange(N) // heights[1], torch.arange(N) % heights[1]], 1)
     else:
         N = 203
-        start = torch.randint(0, heights[0] - 61, ((N + 31) // 32,), generator=g).repeat_interleave(32)[:N]
-        pos = start + torch.randint(0, 62, (N,), generator=g)
+        span = min(62, heights[0])
+        start = torch.randint(0, heights[0] - span + 1, ((N + 31) // 32,), generator=g).repeat_interleave(32)[:N]
+        pos = start + torch.randint(0, span, (N,), generator=g)
     x, dy = (torch.randn(B, N, D, generator=g).bfloat16() for _ in range(2))
-    assert ops.rope_pos_info(pos.cuda())[-1][2] == (3 if heights == (24, 24) else 2)
+    assert ops.rope_pos_info(pos.cuda())[-1][2] == (3 if heights[-1] < 32 else 2)
     fused = _errors(mod, names, pos, x, dy, two_d, heights)
     monkeypatch.setattr(ops.RopeSpec, "fusable", lambda *_, **__: False)
     operators = _errors(mod, names, pos, x, dy, two_d, heights)
