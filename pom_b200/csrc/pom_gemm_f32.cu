@@ -73,12 +73,13 @@ __device__ __forceinline__ void load8(const float* s, long long left, bool vec, 
 
 // Largest and smallest magnitude (but zero) of the values a thread splits, as bits.
 struct Extremes {
-  uint32_t hi = 0, lo = 0x7f800000u;
+  uint32_t hi = 0, lo = 0xffffffffu;  // lo: less one, so that zero comes out on top
   __device__ __forceinline__ void see(float x) {
     const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
     hi = max(hi, u);
-    lo = min(lo, u ? u : lo);
+    lo = min(lo, u - 1u);
   }
+  __device__ __forceinline__ void add(const Extremes& o) { hi = max(hi, o.hi), lo = min(lo, o.lo); }
   // The word of the block (every thread calls it once).
   __device__ __forceinline__ void store(int* word) const {
     __shared__ uint32_t sh[2][kSplitThreads / 32];
@@ -88,7 +89,7 @@ struct Extremes {
     if (threadIdx.x == 0) {
       uint32_t a = sh[0][0], b = sh[1][0];
       for (int w = 1; w < kSplitThreads / 32; ++w) a = max(a, sh[0][w]), b = min(b, sh[1][w]);
-      *word = static_cast<int>(a >> 23 << 16 | b >> 23);
+      *word = static_cast<int>(a >> 23 << 16 | (b == 0xffffffffu ? 255u : (b + 1u) >> 23));
     }
   }
 };
@@ -143,7 +144,8 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
   const long long plane = m.rows * m.groups;
   Extremes seen;
   for (long long r = blockIdx.x * 1ll * warps + (threadIdx.x >> 5); r < m.rows; r += 1ll * m.blocks * warps) {
-    float sq = 0.f, top = 0.f;
+    float sq = 0.f;
+    Extremes row;
     for (long long g = lane; g < m.groups; g += 32) {
       float v[8];
       load8(m.src + r * m.ld + g * 8, m.cols - g * 8, vec, v);
@@ -151,18 +153,16 @@ __global__ void __launch_bounds__(kSplitThreads) split_rows_kernel(const SplitMa
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         sq = fmaf(v[2 * e], v[2 * e], fmaf(v[2 * e + 1], v[2 * e + 1], sq));
-        top = fmaxf(top, fmaxf(fabsf(v[2 * e]), fabsf(v[2 * e + 1])));
-        split_pair(v[2 * e], v[2 * e + 1], p[e], seen);
+        split_pair(v[2 * e], v[2 * e + 1], p[e], row);
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k)
         m.dst[k * plane + r * m.groups + g] = make_uint4(p[0][k], p[1][k], p[2][k], p[3][k]);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    }
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    seen.add(row);
+    const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, row.hi)) * (1.f / kScale);
     if (lane == 0) norm[r] = sq < 0x1p-60f ? top * sqrtf(static_cast<float>(m.cols)) : sqrtf(sq);
   }
   seen.store(m.flags + blockIdx.x);

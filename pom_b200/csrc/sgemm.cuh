@@ -36,16 +36,15 @@ struct SgemmFlags {
     return out_of_range(scan(a, na, lane, 32), scan(b, nb, lane, 32));
   }
   __device__ __forceinline__ bool any_in_block() const {
-    __shared__ int sh[4];
-    if (threadIdx.x < 4) sh[threadIdx.x] = threadIdx.x < 2 ? 0 : 255;
+    __shared__ int4 sh[8];  // per warp (blocks of up to 256 threads)
+    Range x = scan(a, na, threadIdx.x, blockDim.x), y = scan(b, nb, threadIdx.x, blockDim.x);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_int4(x.hi, x.lo, y.hi, y.lo);
     __syncthreads();
-    const Range x = scan(a, na, threadIdx.x, blockDim.x), y = scan(b, nb, threadIdx.x, blockDim.x);
-    if ((threadIdx.x & 31) == 0) {
-      atomicMax(sh, x.hi), atomicMax(sh + 1, y.hi);
-      atomicMin(sh + 2, x.lo), atomicMin(sh + 3, y.lo);
+    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
+      const int4 v = sh[w];
+      x = Range{max(x.hi, v.x), min(x.lo, v.y)}, y = Range{max(y.hi, v.z), min(y.lo, v.w)};
     }
-    __syncthreads();
-    return out_of_range(Range{sh[0], sh[2]}, Range{sh[1], sh[3]});
+    return out_of_range(x, y);
   }
 };
 
