@@ -21,10 +21,12 @@ struct SgemmFlags {
   // Of the words first, first + step, ... and the other lanes' (whole warp).
   __device__ __forceinline__ static Range scan(const int* w, int n, int first, int step) {
     int hi = 0, lo = 255;
-#pragma unroll 8
-    for (int i = first; i < n; i += step) {
-      const int v = __ldcg(w + i);
-      hi = max(hi, v >> 16), lo = min(lo, v & 255);
+    for (int i = first; i < n; i += 16 * step) {  // 16 loads in flight (past the end: a word of zeros)
+      int v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = i + j * step < n ? __ldcg(w + i + j * step) : 255;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) hi = max(hi, v[j] >> 16), lo = min(lo, v[j] & 255);
     }
     return Range{__reduce_max_sync(0xffffffffu, hi), __reduce_min_sync(0xffffffffu, lo)};
   }
